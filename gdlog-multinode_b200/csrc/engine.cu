@@ -34,6 +34,7 @@
 #include "index.cuh"
 #include "join.cuh"
 #include "merge.cuh"
+#include "product.cuh"
 #include "pull.cuh"
 #include "sort.cuh"
 #include "tma.cuh"
@@ -50,6 +51,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <tuple>
 #include <mutex>
 #include <vector>
 
@@ -128,6 +130,7 @@ struct LieHost {
   // domain) and the bitmap layout.
   bool dense = false;
   int dk = 0;
+  u32 side = 0;  // 256-id groups up to the largest id (pull.cuh)
   DenseMap map{};
   // Batched form: per-instance new-tuple counts of the running iteration and
   // the last iteration (+1) in which each instance produced new tuples.
@@ -223,11 +226,11 @@ struct gdl_engine {
   // engine (destroying one takes ~0.1 ms of host time that the caller's
   // next program need not wait for; none of them can be running).
   // Tensor maps of the square-domain bitmaps for the TMA passes (tma.cuh),
-  // by (base address, domain bits); tma_ok: the driver's encoder was found
+  // by (base address, domain bits, rows); tma_ok: the driver's encoder was found
   // (GDLOG_NO_TMA=1 keeps the LDG/STG passes of pull.cuh).
   bool tma_ok = false;
   void *tma_encode = nullptr;
-  std::map<std::pair<const void *, int>, CUtensorMap> tmaps;
+  std::map<std::tuple<const void *, int, u32>, CUtensorMap> tmaps;
   std::vector<cudaGraphExec_t> graveyard;
   std::mutex reap_mu;
   std::condition_variable reap_cv;
@@ -531,11 +534,11 @@ gdl_status push(gdl_engine *e) {
   return GDL_OK;
 }
 
-// The 2-D tensor map of a square-domain bitmap (2^dk rows of 2^(dk-5)
+// The 2-D tensor map of a square-domain bitmap (256 x side rows of 2^(dk-5)
 // words) with a box of one 256 x 256-bit tile; null if it cannot be made.
-const CUtensorMap *bm_tmap(gdl_engine *e, const u32 *bm, int dk) {
+const CUtensorMap *bm_tmap(gdl_engine *e, const u32 *bm, int dk, u32 side) {
   if (!e->tma_ok || !bm || dk < 8) return nullptr;
-  auto key = std::make_pair((const void *)bm, dk);
+  auto key = std::make_tuple((const void *)bm, dk, side);
   auto it = e->tmaps.find(key);
   if (it != e->tmaps.end()) return &it->second;
   using Encode = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
@@ -543,7 +546,7 @@ const CUtensorMap *bm_tmap(gdl_engine *e, const u32 *bm, int dk) {
                               const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
                               CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
   CUtensorMap m;
-  const cuuint64_t dims[2] = {1ull << (dk - 5), 1ull << dk};
+  const cuuint64_t dims[2] = {1ull << (dk - 5), 256ull * side};
   const cuuint64_t strides[1] = {(1ull << (dk - 5)) * 4};
   const cuuint32_t box[2] = {8, 256};
   const cuuint32_t estr[2] = {1, 1};
@@ -962,6 +965,8 @@ struct Plan {
   // per op: a row-gather join whose output bitmap (a transposed twin) is
   // all zero when it starts (pull.cuh, RowsArgs::dst_zero)
   std::vector<char> twin_zero;
+  // per op: pull form computed as a boolean product (product.cuh)
+  std::vector<char> product;
   // per op: a row-gather join writing an update relation's NEWT directly,
   // first of the iteration's ops to write that relation (the update step
   // leaves NEWT zero, so its rows are zero when the join starts)
@@ -992,6 +997,7 @@ Plan make_plan(gdl_engine *e, const LieHost &L) {
   p.static_once.assign(L.ops.size(), 0);
   p.twin_zero.assign(L.ops.size(), 0);
   p.g_zero.assign(L.ops.size(), 0);
+  p.product.assign(L.ops.size(), 0);
   {
     std::vector<char> is_static(n, 0), is_update(n, 0), newt_read(n, 0);
     for (int r : L.statics) is_static[r] = 1;
@@ -1040,8 +1046,7 @@ bool fused_update(const Plan &p, int r) { return p.fused[r] != 0; }
 // which the list is written if the loop ends with a DELTA left.
 void plan_pull(const gdl_engine *e, const LieHost &L, Plan &p) {
   if (!L.dense || e->instances || L.dk < kPullMinBits) return;
-  const bool pull_on = e->pull_joins == 3 || (e->pull_joins == 2 && L.dk >= kPullAutoBits);
-  if (!pull_on) {
+  if (e->pull_joins == 1) {
     for (int r : L.update)
       if (!p.delta_list[r] && !p.full_list[r]) p.fused[r] = p.delta_n[r] = 1;
     return;
@@ -1077,8 +1082,14 @@ void plan_pull(const gdl_engine *e, const LieHost &L, Plan &p) {
     const bool rev = plain && op.sel.s0 == 1 && op.sel.s1 == 3;
     const bool outer_ok = (op.outer_ver == GDL_DELTA && is_update[op.outer]) ||
                           (op.outer_ver == GDL_NEWT && is_tmp[op.outer]) || statics;
-    if ((fwd || rev) && outer_ok) {
+    // an inner FULL that is, or can be set as, a bitmap: a boolean product.
+    // Below 2^kPullAutoBits ids every other pull-form join is pushed.
+    const bool product = e->pull_joins == 2 && !statics && op.inner_ver != GDL_DELTA &&
+                         (is_update[op.inner] || is_static_r[op.inner]);
+    const bool pull_ok = product || e->pull_joins == 3 || L.dk >= kPullAutoBits;
+    if ((fwd || rev) && outer_ok && pull_ok) {
       p.pull[oi] = 1;
+      p.product[oi] = product;
       if (rev) p.pull_t[oi] = 1;
     } else if (op.outer_ver == GDL_NEWT) {
       p.newt_list[op.outer] = 1;
@@ -1089,6 +1100,18 @@ void plan_pull(const gdl_engine *e, const LieHost &L, Plan &p) {
   }
   for (size_t oi = 0; oi < L.ops.size(); oi++)
     if (L.ops[oi].kind == 1 && L.ops[oi].inner_ver == GDL_DELTA) p.delta_list[L.ops[oi].inner] = 1;
+  // Products read the inner's bitmap: no list of it, no index.
+  std::fill(p.full_list.begin(), p.full_list.end(), 0);
+  std::fill(p.full_idx.begin(), p.full_idx.end(), 0);
+  for (size_t oi = 0; oi < L.ops.size(); oi++) {
+    const OpHost &op = L.ops[oi];
+    if (op.kind == 0) {
+      if (op.inner_ver != GDL_DELTA && !p.product[oi]) p.full_list[op.inner] = p.full_idx[op.inner] = 1;
+      if (op.outer_ver == GDL_FULL) p.full_list[op.outer] = 1;
+    } else if (op.kind == 1 && op.inner_ver == GDL_FULL) {
+      p.full_list[op.inner] = 1;
+    }
+  }
   for (int r : L.update)
     if (!p.delta_list[r] && !p.full_list[r]) p.fused[r] = 1;
   // Row-gather form (pull.cuh, k_join_rows_bm) for the pull-form joins over
@@ -1107,6 +1130,15 @@ void plan_pull(const gdl_engine *e, const LieHost &L, Plan &p) {
     if (e->row_gather != 3 && bytes > kRowsBudget) continue;
     if (op.outer_ver == GDL_DELTA && !fused_update(p, op.outer)) continue;
     p.rows[oi] = 1;
+    p.product[oi] = 0;
+  }
+  // (row-gather joins read in-edge lists: an index only where another join
+  // probes it)
+  std::fill(p.full_idx.begin(), p.full_idx.end(), 0);
+  for (size_t oi = 0; oi < L.ops.size(); oi++) {
+    const OpHost &op = L.ops[oi];
+    if (op.kind == 0 && op.inner_ver != GDL_DELTA && !p.product[oi] && !p.rows[oi])
+      p.full_idx[op.inner] = 1;
   }
   // Which orientations of DELTA and NEWT the joins read.  A fused update
   // step keeps DELTA as rows when nothing reads it transposed (the record
@@ -1180,10 +1212,14 @@ gdl_status ensure_tbitmaps(gdl_engine *e, const Plan &p, int r, u64 words) {
   return GDL_OK;
 }
 
-// Bitmap size, in 32-bit words, of one relation version over the square
-// domain of dk-bit columns, padded to whole scan tiles (the scan kernels
+// Rows of a square-domain bitmap of dk-bit columns: the ids up to the
+// largest one loaded, in whole groups of 256 (from 2^8 ids on).
+u32 square_rows(int dk, u32 side) { return dk >= kPullMinBits ? 256 * side : 1u << dk; }
+// Its size in 32-bit words, padded to whole scan tiles (the scan kernels
 // work on whole tiles; padding bits are never set).
-u64 dense_words(int dk) { return round_up(1ull << (2 * dk - 5), kBmTileWords); }
+u64 dense_words(int dk, u32 side) {
+  return round_up((u64)square_rows(dk, side) << (dk - 5), kBmTileWords);
+}
 
 // One bitmap scan (dense.cuh) of relation `rel`: tile counts and their
 // prefix, then (unless the caller gates it) the write pass.
@@ -1243,14 +1279,15 @@ BmScanArgs scan_none(const DenseMap &map) {
 
 // (zeroed first: argument bytes, padding included, are compared by the
 // executable cache)
-TransposeArgs transpose_args(const u32 *g, const u32 *f, u32 *dst, int dk, DArr *count_to,
-                             u64 *count_acc, LaunchRec *lrec, Ctl *ctl) {
+TransposeArgs transpose_args(const u32 *g, const u32 *f, u32 *dst, int dk, u32 side,
+                             DArr *count_to, u64 *count_acc, LaunchRec *lrec, Ctl *ctl) {
   TransposeArgs t;
   memset(&t, 0, sizeof t);
   t.g = g;
   t.f = f;
   t.dst = dst;
   t.dk = dk;
+  t.side = side;
   t.count_to = count_to;
   t.count_acc = count_acc;
   t.lrec = lrec;
@@ -1278,6 +1315,28 @@ void launch_rows(gdl_engine *e, const RowsArgs &ra, Counts *kc) {
   }
 }
 
+// A boolean-product join (product.cuh): tables from 2^kProdTableBits ids on.
+// The key range is split until there are four units of work a block: at
+// 20,000 ids 400 row-by-column blocks share 148 SMs unevenly (3 rounds for
+// 2.7), and at 2^12 there are only 16.
+void launch_product(gdl_engine *e, ProdArgs &pa, Counts *kc) {
+  const bool tables = pa.dk >= kProdTableBits;
+  const u32 ids = pa.side * 256, mr = prod_rows(tables);
+  const u64 blocks = (u64)((ids + mr - 1) / mr) * ((ids + 1023) / 1024);
+  const int per_sm = tables ? 1 : 2;
+  const u64 want = (u64)e->sms * per_sm * (tables ? 4 : 1);
+  const u64 split = std::min<u64>(pa.side, std::max<u64>(1, (want + blocks - 1) / blocks));
+  pa.ksteps = (u32)((pa.side + split - 1) / split);
+  const u64 units = blocks * ((pa.side + pa.ksteps - 1) / pa.ksteps);
+  const int g = grid_for(e, units, 1, per_sm);
+  if (tables)
+    PLAUNCH(kc, kPJoinMat, k_join_product<kProdBigRows, true>
+            <<<g, kProdBlock, prod_smem(true), e->s>>>(pa));
+  else
+    PLAUNCH(kc, kPJoinMat, k_join_product<kProdSmallRows, false>
+            <<<g, kProdBlock, prod_smem(false), e->s>>>(pa));
+}
+
 // The sorted key list of a square-domain bitmap of `words` words (rows of
 // 2^rs words) into `out` (k_bm_list_*, dense.cuh): tile counts, offsets and
 // the list's size, keys.  out->n must hold the expected count.
@@ -1298,33 +1357,34 @@ gdl_status launch_list(gdl_engine *e, const u32 *bm, u64 words, int rs, DArr *ou
 
 // dst |= transpose(src) (or := with over), src cleared: the TMA pass
 // (tma.cuh) when both bitmaps have tensor maps, else the LDG/STG pass.
-void launch_fold(gdl_engine *e, u32 *src, u32 *dst, u8 *dirty, int dk, int over, Counts *kc,
-                 cudaStream_t s) {
-  const u64 side = 1ull << (dk - kPullMinBits);
-  const CUtensorMap *ms = bm_tmap(e, src, dk), *md = bm_tmap(e, dst, dk);
+void launch_fold(gdl_engine *e, u32 *src, u32 *dst, u8 *dirty, int dk, u32 side, int over,
+                 Counts *kc, cudaStream_t s) {
+  const u64 tiles = (u64)side * side;
+  const CUtensorMap *ms = bm_tmap(e, src, dk, side), *md = bm_tmap(e, dst, dk, side);
   if (ms && md) {
     FoldMaps m;
     m.src = *ms;
     m.dst = *md;
     const int ns = fold_tma_stages(over);
     PLAUNCH(kc, kPBitmap,
-            k_bm_fold_tma<<<grid_for(e, side * side, 1, over ? 3 : 2), kTrBlock,
-                            fold_tma_smem(ns, over), s>>>(m, dirty, dk, over, ns, e->d_ctl));
+            k_bm_fold_tma<<<grid_for(e, tiles, 1, over ? 3 : 2), kTrBlock,
+                            fold_tma_smem(ns, over), s>>>(m, dirty, dk, side, over, ns, e->d_ctl));
     return;
   }
-  PLAUNCH(kc, kPBitmap, k_bm_fold_t<<<grid_for(e, side * side, 1, 8), kTrBlock, 0, s>>>(
-                            src, dst, dirty, dk, over, e->d_ctl));
+  PLAUNCH(kc, kPBitmap, k_bm_fold_t<<<grid_for(e, tiles, 1, 8), kTrBlock, 0, s>>>(
+                            src, dst, dirty, dk, side, over, e->d_ctl));
 }
 
 // The fused update step of relation r (k_bm_update_t): NEWT from its
 // transposed twin gt or its rows, DELTA written as rows dn and/or
 // transposed dt; the TMA pass when every bitmap has a tensor map.
 void launch_update_t(gdl_engine *e, const BmScanArgs &a, int r, u32 *gt, u32 *dn, u32 *dt,
-                     int dk, Counts *kc, cudaStream_t s) {
+                     int dk, u32 side, Counts *kc, cudaStream_t s) {
   const RelDev &h = e->h[r];
-  const u64 side = 1ull << (dk - kPullMinBits);
-  const CUtensorMap *mn = bm_tmap(e, gt ? gt : h.bmG, dk), *mf = bm_tmap(e, h.bmF, dk);
-  const CUtensorMap *mdn = dn ? bm_tmap(e, dn, dk) : mf, *mdt = dt ? bm_tmap(e, dt, dk) : mf;
+  const u64 tiles = (u64)side * side;
+  const CUtensorMap *mn = bm_tmap(e, gt ? gt : h.bmG, dk, side), *mf = bm_tmap(e, h.bmF, dk, side);
+  const CUtensorMap *mdn = dn ? bm_tmap(e, dn, dk, side) : mf;
+  const CUtensorMap *mdt = dt ? bm_tmap(e, dt, dk, side) : mf;
   if (mn && mf && mdn && mdt) {
     UpdMaps m;
     m.nsrc = *mn;
@@ -1333,13 +1393,13 @@ void launch_update_t(gdl_engine *e, const BmScanArgs &a, int r, u32 *gt, u32 *dn
     m.dt = *mdt;
     const int ns = upd_tma_stages(dt != nullptr);
     PLAUNCH(kc, kPBitmap,
-            k_bm_update_tma<<<grid_for(e, side * side, 1, 2), kTrBlock,
+            k_bm_update_tma<<<grid_for(e, tiles, 1, 2), kTrBlock,
                               upd_tma_smem(ns, dt != nullptr), s>>>(
-                a, m, dk, gt != nullptr, dn != nullptr, dt != nullptr, ns));
+                a, m, side, gt != nullptr, dn != nullptr, dt != nullptr, ns));
     return;
   }
   PLAUNCH(kc, kPBitmap,
-          k_bm_update_t<<<grid_for(e, side * side, 1, 8), kTrBlock, 0, s>>>(a, dt, dk, gt, dn));
+          k_bm_update_t<<<grid_for(e, tiles, 1, 8), kTrBlock, 0, s>>>(a, dt, dk, side, gt, dn));
 }
 
 // In-edges of relation r's FULL list over 2^dk ids (k_inv_*, pull.cuh).
@@ -1501,6 +1561,7 @@ void enqueue_iteration(gdl_engine *e, LieHost &L, const Plan &plan, Counts *kc, 
         ra.j.rec = &e->recs[6];
         ra.O = op.outer_ver == GDL_DELTA ? oh.bmDN : op.outer_ver == GDL_FULL ? oh.bmF : oh.bmG;
         ra.outer_clear = op.outer_ver == GDL_NEWT ? oh.bmG : nullptr;
+        ra.outer_words = words;
         ra.clear_diag = op.pred.kind == GDL_PRED_NE;
         if (plan.static_once[oi]) {
           ra.j.once = &L.d_lie->jonce[oi];
@@ -1520,21 +1581,39 @@ void enqueue_iteration(gdl_engine *e, LieHost &L, const Plan &plan, Counts *kc, 
         ra.dk = L.dk;
         launch_rows(e, ra, kc);
         if (plan.out_twin[oi] && !plan.fold_late[op.out])
-          launch_fold(e, out.bmOT, out.bmG, out.dirty, L.dk, plan.fold_over[oi] && !out.dirty, kc,
-                      s);
+          launch_fold(e, out.bmOT, out.bmG, out.dirty, L.dk, L.side,
+                      plan.fold_over[oi] && !out.dirty, kc, s);
         continue;
       }
       if (plan.pull[oi]) {
         const u32 *OT = oh.bmDT;
-        const u64 side = 1ull << (L.dk - kPullMinBits);
         if (op.outer_ver == GDL_NEWT) {
-          TransposeArgs t = transpose_args(oh.bmG, nullptr, oh.bmGT, L.dk, &R[op.outer].newt,
-                                           e->d_pull_count, &e->recs[7], e->d_ctl);
-          PLAUNCH(kc, kPBitmap,
-                  k_bm_transpose<<<grid_for(e, side * side, 1, 8), kTrBlock, 0, s>>>(t));
+          TransposeArgs t = transpose_args(oh.bmG, nullptr, oh.bmGT, L.dk, L.side,
+                                           &R[op.outer].newt, e->d_pull_count, &e->recs[7],
+                                           e->d_ctl);
+          PLAUNCH(kc, kPBitmap, k_bm_transpose<<<grid_for(e, (u64)L.side * L.side, 1, 8), kTrBlock,
+                                                 0, s>>>(t));
           OT = oh.bmGT;
         }
         a.rec = &e->recs[6];
+        if (plan.product[oi]) {
+          // the inner is a FULL kept as a bitmap: a boolean product
+          const RelDev &out = e->h[op.out];
+          ProdArgs pa;
+          memset(&pa, 0, sizeof pa);
+          memcpy(&pa.j, &a, sizeof a);
+          pa.OT = OT;
+          pa.F = e->h[op.inner].bmF;
+          pa.G = plan.pull_t[oi] ? out.bmOT : out.bmG;
+          pa.dirty = plan.pull_t[oi] ? nullptr : out.dirty;
+          pa.dk = L.dk;
+          pa.side = L.side;
+          launch_product(e, pa, kc);
+          if (plan.pull_t[oi] && !plan.fold_late[op.out])
+            launch_fold(e, out.bmOT, out.bmG, out.dirty, L.dk, L.side,
+                        plan.fold_over[oi] && !out.dirty, kc, s);
+          continue;
+        }
         // row-OR: the gathered row is the inner's column 1 in both
         // orientations
         a.row_or = e->row_or_joins && op.inner_ver != GDL_DELTA && e->h[op.inner].dense &&
@@ -1543,10 +1622,10 @@ void enqueue_iteration(gdl_engine *e, LieHost &L, const Plan &plan, Counts *kc, 
         PLAUNCH(kc, kPJoinMat,
                 k_join_pull_bm<<<(int)e->sms * 8, kPullBlock, pull_acc_words(L.dk) * 4, s>>>(
                     a, plan.pull_t[oi] ? out.bmOT : out.bmG,
-                    plan.pull_t[oi] ? nullptr : out.dirty, OT, L.dk));
+                    plan.pull_t[oi] ? nullptr : out.dirty, OT, L.dk, words));
         if (plan.pull_t[oi] && !plan.fold_late[op.out])
-          launch_fold(e, out.bmOT, out.bmG, out.dirty, L.dk, plan.fold_over[oi] && !out.dirty, kc,
-                      s);
+          launch_fold(e, out.bmOT, out.bmG, out.dirty, L.dk, L.side,
+                      plan.fold_over[oi] && !out.dirty, kc, s);
         continue;
       }
       u64 outer_cap = std::max({oh.delta.cap, oh.delta_next.cap, oh.full.cap, oh.full_next.cap,
@@ -1635,6 +1714,16 @@ void enqueue_iteration(gdl_engine *e, LieHost &L, const Plan &plan, Counts *kc, 
       if (dense && op.kind == 2) {
         // RelationalACopy: dest NEWT := sel(src NEWT), bitmap to bitmap.
         const u64 tiles = words / kBmTileWords;
+        if (L.dk >= kPullMinBits && sh.bmG && !e->h[op.out].dirty && op.inner != op.out &&
+            op.sel.s0 == 1 && op.sel.s1 == 0) {
+          // (src[1], src[0]): the source's NEWT transposed, every word of
+          // the destination's NEWT written
+          TransposeArgs t = transpose_args(sh.bmG, nullptr, e->h[op.out].bmG, L.dk, L.side,
+                                           nullptr, nullptr, &e->recs[7], e->d_ctl);
+          PLAUNCH(kc, kPBitmap, k_bm_transpose<<<grid_for(e, (u64)L.side * L.side, 1, 8), kTrBlock,
+                                                 0, s>>>(t));
+          continue;
+        }
         PLAUNCH(kc, kPBitmap, k_bm_clear_dirty<<<grid_for(e, tiles, 1, 8), 256, 0, s>>>(
                                   &R[op.out], map, e->d_ctl));
         if (sh.bmG)  // a source without a NEWT bitmap (static) has an empty NEWT
@@ -1714,17 +1803,17 @@ void enqueue_update_step(gdl_engine *e, LieHost &L, const Plan &plan, Counts *kc
     for (const BmScanArgs &a : scans) {
       const int r = (int)(a.rd - R);
       if (plan.delta_t[r]) {
-        const u64 side = 1ull << (L.dk - kPullMinBits);
-        TransposeArgs t = transpose_args(e->h[r].bmG, e->h[r].bmF, e->h[r].bmDT, L.dk, nullptr,
-                                         nullptr, &e->recs[7], e->d_ctl);
-        PLAUNCH(kc, kPBitmap, k_bm_transpose<<<grid_for(e, side * side, 1, 8), kTrBlock, 0, s>>>(t));
+        TransposeArgs t = transpose_args(e->h[r].bmG, e->h[r].bmF, e->h[r].bmDT, L.dk, L.side,
+                                         nullptr, nullptr, &e->recs[7], e->d_ctl);
+        PLAUNCH(kc, kPBitmap, k_bm_transpose<<<grid_for(e, (u64)L.side * L.side, 1, 8), kTrBlock, 0,
+                                               s>>>(t));
       }
     }
     for (const BmScanArgs &a : fused) {
       const int r = (int)(a.rd - R);
       launch_update_t(e, a, r, plan.fold_late[r] ? e->h[r].bmOT : nullptr,
                       plan.delta_n[r] ? e->h[r].bmDN : nullptr,
-                      plan.delta_t[r] ? e->h[r].bmDT : nullptr, L.dk, kc, s);
+                      plan.delta_t[r] ? e->h[r].bmDT : nullptr, L.dk, L.side, kc, s);
     }
     for (const BmScanArgs &a : scans) launch_scan_write(e, a, kc);
     // tmp relations: NEWT is cleared after the operators (src/lie.cu:85-87),
@@ -2223,7 +2312,10 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
                   "FULL of %s is kept as a bitmap only (batched form, too large for a list)",
                   e->rels[r].name.c_str());
   {
-    const int dk = std::max(e->kbits, 5);
+    // (by default at least one 256 x 256-bit tile, so that every domain has
+    // the passes over tiles; pull.cuh, product.cuh)
+    const int dk = std::max(
+        e->kbits, e->pull_joins == 2 && 2 * kPullMinBits <= e->dense_max_bits ? kPullMinBits : 5);
     // Bitmaps hold arity-2 tuples without dependent columns only.
     bool plain = !e->wide;
     for (auto *v : {&L.update, &L.statics, &L.tmps})
@@ -2231,12 +2323,15 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
     for (const OpHost &op : L.ops) plain = plain && !op.generic;
     L.dense = plain && (e->instances || (e->dedup_mode != 1 && 2 * dk <= e->dense_max_bits));
     L.dk = L.dense && !e->instances ? dk : 0;
+    L.side = (u32)(e->max_value >> 8) + 1;
     plan_pull(e, L, plan);
   }
   for (RelDev &h : e->h) {
     h.dense = h.full_lazy = 0;
     h.dirty = nullptr;
   }
+  // static relations whose FULL is set as a bitmap for this LIE
+  std::vector<char> static_bm(e->rels.size(), 0);
   if (L.dense) {
     if (e->instances) {
       L.map = DenseMap{e->d_segs, e->d_tile_inst, (u32)e->segs.size(), e->seg_shift, e->seg_words};
@@ -2252,9 +2347,9 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
       CK(e, cudaMemsetAsync(L.d_inst_last, 0, n * sizeof(u64), e->s));
     } else {
       if (!e->d_square_seg) TRY(dalloc(e, (void **)&e->d_square_seg, sizeof(SegInfo)));
-      const SegInfo sq{0, (u32)(L.dk - 5), 1u << L.dk};
+      const SegInfo sq{0, (u32)(L.dk - 5), square_rows(L.dk, L.side)};
       CK(e, cudaMemcpyAsync(e->d_square_seg, &sq, sizeof sq, cudaMemcpyHostToDevice, e->s));
-      L.map = DenseMap{e->d_square_seg, nullptr, 1, 31, dense_words(L.dk)};
+      L.map = DenseMap{e->d_square_seg, nullptr, 1, 31, dense_words(L.dk, L.side)};
     }
     const u64 words = L.map.words;
     for (int r : L.update) {
@@ -2270,6 +2365,15 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
     }
     for (auto *v : {&L.update, &L.tmps})
       for (int r : *v) TRY(ensure_tbitmaps(e, plan, r, words));
+    // (before the relation table is uploaded: a later read-back of the table
+    // replaces the host mirror)
+    for (size_t oi = 0; oi < L.ops.size(); oi++) {
+      const OpHost &op = L.ops[oi];
+      if (plan.rows[oi] && op.outer_ver == GDL_FULL) static_bm[op.outer] = 1;
+      if (plan.product[oi] && !is_update[op.inner]) static_bm[op.inner] = 1;
+    }
+    for (size_t r = 0; r < static_bm.size(); r++)
+      if (static_bm[r]) TRY(ensure_static_bitmap(e, (int)r, words));
     mark("bitmap_alloc");
     // A dirty map pays when a NEWT bitmap is too large to scan whole every
     // iteration; for small ones the scans read everything and the joins
@@ -2348,21 +2452,19 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
     for (auto *v : {&L.update, &L.tmps})
       for (int r : *v)
         if (plan.out_t[r]) CK(e, cudaMemsetAsync(e->h[r].bmOT, 0, words * 4, e->s));
-    // the FULL bitmaps of the static outers of row-gather joins
-    {
-      std::vector<char> built_o(e->rels.size(), 0);
-      for (size_t oi = 0; oi < L.ops.size(); oi++) {
-        const OpHost &op = L.ops[oi];
-        if (!plan.rows[oi] || op.outer_ver != GDL_FULL || built_o[op.outer]) continue;
-        TRY(ensure_static_bitmap(e, op.outer, words));
-        const RelDev &h = e->h[op.outer];
-        CK(e, cudaMemsetAsync(h.bmF, 0, words * 4, e->s));
-        if (h.full.n) {
-          k_bm_from_list<<<grid_for(e, h.full.n, 256, 8), 256, 0, e->s>>>(
-              &e->d_rels[op.outer].full, h.bmF, L.map, e->d_ctl);
-          e->aux_launches++;
-        }
-        built_o[op.outer] = 1;
+    // (transposes write the tiles that hold ids; the pull form reads whole rows)
+    for (int r : L.tmps)
+      if (plan.newt_t[r]) CK(e, cudaMemsetAsync(e->h[r].bmGT, 0, words * 4, e->s));
+    // the FULL bitmaps of the static outers of row-gather joins and of the
+    // static inners of products
+    for (size_t r = 0; r < static_bm.size(); r++) {
+      if (!static_bm[r]) continue;
+      const RelDev &h = e->h[r];
+      CK(e, cudaMemsetAsync(h.bmF, 0, words * 4, e->s));
+      if (h.full.n) {
+        k_bm_from_list<<<grid_for(e, h.full.n, 256, 8), 256, 0, e->s>>>(
+            &e->d_rels[r].full, h.bmF, L.map, e->d_ctl);
+        e->aux_launches++;
       }
     }
     // the in-edges of the static inners of row-gather joins
@@ -2799,7 +2901,6 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
     if (any_delta) {
       TRY(resume_ctl());
       TRY(push(e));
-      const u64 side = 1ull << (L.dk - kPullMinBits);
       for (int r : L.update) {
         const RelDev &h = e->h[r];
         if (!(delta_unlisted(r) && h.delta.n)) continue;
@@ -2807,9 +2908,9 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
         // (empty) NEWT bitmap
         const u32 *rows = h.bmDN;
         if (!plan.delta_n[r]) {
-          TransposeArgs t = transpose_args(h.bmDT, nullptr, h.bmG, L.dk, nullptr, nullptr,
+          TransposeArgs t = transpose_args(h.bmDT, nullptr, h.bmG, L.dk, L.side, nullptr, nullptr,
                                            &e->recs[7], e->d_ctl);
-          k_bm_transpose<<<grid_for(e, side * side, 1, 8), kTrBlock, 0, e->s>>>(t);
+          k_bm_transpose<<<grid_for(e, (u64)L.side * L.side, 1, 8), kTrBlock, 0, e->s>>>(t);
           e->aux_launches++;
           rows = h.bmG;
         }
@@ -2955,6 +3056,12 @@ gdl_status gdl_engine_create(int32_t device, void *stream, gdl_engine **out) {
                                (int)sort_smem_bytes<10>())) ||
       bad(cudaFuncSetAttribute(k_merge_diff, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kMergeSmemBytes)) ||
+      bad(cudaFuncSetAttribute(k_join_product<kProdBigRows, true>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)prod_smem(true))) ||
+      bad(cudaFuncSetAttribute(k_join_product<kProdSmallRows, false>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)prod_smem(false))) ||
       bad(cudaFuncSetAttribute(k_join_pull_bm, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)(pull_acc_words(16) * 4))) ||
       bad(cudaMalloc(&e->d_rels, kMaxRels * sizeof(RelDev))) ||
@@ -3602,7 +3709,7 @@ gdl_status gdl_relation_digest(gdl_engine *e, int32_t rel, int32_t ver, uint64_t
     // FULL beyond the list limit, kept as its square-domain bitmap
     TRY(pull(e));
     if (!e->d_square_seg) TRY(dalloc(e, (void **)&e->d_square_seg, sizeof(SegInfo)));
-    const SegInfo sq{0, (u32)(rr.bm_dk - 5), 1u << rr.bm_dk};
+    const SegInfo sq{0, (u32)(rr.bm_dk - 5), (u32)(rr.bm_words >> (rr.bm_dk - 5))};
     CK(e, cudaMemcpyAsync(e->d_square_seg, &sq, sizeof sq, cudaMemcpyHostToDevice, e->s));
     const DenseMap map{e->d_square_seg, nullptr, 1, 31, rr.bm_words};
     std::vector<u64> size, dig;

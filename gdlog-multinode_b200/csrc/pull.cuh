@@ -39,7 +39,10 @@
 //                   column 1 into a transposed twin of the output NEWT,
 //                   which this pass ORs into NEWT transposed and clears.
 //
-// The square domain only (ids below 2^dk, 8 <= dk <= 16; one instance).
+// The square domain only (ids below 2^dk, 8 <= dk <= 16; one instance).  A
+// bitmap has rows of 2^(dk-5) words for the ids up to the largest one loaded
+// (rounded up to 256: `side` tiles of 256), so passes over tiles visit
+// side x side of them (20,000 ids of 2^15: 79^2 of 128^2).
 #pragma once
 
 #include "common.cuh"
@@ -83,7 +86,8 @@ struct TransposeArgs {
   const u32 *g;   // source bitmap
   const u32 *f;   // if set: the source is g & ~f
   u32 *dst;       // transposed bitmap (every word written)
-  int dk;         // 2^dk ids, rows of 2^(dk-5) words
+  int dk;         // rows of 2^(dk-5) words
+  u32 side;       // 256 x 256-bit tiles per side that hold ids
   DArr *count_to; // if set: receives the number of bits as its n
   u64 *count_acc; // zero between launches
   LaunchRec *lrec;
@@ -95,7 +99,7 @@ __global__ void __launch_bounds__(kTrBlock) k_bm_transpose(TransposeArgs a) {
   __shared__ unsigned long long s_bits;
   if (ctl_stop(a.ctl)) return;
   const int rs = a.dk - 5;
-  const u64 per = 1ull << (a.dk - 8);  // tiles per side
+  const u64 per = a.side;
   const u64 tiles = per * per;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   u64 bits = 0, moved = 0;
@@ -167,8 +171,8 @@ __global__ void __launch_bounds__(kTrBlock) k_bm_transpose(TransposeArgs a) {
 // every join that writes the relation has a transposed output and nothing
 // reads its NEWT during the iteration, NEWT is only that transposed twin
 // (never folded): it is read transposed, tile by tile, and cleared.
-__global__ void __launch_bounds__(kTrBlock, 4) k_bm_update_t(BmScanArgs a, u32 *dt, int dk, u32 *gt,
-                                                          u32 *dn) {
+__global__ void __launch_bounds__(kTrBlock, 4) k_bm_update_t(BmScanArgs a, u32 *dt, int dk, u32 side,
+                                                          u32 *gt, u32 *dn) {
   __shared__ u32 s_t[256][9];
   __shared__ unsigned long long s_cnt[2];
   if (ctl_stop(a.ctl)) return;
@@ -177,7 +181,7 @@ __global__ void __launch_bounds__(kTrBlock, 4) k_bm_update_t(BmScanArgs a, u32 *
   u32 *G = const_cast<u32 *>(a.g);
   u32 *F = a.f;
   const int rs = dk - 5;
-  const u64 per = 1ull << (dk - 8);
+  const u64 per = side;
   const u64 tiles = per * per;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0;
@@ -336,7 +340,7 @@ __host__ __device__ __forceinline__ u32 pull_acc_words(int dk) {
 // relation's NEWT, or its transposed twin for a join whose output is
 // (inner column 1, outer column 1).
 __global__ void __launch_bounds__(kPullBlock, 8) k_join_pull_bm(JoinArgs a, u32 *G, u8 *D,
-                                                               const u32 *OT, int dk) {
+                                                               const u32 *OT, int dk, u64 words) {
   __shared__ PullSmem sm;
   extern __shared__ u32 acc[];
   if (ctl_stop(a.ctl)) return;
@@ -352,7 +356,7 @@ __global__ void __launch_bounds__(kPullBlock, 8) k_join_pull_bm(JoinArgs a, u32 
   const int rs = dk - 5;
   const u32 row_mask = (1u << rs) - 1;
   const u32 acc_words = pull_acc_words(dk);
-  const u32 units = (u32)((1ull << (2 * dk - 5)) / kPullUnit);
+  const u32 units = (u32)(words / kPullUnit);
   const u32 n_ids = 1u << dk;
   // Row-OR (the inner is a FULL kept as a bitmap): a run of at least a
   // quarter of a row is ORed from the inner's bitmap row instead of being
@@ -578,6 +582,7 @@ struct RowsArgs {
   const u32 *O;        // the outer's rows: DELTA (non-transposed copy), a tmp NEWT, or a
                        // static FULL's bitmap
   u32 *outer_clear;    // bitmap to clear if an empty inner zeroes a NEWT outer
+  u64 outer_words;     // ... its size
   const u32 *inv_keys;  // in-edge sources, grouped by y
   const u32 *inv_ys;    // the y of each in-edge
   const u32 *inv_off;   // inv_off[2^dk]: the number of in-edges
@@ -652,7 +657,7 @@ __global__ void __launch_bounds__(256) k_join_rows_bm(RowsArgs a) {
     }
     if (a.outer_clear) {
       uint4 *p = reinterpret_cast<uint4 *>(a.outer_clear);
-      const u64 n4 = (1ull << (2 * a.dk - 5)) / 4;
+      const u64 n4 = a.outer_words / 4;
       for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n4;
            i += (u64)gridDim.x * blockDim.x)
         p[i] = make_uint4(0, 0, 0, 0);
@@ -774,11 +779,11 @@ __global__ void __launch_bounds__(256) k_join_rows_bm(RowsArgs a) {
 // writer of a tmp relation's NEWT in an iteration, without a dirty map: what
 // dst held before is not part of this iteration's NEWT).
 __global__ void __launch_bounds__(kTrBlock) k_bm_fold_t(u32 *src, u32 *dst, u8 *dirty, int dk,
-                                                        int overwrite, Ctl *ctl) {
+                                                        u32 side, int overwrite, Ctl *ctl) {
   __shared__ u32 s_t[256][9];
   if (ctl_stop(ctl)) return;
   const int rs = dk - 5;
-  const u64 per = 1ull << (dk - 8);
+  const u64 per = side;
   const u64 tiles = per * per;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   u64 moved = 0;

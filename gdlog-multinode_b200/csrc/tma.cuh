@@ -145,7 +145,7 @@ enum UpdFlag : u32 { kFAnyN = 1, kFAnyG = 2, kFFail = 4 };
 // bitmap G (m.nsrc over G; cleared where it has bits).  has_dn / has_dt:
 // write DELTA's rows / DELTA transposed (every word).  ns input stages.
 __global__ void __launch_bounds__(kTrBlock, 2)
-    k_bm_update_tma(BmScanArgs a, const __grid_constant__ UpdMaps m, int dk, int gt, int has_dn,
+    k_bm_update_tma(BmScanArgs a, const __grid_constant__ UpdMaps m, u32 side, int gt, int has_dn,
                     int has_dt, int ns) {
   extern __shared__ unsigned char tma_smem_raw[];
   __shared__ u32 s_t[256][9];
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(kTrBlock, 2)
   auto out_dt = [&](int o) { return tile_at(2 * ns + o * nout + 2); };
   u32 *zero = tile_at(2 * ns + 2 * nout);
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const u64 per = 1ull << (dk - 8);
+  const u64 per = side;
   const u64 tiles = per * per;
   const u32 limit = a.ctl->spin_limit;
   for (int i = tid; i < kTmaTile / 16; i += kTrBlock)
@@ -317,8 +317,8 @@ __global__ void __launch_bounds__(kTrBlock, 2)
 // overwrite, dst := transpose(src), every word stored), src cleared where it
 // has bits, the dirty map of dst set for its non-zero rows.  ns input stages.
 __global__ void __launch_bounds__(kTrBlock, 2)
-    k_bm_fold_tma(const __grid_constant__ FoldMaps m, u8 *dirty, int dk, int overwrite, int ns,
-                  Ctl *ctl) {
+    k_bm_fold_tma(const __grid_constant__ FoldMaps m, u8 *dirty, int dk, u32 side, int overwrite,
+                  int ns, Ctl *ctl) {
   extern __shared__ unsigned char tma_smem_raw[];
   __shared__ u32 s_t[256][9];
   __shared__ u32 s_wf[2][kTrBlock / 32];
@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(kTrBlock, 2)
   u32 *zero = tile_at(ni * ns + 2);
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int rs = dk - 5;
-  const u64 per = 1ull << (dk - 8);
+  const u64 per = side;
   const u64 tiles = per * per;
   const u32 limit = ctl->spin_limit;
   for (int i = tid; i < kTmaTile / 16; i += kTrBlock)
