@@ -123,15 +123,13 @@ __device__ __forceinline__ void dswap(T &a, T &b) {
 // graph body then needs no k_begin of its own; the host launches one
 // before each graph launch).  One warp: lane l commits entries l, l + 32,
 // ... of each list; the loop-level decisions are warp-uniform.
-__global__ void k_commit(RelDev *rels, LieDev *L, Ctl *ctl, int begin_next) {
-  const int lane = threadIdx.x;
-  if (lane >= 32) return;
+// Returns whether the loop stops here.
+__device__ __forceinline__ bool commit_iteration(RelDev *rels, LieDev *L, Ctl *ctl, int begin_next,
+                                                 int lane) {
   // the control words and the lists, all loads in flight together
   bool stop = ctl->done | ctl->pause | ctl->overflow | ctl->timeout;
   const u64 it = ctl->iteration, trace_base = ctl->trace_base;
   const u64 trace_rows = ctl->trace_rows, max_it = ctl->max_iteration, stop_at = ctl->stop_at;
-  const u32 cond_set = ctl->cond_set;
-  const unsigned long long cond_handle = ctl->cond_handle;
   const LaneLists x = lane_lists(L, lane);
   u64 *trace = L->trace;
   if (!stop) {
@@ -214,6 +212,15 @@ __global__ void k_commit(RelDev *rels, LieDev *L, Ctl *ctl, int begin_next) {
     if (begin_next && !stop) begin_iteration(rels, L, x, lane);
     __threadfence();
   }
+  return stop;
+}
+
+__global__ void k_commit(RelDev *rels, LieDev *L, Ctl *ctl, int begin_next) {
+  const int lane = threadIdx.x;
+  if (lane >= 32) return;
+  const u32 cond_set = ctl->cond_set;
+  const unsigned long long cond_handle = ctl->cond_handle;
+  const bool stop = commit_iteration(rels, L, ctl, begin_next, lane);
   if (lane == 0 && cond_set)
     cudaGraphSetConditional((cudaGraphConditionalHandle)cond_handle, stop ? 0u : 1u);
 }

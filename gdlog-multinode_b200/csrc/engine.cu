@@ -33,6 +33,7 @@
 #include "dense.cuh"
 #include "index.cuh"
 #include "join.cuh"
+#include "loop.cuh"
 #include "merge.cuh"
 #include "product.cuh"
 #include "pull.cuh"
@@ -126,6 +127,12 @@ struct LieHost {
   bool graph_reused = false;  // the last fixpoint's executable came from it
   bool graph_dirty = true;
   Counts per_iter;  // launches of one enqueued iteration
+  // Resident loop (loop.cuh): the graph's body is one launch that runs every
+  // iteration; its steps and update list in device memory.
+  bool resident = false;
+  LoopStep *d_steps = nullptr;
+  LoopUpd *d_upd = nullptr;
+  int n_steps = 0, n_upd = 0;
   // Dense form of the running fixpoint (dense.cuh): bits per column (square
   // domain) and the bitmap layout.
   bool dense = false;
@@ -295,7 +302,7 @@ struct gdl_engine {
   u64 lb_cnt_tiles = 0, lb_nz_tiles = 0, lb_merge_tiles = 0;
   LaunchRec *recs = nullptr;  // [0] join count, [1] join mat, [2] merge, [3] copy,
                               // [4] [5] bitmap scans, [6] pull join, [7] transpose,
-                              // [8] bitmap listing
+                              // [8] bitmap listing, [9] products over listed keys
   DArr *d_tmp = nullptr;      // [4] temporary descriptors for loads
   void *d_count = nullptr;    // gdl_join_count's scratch (CountScratch)
   void *d_part = nullptr;     // gdl_partition_rows: counts and cursors per destination
@@ -1082,10 +1089,12 @@ void plan_pull(const gdl_engine *e, const LieHost &L, Plan &p) {
     const bool rev = plain && op.sel.s0 == 1 && op.sel.s1 == 3;
     const bool outer_ok = (op.outer_ver == GDL_DELTA && is_update[op.outer]) ||
                           (op.outer_ver == GDL_NEWT && is_tmp[op.outer]) || statics;
-    // an inner FULL that is, or can be set as, a bitmap: a boolean product.
+    // an inner FULL kept as a bitmap: a boolean product (a static inner's
+    // bitmap is as large but sparse: only where a product is the small one).
     // Below 2^kPullAutoBits ids every other pull-form join is pushed.
     const bool product = e->pull_joins == 2 && !statics && op.inner_ver != GDL_DELTA &&
-                         (is_update[op.inner] || is_static_r[op.inner]);
+                         (is_update[op.inner] ||
+                          (is_static_r[op.inner] && L.dk < kProdTableBits));
     const bool pull_ok = product || e->pull_joins == 3 || L.dk >= kPullAutoBits;
     if ((fwd || rev) && outer_ok && pull_ok) {
       p.pull[oi] = 1;
@@ -1315,26 +1324,35 @@ void launch_rows(gdl_engine *e, const RowsArgs &ra, Counts *kc) {
   }
 }
 
-// A boolean-product join (product.cuh): tables from 2^kProdTableBits ids on.
-// The key range is split until there are four units of work a block: at
-// 20,000 ids 400 row-by-column blocks share 148 SMs unevenly (3 rounds for
-// 2.7), and at 2^12 there are only 16.
+// A boolean-product join (product.cuh).  With tables, from
+// 2^kProdTableBits ids on, the key range is split until there are four units
+// of work a block: at 20,000 ids 400 row-by-column blocks share 148 SMs
+// unevenly (3 rounds for 2.7), and at 2^12 there are only 16.
 void launch_product(gdl_engine *e, ProdArgs &pa, Counts *kc) {
-  const bool tables = pa.dk >= kProdTableBits;
-  const u32 ids = pa.side * 256, mr = prod_rows(tables);
-  const u64 blocks = (u64)((ids + mr - 1) / mr) * ((ids + 1023) / 1024);
-  const int per_sm = tables ? 1 : 2;
-  const u64 want = (u64)e->sms * per_sm * (tables ? 4 : 1);
-  const u64 split = std::min<u64>(pa.side, std::max<u64>(1, (want + blocks - 1) / blocks));
+  const u32 ids = pa.side * 256;
+  if (pa.dk < kProdTableBits) {
+    PLAUNCH(kc, kPJoinMat, k_join_product_small
+            <<<grid_for(e, (u64)ids * pa.splits, 8, 4), 256, 0, e->s>>>(pa));
+    return;
+  }
+  const u64 blocks = (u64)((ids + kProdRows - 1) / kProdRows) * ((ids + 1023) / 1024);
+  const u64 split =
+      std::min<u64>(pa.side, std::max<u64>(1, ((u64)e->sms * 4 + blocks - 1) / blocks));
   pa.ksteps = (u32)((pa.side + split - 1) / split);
   const u64 units = blocks * ((pa.side + pa.ksteps - 1) / pa.ksteps);
-  const int g = grid_for(e, units, 1, per_sm);
-  if (tables)
-    PLAUNCH(kc, kPJoinMat, k_join_product<kProdBigRows, true>
-            <<<g, kProdBlock, prod_smem(true), e->s>>>(pa));
-  else
-    PLAUNCH(kc, kPJoinMat, k_join_product<kProdSmallRows, false>
-            <<<g, kProdBlock, prod_smem(false), e->s>>>(pa));
+  PLAUNCH(kc, kPJoinMat, k_join_product<<<grid_for(e, units, 1, 1), kProdBlock, kProdSmem, e->s>>>(
+                             pa));
+  const int gr = (int)e->sms * (pa.dk >= 16 ? 1 : 2);
+#define GDL_PROD_ROWS(V) \
+  PLAUNCH(kc, kPJoinMat, k_join_product_rows<V><<<gr, kProdRowsBlock, 0, e->s>>>(pa))
+  switch (pa.dk) {
+    case 12: GDL_PROD_ROWS(1); break;
+    case 13: GDL_PROD_ROWS(2); break;
+    case 14: GDL_PROD_ROWS(4); break;
+    case 15: GDL_PROD_ROWS(8); break;
+    default: GDL_PROD_ROWS(16); break;
+  }
+#undef GDL_PROD_ROWS
 }
 
 // The sorted key list of a square-domain bitmap of `words` words (rows of
@@ -1459,6 +1477,327 @@ gdl_hook_work hook_work(gdl_engine *e, const OpHost &op, JoinRec *rec, const DAr
   return w;
 }
 
+// An ACopy that swaps its columns, NEWT bitmap to NEWT bitmap: a transpose.
+bool swap_acopy(const gdl_engine *e, const LieHost &L, const OpHost &op) {
+  return L.dk >= kPullMinBits && e->h[op.inner].bmG && e->h[op.out].bmG && !e->h[op.out].dirty &&
+         op.inner != op.out && op.sel.s0 == 1 && op.sel.s1 == 0;
+}
+
+// The descriptors of join oi (zeroed first: argument bytes, padding
+// included, are compared by the executable cache).
+JoinArgs join_args(gdl_engine *e, LieHost &L, const Plan &plan, size_t oi) {
+  const OpHost &op = L.ops[oi];
+  RelDev *R = e->d_rels;
+  const bool dense = L.dense;
+  const u64 words = dense ? L.map.words : 0;
+  JoinArgs a;
+  memset(&a, 0, sizeof a);
+  const RelDev &oh = e->h[op.outer];
+  if (op.outer_ver == GDL_DELTA) {
+    a.outer = &R[op.outer].delta;
+    a.outer_vis = &R[op.outer].w_delta_vis;
+  } else if (op.outer_ver == GDL_FULL) {
+    a.outer = &R[op.outer].full;
+    a.outer_vis = &R[op.outer].w_full_vis;
+  } else {
+    a.outer = &R[op.outer].newt;
+    a.outer_vis = nullptr;
+    if (dense && oh.bmG && plan.pull[oi]) {
+      // pull form: NEWT's bitmap transposed, its size counted (no list)
+      a.outer_bm = oh.bmG;
+      a.outer_bm_words = words;
+    } else if (dense && oh.bmG) {
+      a.outer_bm = oh.bmG;
+      a.outer_bm_words = words;
+    }
+  }
+  if (op.inner_ver == GDL_DELTA) {
+    a.inner = &R[op.inner].delta;
+    a.inner_vis = &R[op.inner].w_delta_vis;
+    a.inner_idx = &R[op.inner].delta_idx;
+  } else {  // FULL (a NEWT inner reads FULL, src/join.cu:14-19)
+    a.inner = &R[op.inner].full;
+    a.inner_vis = &R[op.inner].w_full_vis;
+    a.inner_idx = &R[op.inner].full_idx;
+  }
+  a.out_newt = &R[op.out].newt;
+  a.sel = op.sel;
+  a.generic = op.generic;
+  a.gen = op.gen;
+  a.gen.k2 = e->k2;
+  a.pred = op.pred;
+  a.op = L.d_joinrec + oi;
+  a.rec = &e->recs[0];
+  a.lb_cnt = e->lb_cnt;
+  a.lb_nz = e->lb_nz;
+  a.crow_off = e->crow_off;
+  a.crow_start = e->crow_start;
+  a.crow_len = e->crow_len;
+  a.crow_key = e->crow_key;
+  a.crow_cap = e->crow_cap;
+  a.ctl = e->d_ctl;
+  a.out_rel = op.out;
+  a.dense = dense;
+  // Row-OR: inner FULL kept as a bitmap, output (outer column, inner
+  // column 1), no predicate (dense.cuh, k_join_bm).
+  a.inner_rd = &R[op.inner];
+  a.row_or = dense && e->row_or_joins && op.inner_ver != GDL_DELTA &&
+             e->h[op.inner].dense && e->h[op.inner].bmF && op.pred.kind == 0 &&
+             (op.sel.s0 == 2 || op.sel.s0 == 3) && op.sel.s1 == 1;
+  return a;
+}
+
+// A row-gather join (pull.cuh, k_join_rows_bm).
+RowsArgs rows_args(gdl_engine *e, LieHost &L, const Plan &plan, size_t oi, const JoinArgs &a) {
+  const OpHost &op = L.ops[oi];
+  RelDev *R = e->d_rels;
+  const RelDev &oh = e->h[op.outer], &out = e->h[op.out];
+  RowsArgs ra;
+  memset(&ra, 0, sizeof ra);
+  memcpy(&ra.j, &a, sizeof a);
+  ra.j.rec = &e->recs[6];
+  ra.O = op.outer_ver == GDL_DELTA ? oh.bmDN : op.outer_ver == GDL_FULL ? oh.bmF : oh.bmG;
+  ra.outer_clear = op.outer_ver == GDL_NEWT ? oh.bmG : nullptr;
+  ra.outer_words = L.map.words;
+  ra.clear_diag = op.pred.kind == GDL_PRED_NE;
+  if (plan.static_once[oi]) {
+    ra.j.once = &L.d_lie->jonce[oi];
+    ra.j.once_pending = &L.d_lie->jonce_pending[oi];
+    ra.j.produced = &L.d_lie->produced[oi];
+    ra.j.phantom = &R[op.out].newt_phantom;
+  }
+  const RelHost &ih = e->rels[op.inner];
+  ra.inv_keys = ih.inv_keys;
+  ra.inv_ys = ih.inv_ys;
+  ra.inv_off = ih.inv_off;
+  ra.unit = (u32)e->rows_piece;
+  ra.dst = plan.out_twin[oi] ? out.bmOT : out.bmG;
+  ra.dirty = plan.out_twin[oi] ? nullptr : out.dirty;
+  ra.dst_zero = plan.twin_zero[oi] || plan.g_zero[oi];
+  ra.dk = L.dk;
+  return ra;
+}
+
+// A boolean product (product.cuh).
+ProdArgs product_args(gdl_engine *e, LieHost &L, const Plan &plan, size_t oi, const JoinArgs &a) {
+  const OpHost &op = L.ops[oi];
+  const RelDev &oh = e->h[op.outer], &out = e->h[op.out];
+  ProdArgs pa;
+  memset(&pa, 0, sizeof pa);
+  memcpy(&pa.j, &a, sizeof a);
+  pa.j.rec = &e->recs[6];
+  pa.OT = op.outer_ver == GDL_NEWT ? oh.bmGT : oh.bmDT;
+  pa.F = e->h[op.inner].bmF;
+  pa.rows_rec = &e->recs[9];
+  pa.G = plan.pull_t[oi] ? out.bmOT : out.bmG;
+  pa.dirty = plan.pull_t[oi] ? nullptr : out.dirty;
+  pa.dk = L.dk;
+  pa.side = L.side;
+  pa.splits = prod_small_splits(L.side);
+  return pa;
+}
+
+// Whether the loop of this LIE runs as one resident kernel (loop.cuh).
+bool resident_loop(const gdl_engine *e, const LieHost &L, const Plan &plan) {
+  if (!L.dense || e->instances || e->pull_joins != 2 || L.dk < kPullMinBits ||
+      L.dk > kLoopMaxBits || L.ops.size() > kMaxOps)
+    return false;
+  for (size_t oi = 0; oi < L.ops.size(); oi++) {
+    const OpHost &op = L.ops[oi];
+    if (op.hook) return false;
+    if (op.kind == 0 && plan.pull[oi] &&
+        (L.dk >= kProdTableBits ? plan.rows[oi] : plan.product[oi]))
+      continue;
+    if (op.kind == 2 && swap_acopy(e, L, op)) continue;
+    return false;
+  }
+  for (int r : L.update)
+    if (!plan.fused[r] || plan.delta_idx[r]) return false;
+  for (auto *v : {&L.update, &L.tmps})
+    for (int r : *v)
+      if (e->h[r].dirty) return false;
+  return true;
+}
+
+// The resident loop's steps and update list, in device memory.  A step's
+// level is one past the last earlier step it conflicts with.  A relation's
+// transposed twin is folded into its NEWT once, before the first step that
+// reads that NEWT (or the update step).
+gdl_status push_loop(gdl_engine *e, LieHost &L, const Plan &plan) {
+  struct Use {
+    std::vector<const void *> reads, ors, writes;
+  };
+  std::vector<LoopStep> steps;
+  std::vector<Use> uses;
+  auto meets = [](const std::vector<const void *> &x, const std::vector<const void *> &y) {
+    for (const void *p : x)
+      for (const void *q : y)
+        if (p && p == q) return true;
+    return false;
+  };
+  auto add = [&](LoopStep st, Use u) {
+    st.level = 0;
+    for (size_t k = 0; k < steps.size(); k++) {
+      const Use &v = uses[k];
+      if (meets(u.reads, v.ors) || meets(u.reads, v.writes) || meets(u.ors, v.reads) ||
+          meets(u.ors, v.writes) || meets(u.writes, v.reads) || meets(u.writes, v.ors) ||
+          meets(u.writes, v.writes))
+        st.level = std::max(st.level, steps[k].level + 1);
+    }
+    steps.push_back(st);
+    uses.push_back(std::move(u));
+  };
+  auto blank = [](int kind) {
+    LoopStep st;
+    memset(&st, 0, sizeof st);
+    st.kind = kind;
+    return st;
+  };
+  std::vector<char> twin_full(e->rels.size(), 0);  // twin written and not folded yet
+  auto fold = [&](int r) {
+    if (!twin_full[r]) return;
+    twin_full[r] = 0;
+    LoopStep st = blank(kLoopFold);
+    st.src = e->h[r].bmOT;
+    st.dst = e->h[r].bmG;
+    add(st, Use{{}, {}, {st.src, st.dst}});
+  };
+  for (size_t oi = 0; oi < L.ops.size(); oi++) {
+    const OpHost &op = L.ops[oi];
+    const RelDev &out = e->h[op.out];
+    if (op.kind == 2) {
+      fold(op.inner);
+      twin_full[op.out] = 0;  // (the copy replaces NEWT)
+      LoopStep st = blank(kLoopTranspose);
+      st.src = e->h[op.inner].bmG;
+      st.dst = out.bmG;
+      add(st, Use{{st.src}, {}, {st.dst, out.bmOT}});
+      continue;
+    }
+    const JoinArgs a = join_args(e, L, plan, oi);
+    if (op.outer_ver == GDL_NEWT) fold(op.outer);
+    LoopStep st = blank(plan.rows[oi] ? kLoopRows : kLoopProduct);
+    st.outer = a.outer;
+    st.inner = a.inner;
+    st.outer_vis = a.outer_vis;
+    st.inner_vis = a.inner_vis;
+    st.outer_bm = a.outer_bm;
+    st.outer_words = a.outer_bm_words;
+    st.outer_rel = op.outer;
+    if (plan.rows[oi]) {
+      if (plan.out_twin[oi]) fold(op.out);  // (it may expect a zero twin)
+      const RowsArgs ra = rows_args(e, L, plan, oi, a);
+      st.src = ra.O;
+      st.dst = ra.dst;
+      st.inv_keys = ra.inv_keys;
+      st.inv_ys = ra.inv_ys;
+      st.n_edges = (u32)e->rels[op.inner].inv_n;
+      // few edges a warp: units of four, one group of rows in flight
+      st.unit = st.n_edges < (u64)e->sms * 16 * 8 ? 8 : ra.unit;
+      st.dst_zero = ra.dst_zero;
+      st.clear_diag = ra.clear_diag;
+      st.once = ra.j.once;
+      st.once_pending = ra.j.once_pending;
+      st.produced = ra.j.produced;
+      st.phantom = ra.j.phantom;
+      add(st, Use{{st.src, st.inner, st.inner_vis},
+                  {},
+                  {st.dst, st.outer, st.outer_vis, st.outer_bm}});
+    } else {
+      if (op.outer_ver == GDL_NEWT) {
+        LoopStep t = blank(kLoopTranspose);
+        t.src = e->h[op.outer].bmG;
+        t.dst = e->h[op.outer].bmGT;
+        t.count_to = &e->d_rels[op.outer].newt;
+        t.count_acc = &e->d_rels[op.outer].scan.pop_g;
+        add(t, Use{{t.src}, {}, {t.dst, t.count_to}});
+      }
+      const ProdArgs pa = product_args(e, L, plan, oi, a);
+      st.src = pa.OT;
+      st.F = pa.F;
+      st.dst = pa.G;
+      // (a DELTA outer zeroed by an empty inner: in operator order within a
+      // level, published at its end)
+      Use u{{st.src, st.F, st.inner, st.inner_vis}, {st.dst}, {}};
+      if (!st.outer_vis) u.writes = {st.outer, st.outer_bm};
+      add(st, u);
+    }
+    if (plan.out_twin[oi] && !plan.fold_late[op.out]) twin_full[op.out] = 1;
+  }
+  for (int r : L.update) fold(r);
+  for (int r : L.tmps) fold(r);  // (leaves the twin zero)
+  std::stable_sort(steps.begin(), steps.end(),
+                   [](const LoopStep &x, const LoopStep &y) { return x.level < y.level; });
+  bool fits = steps.size() <= (size_t)kLoopMaxSteps &&
+              L.update.size() + L.tmps.size() <= (size_t)kLoopMaxUpd;
+  for (size_t i = 0, j = 0; i < steps.size(); i = j) {
+    while (j < steps.size() && steps[j].level == steps[i].level) j++;
+    for (size_t k = i; k < j; k++) steps[k].level_end = (int)j;
+    fits = fits && j - i <= 32;
+  }
+  if (!fits) {
+    L.resident = false;
+    return GDL_OK;
+  }
+  std::vector<LoopUpd> upd;
+  for (int r : L.update) {
+    const RelDev &h = e->h[r];
+    LoopUpd u;
+    memset(&u, 0, sizeof u);
+    u.rd = &e->d_rels[r];
+    u.F = h.bmF;
+    u.G = h.bmG;
+    u.gt = plan.fold_late[r] ? h.bmOT : nullptr;
+    u.dn = plan.delta_n[r] ? h.bmDN : nullptr;
+    u.dt = plan.delta_t[r] ? h.bmDT : nullptr;
+    // (a relation with the fused update step keeps no dirty map: its bytes
+    // hold the tile flags, zero at LIE start)
+    u.clean = h.bmD;
+    upd.push_back(u);
+  }
+  for (int r : L.tmps) {
+    LoopUpd u;
+    memset(&u, 0, sizeof u);
+    u.G = e->h[r].bmG;
+    upd.push_back(u);
+  }
+  if (!L.d_steps) TRY(dalloc(e, (void **)&L.d_steps, kLoopMaxSteps * sizeof(LoopStep)));
+  if (!L.d_upd) TRY(dalloc(e, (void **)&L.d_upd, kMaxRels * sizeof(LoopUpd)));
+  CK(e, cudaMemcpyAsync(L.d_steps, steps.data(), steps.size() * sizeof(LoopStep),
+                        cudaMemcpyHostToDevice, e->s));
+  CK(e, cudaMemcpyAsync(L.d_upd, upd.data(), upd.size() * sizeof(LoopUpd), cudaMemcpyHostToDevice,
+                        e->s));
+  L.n_steps = (int)steps.size();
+  L.n_upd = (int)upd.size();
+  return GDL_OK;
+}
+
+// The resident loop as the graph body's one launch.  Two blocks an SM at
+// most (all resident); fewer where a domain has less work than that (a
+// barrier's cost grows with its blocks).
+cudaError_t launch_loop(gdl_engine *e, LieHost &L, Counts *kc) {
+  LoopArgs a;
+  memset(&a, 0, sizeof a);
+  a.steps = L.d_steps;
+  a.upd = L.d_upd;
+  a.n_steps = L.n_steps;
+  a.n_upd = L.n_upd;
+  a.dk = L.dk;
+  a.side = L.side;
+  a.splits = prod_small_splits(L.side);
+  a.rels = e->d_rels;
+  a.lie = L.d_lie;
+  a.ctl = e->d_ctl;
+  const void *f = L.dk < 12    ? (const void *)k_lie_loop<0>
+                  : L.dk == 12 ? (const void *)k_lie_loop<1>
+                               : (const void *)k_lie_loop<2>;
+  const u64 warps = L.dk < 12 ? (u64)L.side * 256 * prod_small_splits(L.side) : ~0ull / 16;
+  const int g = grid_for(e, warps, 8, 2);
+  void *args[] = {&a};
+  kc->add(kPControl);
+  return cudaLaunchCooperativeKernel(f, dim3(g), dim3(kLoopBlock), args, 0, e->s);
+}
+
 void enqueue_iteration(gdl_engine *e, LieHost &L, const Plan &plan, Counts *kc, bool in_graph) {
   cudaStream_t s = e->s;
   RelDev *R = e->d_rels;
@@ -1469,70 +1808,22 @@ void enqueue_iteration(gdl_engine *e, LieHost &L, const Plan &plan, Counts *kc, 
   for (size_t oi = 0; oi < L.ops.size(); oi++) {
     const OpHost &op = L.ops[oi];
     if (op.kind == 0) {
+      const JoinArgs a0 = join_args(e, L, plan, oi);
       JoinArgs a;
-      memset(&a, 0, sizeof a);
+      memcpy(&a, &a0, sizeof a);
       const RelDev &oh = e->h[op.outer];
-      if (op.outer_ver == GDL_DELTA) {
-        a.outer = &R[op.outer].delta;
-        a.outer_vis = &R[op.outer].w_delta_vis;
-      } else if (op.outer_ver == GDL_FULL) {
-        a.outer = &R[op.outer].full;
-        a.outer_vis = &R[op.outer].w_full_vis;
-      } else {
-        a.outer = &R[op.outer].newt;
-        a.outer_vis = nullptr;
-        if (dense && oh.bmG && plan.pull[oi]) {
-          // pull form: NEWT's bitmap transposed, its size counted (no list)
-          a.outer_bm = oh.bmG;
-          a.outer_bm_words = words;
-        } else if (dense && oh.bmG) {
-          // NEWT as a join outer: the sorted list of its bitmap (dirty
-          // chunks only).
-          BmScanArgs c = scan_none(map);
-          c.g = oh.bmG;
-          c.dirty = oh.dirty;
-          c.skip_clean = oh.dirty != nullptr;
-          c.ex_a = kBmUnion;
-          c.list_a = &R[op.outer].newt;
-          c.need_a = need_index(op.outer, kNeedNewt);
-          launch_scan(e, c, op.outer, kc);
-          a.outer_bm = oh.bmG;
-          a.outer_bm_words = words;
-        }
+      if (op.outer_ver == GDL_NEWT && dense && oh.bmG && !plan.pull[oi]) {
+        // NEWT as a join outer: the sorted list of its bitmap (dirty chunks
+        // only).
+        BmScanArgs c = scan_none(map);
+        c.g = oh.bmG;
+        c.dirty = oh.dirty;
+        c.skip_clean = oh.dirty != nullptr;
+        c.ex_a = kBmUnion;
+        c.list_a = &R[op.outer].newt;
+        c.need_a = need_index(op.outer, kNeedNewt);
+        launch_scan(e, c, op.outer, kc);
       }
-      if (op.inner_ver == GDL_DELTA) {
-        a.inner = &R[op.inner].delta;
-        a.inner_vis = &R[op.inner].w_delta_vis;
-        a.inner_idx = &R[op.inner].delta_idx;
-      } else {  // FULL (a NEWT inner reads FULL, src/join.cu:14-19)
-        a.inner = &R[op.inner].full;
-        a.inner_vis = &R[op.inner].w_full_vis;
-        a.inner_idx = &R[op.inner].full_idx;
-      }
-      a.out_newt = &R[op.out].newt;
-      a.sel = op.sel;
-      a.generic = op.generic;
-      a.gen = op.gen;
-      a.gen.k2 = e->k2;
-      a.pred = op.pred;
-      a.op = L.d_joinrec + oi;
-      a.rec = &e->recs[0];
-      a.lb_cnt = e->lb_cnt;
-      a.lb_nz = e->lb_nz;
-      a.crow_off = e->crow_off;
-      a.crow_start = e->crow_start;
-      a.crow_len = e->crow_len;
-      a.crow_key = e->crow_key;
-      a.crow_cap = e->crow_cap;
-      a.ctl = e->d_ctl;
-      a.out_rel = op.out;
-      a.dense = dense;
-      // Row-OR: inner FULL kept as a bitmap, output (outer column, inner
-      // column 1), no predicate (dense.cuh, k_join_bm).
-      a.inner_rd = &R[op.inner];
-      a.row_or = dense && e->row_or_joins && op.inner_ver != GDL_DELTA &&
-                 e->h[op.inner].dense && e->h[op.inner].bmF && op.pred.kind == 0 &&
-                 (op.sel.s0 == 2 || op.sel.s0 == 3) && op.sel.s1 == 1;
       if (op.hook) {
         // The count pass enumerates the candidates; the caller's kernel runs
         // the hooks over them and appends what it keeps.
@@ -1555,30 +1846,8 @@ void enqueue_iteration(gdl_engine *e, LieHost &L, const Plan &plan, Counts *kc, 
       }
       if (plan.pull[oi] && plan.rows[oi]) {
         // gathered along the inner's in-edges from the outer's rows
-        RowsArgs ra;
-        memset(&ra, 0, sizeof ra);
-        ra.j = a;
-        ra.j.rec = &e->recs[6];
-        ra.O = op.outer_ver == GDL_DELTA ? oh.bmDN : op.outer_ver == GDL_FULL ? oh.bmF : oh.bmG;
-        ra.outer_clear = op.outer_ver == GDL_NEWT ? oh.bmG : nullptr;
-        ra.outer_words = words;
-        ra.clear_diag = op.pred.kind == GDL_PRED_NE;
-        if (plan.static_once[oi]) {
-          ra.j.once = &L.d_lie->jonce[oi];
-          ra.j.once_pending = &L.d_lie->jonce_pending[oi];
-          ra.j.produced = &L.d_lie->produced[oi];
-          ra.j.phantom = &R[op.out].newt_phantom;
-        }
-        const RelHost &ih = e->rels[op.inner];
-        ra.inv_keys = ih.inv_keys;
-        ra.inv_ys = ih.inv_ys;
-        ra.inv_off = ih.inv_off;
-        ra.unit = (u32)e->rows_piece;
+        const RowsArgs ra = rows_args(e, L, plan, oi, a);
         const RelDev &out = e->h[op.out];
-        ra.dst = plan.out_twin[oi] ? out.bmOT : out.bmG;
-        ra.dirty = plan.out_twin[oi] ? nullptr : out.dirty;
-        ra.dst_zero = plan.twin_zero[oi] || plan.g_zero[oi];
-        ra.dk = L.dk;
         launch_rows(e, ra, kc);
         if (plan.out_twin[oi] && !plan.fold_late[op.out])
           launch_fold(e, out.bmOT, out.bmG, out.dirty, L.dk, L.side,
@@ -1599,15 +1868,7 @@ void enqueue_iteration(gdl_engine *e, LieHost &L, const Plan &plan, Counts *kc, 
         if (plan.product[oi]) {
           // the inner is a FULL kept as a bitmap: a boolean product
           const RelDev &out = e->h[op.out];
-          ProdArgs pa;
-          memset(&pa, 0, sizeof pa);
-          memcpy(&pa.j, &a, sizeof a);
-          pa.OT = OT;
-          pa.F = e->h[op.inner].bmF;
-          pa.G = plan.pull_t[oi] ? out.bmOT : out.bmG;
-          pa.dirty = plan.pull_t[oi] ? nullptr : out.dirty;
-          pa.dk = L.dk;
-          pa.side = L.side;
+          ProdArgs pa = product_args(e, L, plan, oi, a);
           launch_product(e, pa, kc);
           if (plan.pull_t[oi] && !plan.fold_late[op.out])
             launch_fold(e, out.bmOT, out.bmG, out.dirty, L.dk, L.side,
@@ -1714,8 +1975,7 @@ void enqueue_iteration(gdl_engine *e, LieHost &L, const Plan &plan, Counts *kc, 
       if (dense && op.kind == 2) {
         // RelationalACopy: dest NEWT := sel(src NEWT), bitmap to bitmap.
         const u64 tiles = words / kBmTileWords;
-        if (L.dk >= kPullMinBits && sh.bmG && !e->h[op.out].dirty && op.inner != op.out &&
-            op.sel.s0 == 1 && op.sel.s1 == 0) {
+        if (swap_acopy(e, L, op)) {
           // (src[1], src[0]): the source's NEWT transposed, every word of
           // the destination's NEWT written
           TransposeArgs t = transpose_args(sh.bmG, nullptr, e->h[op.out].bmG, L.dk, L.side,
@@ -2078,9 +2338,14 @@ gdl_status build_graph(gdl_engine *e, LieHost &L, const Plan &plan) {
                                     cudaStreamCaptureModeThreadLocal);
   Counts kc;
   if (r == cudaSuccess) {
-    enqueue_iteration(e, L, plan, &kc, true);
+    cudaError_t lr = cudaSuccess;
+    if (L.resident)
+      lr = launch_loop(e, L, &kc);
+    else
+      enqueue_iteration(e, L, plan, &kc, true);
     cudaGraph_t captured = nullptr;
     r = cudaStreamEndCapture(e->s, &captured);
+    if (r == cudaSuccess) r = lr;
   }
   if (r != cudaSuccess) {
     cudaGraphDestroy(g);
@@ -2572,6 +2837,8 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
   L.kernels = 0;
   L.graph_dirty = true;
   const bool use_graph = getenv("GDLOG_NO_GRAPH") == nullptr && !e->profile;
+  L.resident = use_graph && resident_loop(e, L, plan);
+  if (L.resident) TRY(push_loop(e, L, plan));
   u64 batch = 4;
   bool first_batch = true;
   bool tail_listed = false;
@@ -2623,7 +2890,8 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
     // and instantiates the graph for the iterations after it; when that
     // iteration already ended the loop (and the host sees it), no graph
     // launch follows.
-    const bool pre = use_graph && L.graph_dirty && first_batch;
+    // (A resident loop runs its first iteration too.)
+    const bool pre = use_graph && L.graph_dirty && first_batch && !L.resident;
     first_batch = false;
     Counts pre_kc;
     if (pre) {
@@ -2704,6 +2972,7 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
     } else if (use_graph) {
       bodies = 0;
     }
+    if (L.resident) bodies = 1;
     L.kernels += bodies * (u64)L.per_iter.total;
     for (int k = 0; k < kPKinds; k++) e->prof_launches[k] += bodies * (u64)L.per_iter.kind[k];
     if (L.trace_on && ran) {
@@ -3056,12 +3325,8 @@ gdl_status gdl_engine_create(int32_t device, void *stream, gdl_engine **out) {
                                (int)sort_smem_bytes<10>())) ||
       bad(cudaFuncSetAttribute(k_merge_diff, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kMergeSmemBytes)) ||
-      bad(cudaFuncSetAttribute(k_join_product<kProdBigRows, true>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)prod_smem(true))) ||
-      bad(cudaFuncSetAttribute(k_join_product<kProdSmallRows, false>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)prod_smem(false))) ||
+      bad(cudaFuncSetAttribute(k_join_product, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)kProdSmem)) ||
       bad(cudaFuncSetAttribute(k_join_pull_bm, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)(pull_acc_words(16) * 4))) ||
       bad(cudaMalloc(&e->d_rels, kMaxRels * sizeof(RelDev))) ||
@@ -3130,7 +3395,8 @@ static void release_program(gdl_engine *e) {
   for (LieHost &L : e->lies) {
     release_graph(e, L);
     // stream-ordered frees (a cudaFree would wait for the whole device)
-    for (void *p : {(void *)L.d_trace, (void *)L.d_lie, (void *)L.d_joinrec})
+    for (void *p : {(void *)L.d_trace, (void *)L.d_lie, (void *)L.d_joinrec, (void *)L.d_steps,
+                    (void *)L.d_upd})
       dfree(e, p);
     dfree(e, L.d_inst_delta);
     dfree(e, L.d_inst_last);

@@ -90,8 +90,11 @@ __device__ __forceinline__ u64 join_out(const JoinArgs &a, u64 inner, u64 outer)
   return a.generic ? gen_spec(a.gen, inner, outer, &a.ctl->oob) : gen_join(a.sel, inner, outer);
 }
 
+// (both words load at once)
 __device__ __forceinline__ u64 eff_count(const DArr *a, const u32 *vis) {
-  return (vis && *vis == 0) ? 0 : a->n;
+  const u64 n = a->n;
+  const u32 v = vis ? *vis : 1u;
+  return v ? n : 0;
 }
 
 // src/join.cu:38-45: either side empty -> no output, and the OUTER's

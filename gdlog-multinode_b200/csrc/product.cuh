@@ -7,26 +7,38 @@
 // (test/cspa.cu:279-352) spends its time in nine such products of relations
 // that fill a fifth to nine tenths of their domain; listing the inner,
 // indexing it and expanding candidate tuples cost 11 ms a join at 20,000
-// ids.  Here no list and no index exist: a block owns MR output rows by a
-// slice of 1024 columns (a word a lane, MR / 16 rows a warp, accumulated in
-// registers) and walks the keys 32 at a time.
+// ids.  Here no list and no index exist.
 //
-// Per 32 keys (one word of each row of OT), by the bits its rows hold:
+// k_join_product: a block owns MR output rows by a slice of 1024 columns (a
+// word a lane, MR / 16 rows a warp, accumulated in registers) and walks the
+// keys 32 at a time.  Per 32 keys (one word of each row of OT), by the bits
+// its rows hold:
 //   * many: the four-Russians method (Arlazarov, Dinic, Kronrod, Faradzev
 //     1970).  For each of the word's four bytes the 256 ORs of its eight
 //     inner rows are tabled in shared memory (1024 entries of 128 bytes,
 //     built from registers, a store an entry), and a row takes four table
 //     reads instead of one read per key.
 //   * few: the row's keys one by one from the inner rows staged in shared
-//     memory.
+//     memory, rows without a key skipped by a ballot.
 //   * none, or no inner row with bits in the slice: skipped.
-// The bound is shared-memory bandwidth: one 128-byte read a row and byte of
+// The bound is shared-memory bandwidth, one 128-byte read a row and byte of
 // keys, so MR = 1024 rows share a table (its 1024 stores are a fifth of the
-// 4096 + 256 reads).  The next 256 keys' operands load (cp.async for the
-// inner's rows, registers for the outer's words) while these are used.
+// 4096 + 512 reads).  The integer pipe comes second: the outer's words are
+// staged as their bytes' table offsets (two a word, byte * 128), so an
+// address is one instruction, and rows are taken four at a time without a
+// branch.  The next 256 keys' operands load (cp.async for the inner's rows,
+// registers for the outer's words) while these are used.
 //
-// Small domains (below 2^kProdTableBits ids) have too few rows to fill the
-// GPU with tables: blocks of 64 rows, keys one by one, several blocks an SM.
+// k_join_product_rows: an outer of few tuples (their inner rows within
+// kProdRowsBytes) would leave that kernel scanning empty words for every
+// slice.  A block takes 8 rows of OT, lists their keys in shared memory and
+// its warps OR equal shares of the listed inner rows, whole rows at a time.
+// Both kernels are launched; the device-side tuple count picks one.
+//
+// product_small: below 2^kProdTableBits ids there are too few rows to fill
+// the GPU with tables.  A warp takes one output row and a share of its keys
+// and ORs the inner's rows straight from L1 / L2, four keys' loads in flight
+// (at 512 ids two keys a load instruction, at 256 four).
 #pragma once
 
 #include "common.cuh"
@@ -39,17 +51,15 @@ constexpr int kProdBlock = 512;
 constexpr int kProdWarps = kProdBlock / 32;
 constexpr int kProdStep = 256;       // keys per staged step: 8 words of a row
 constexpr int kProdTableBits = 12;   // tables from 2^12 ids on
-constexpr int kProdBigRows = 64;     // rows per warp with tables
-constexpr int kProdSmallRows = 4;    // ... and without
+constexpr int kProdWarpRows = 64;    // output rows per warp
+constexpr u32 kProdRows = kProdWarps * kProdWarpRows;  // per block
+constexpr int kProdPart = 4;         // words of a step staged together
+// inner row bytes below which the outer's keys are listed
+constexpr u64 kProdRowsBytes = 1ull << 30;
 
-__host__ __device__ constexpr u32 prod_rows(bool tables) {
-  return kProdWarps * (tables ? kProdBigRows : kProdSmallRows);
-}
-// dynamic shared memory: the tables, two stages of 256 inner row slices, and
-// the outer's words [8][rows]
-__host__ __device__ constexpr u32 prod_smem(bool tables) {
-  return (tables ? 4 * 256 * 128 : 0) + 2 * kProdStep * 128 + 8 * prod_rows(tables) * 4;
-}
+// Dynamic shared memory: the tables, two stages of 256 inner row slices, and
+// kProdPart of a step's 8 outer words, as two words each.
+constexpr u32 kProdSmem = 4 * 256 * 128 + 2 * kProdStep * 128 + 2 * kProdPart * kProdRows * 4;
 
 struct ProdArgs {
   JoinArgs j;      // descriptors for the emptiness rules, launch record, ctl
@@ -57,9 +67,11 @@ struct ProdArgs {
   const u32 *F;    // the inner's rows
   u32 *G;          // output rows: the output's NEWT or its transposed twin
   u8 *dirty;       // dirty map of G, or null
+  LaunchRec *rows_rec;  // launch record of k_join_product_rows
   int dk;          // rows of 2^(dk-5) words
   u32 side;        // 256-id groups that hold ids
   u32 ksteps;      // groups per unit of work (the key range is split)
+  u32 splits;      // product_small: warps a row's keys are shared among
 };
 
 __device__ __forceinline__ void cp_async16(void *dst, const void *src, u32 bytes) {
@@ -69,24 +81,50 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src, u32 bytes
                : "memory");
 }
 
-template <int RW, bool TAB>
-__global__ void __launch_bounds__(kProdBlock, TAB ? 1 : 2) k_join_product(ProdArgs a) {
-  constexpr u32 MR = kProdWarps * RW;
-  constexpr int RPT = MR >= kProdBlock ? MR / kProdBlock : 1;  // outer rows loaded per thread
+// src/join.cu:38-45 for a product: an empty inner empties the OUTER (every
+// block calls this; a NEWT outer's bitmap is cleared too).  Returns whether
+// there is nothing to join.  The inner is looked at first: no block reads
+// the outer's count while block 0 may be zeroing it.
+__device__ __forceinline__ bool product_empty(const JoinArgs &j, u64 *n_outer) {
+  if (eff_count(j.inner, j.inner_vis) == 0) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      if (j.outer_vis)
+        *j.outer_vis = 0;
+      else
+        ((DArr *)j.outer)->n = 0;
+    }
+    if (!j.outer_vis && j.outer_bm) {
+      uint4 *p = reinterpret_cast<uint4 *>(j.outer_bm);
+      for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < j.outer_bm_words / 4;
+           i += (u64)gridDim.x * blockDim.x)
+        p[i] = make_uint4(0, 0, 0, 0);
+    }
+    return true;
+  }
+  *n_outer = eff_count(j.outer, j.outer_vis);
+  return *n_outer == 0;
+}
+
+__device__ __forceinline__ bool prod_lists_keys(const ProdArgs &a, u64 n_outer) {
+  return a.dk >= kProdTableBits && n_outer * a.side * 32 <= kProdRowsBytes;
+}
+
+__global__ void __launch_bounds__(kProdBlock, 1) k_join_product(ProdArgs a) {
+  constexpr int RW = kProdWarpRows;
+  constexpr u32 MR = kProdRows;
+  constexpr int RPT = MR / kProdBlock;  // outer rows loaded per thread
+  constexpr int kPart = kProdPart;
   extern __shared__ __align__(128) u32 prod_mem[];
   u32 *tab = prod_mem;
-  u32 *sB = tab + (TAB ? 4 * 256 * 32 : 0);
+  u32 *sB = tab + 4 * 256 * 32;
   u32 *sA = sB + 2 * kProdStep * 32;
   __shared__ u32 s_cnt[2][8];            // bits of the outer per word of keys
   __shared__ u32 s_half[kProdWarps];     // inner rows with bits, 16 a warp
   __shared__ long long s_unit;
   if (ctl_stop(a.j.ctl)) return;
-  const u64 n_outer = eff_count(a.j.outer, a.j.outer_vis);
-  const u64 n_inner = eff_count(a.j.inner, a.j.inner_vis);
-  if (n_outer == 0 || n_inner == 0) {
-    join_empty_side(a.j, n_outer);
-    return;
-  }
+  u64 n_outer;
+  if (product_empty(a.j, &n_outer)) return;
+  if (prod_lists_keys(a, n_outer)) return;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int rs = a.dk - 5;
   const u32 row_words = 1u << rs;
@@ -111,7 +149,7 @@ __global__ void __launch_bounds__(kProdBlock, TAB ? 1 : 2) k_join_product(ProdAr
 #pragma unroll
       for (int i = 0; i < RPT; i++) {
         const u32 lr = tid + i * kProdBlock, row = rb * MR + lr;
-        if (lr < MR && row < ids) {
+        if (row < ids) {
           load8(a.OT + ((u64)row << rs) + s * 8, av[i]);
         } else {
 #pragma unroll
@@ -138,93 +176,120 @@ __global__ void __launch_bounds__(kProdBlock, TAB ? 1 : 2) k_join_product(ProdAr
       for (int w = 0; w < 8; w++) {
         u32 c = 0;
 #pragma unroll
-        for (int i = 0; i < RPT; i++) {
-          if (tid + i * kProdBlock < MR) sA[w * MR + tid + i * kProdBlock] = av[i][w];
-          c += __popc(av[i][w]);
-        }
+        for (int i = 0; i < RPT; i++) c += __popc(av[i][w]);
         c = __reduce_add_sync(0xffffffffu, c);
         if (lane == 0 && c) atomicAdd(&s_cnt[st][w], c);
       }
       asm volatile("cp.async.wait_group 0;" ::: "memory");
-      __syncthreads();  // the step's operands and counts
-      if (s + 1 < k1) {
-        load_a(s + 1);
-        load_b(s + 1, st ^ 1);
-      }
-      if (tid < 8) s_cnt[st ^ 1][tid] = 0;
       const u32 *B = sB + st * kProdStep * 32;
-      u32 any = 0;
 #pragma unroll
-      for (int w = 0; w < 8; w++) any |= s_cnt[st][w];
-      if (any) {  // (block-uniform)
-        u32 m = 0;
+      for (int part = 0; part < 8; part += kPart) {
+        // the outer's words of this part, as table offsets: bytes 0, 1 (times 128) in one word, bytes 2, 3 in the next
 #pragma unroll
-        for (int j = 0; j < 16; j++)
-          if (__any_sync(0xffffffffu, B[(wid * 16 + j) * 32 + lane] != 0u)) m |= 1u << j;
-        if (lane == 0) s_half[wid] = m;
-        __syncthreads();
-        for (int w = 0; w < 8; w++) {
-          const u32 cnt = s_cnt[st][w];
-          const u32 bm = s_half[2 * w] | (s_half[2 * w + 1] << 16);
-          if (cnt == 0 || bm == 0) continue;  // (block-uniform)
-          if (tid == 0) used += cnt;
-          const u32 *Bw = B + w * 32 * 32 + lane;
-          const uint4 *Aw = reinterpret_cast<const uint4 *>(sA + w * MR + wid * RW);
-          if (TAB && cnt > 2 * MR) {
-            {
-              // warp wid: byte wid / 4, the 64 entries with top bits wid % 4
-              const u32 *r = Bw + (wid >> 2) * 8 * 32;
-              u32 lo[8], hi[8];
-              lo[0] = 0;
-              lo[1] = r[0];
-              lo[2] = r[32];
-              lo[3] = lo[1] | lo[2];
-              const u32 r2 = r[64];
+        for (int w = 0; w < kPart; w++)
 #pragma unroll
-              for (int i = 0; i < 4; i++) lo[4 + i] = lo[i] | r2;
-              hi[0] = ((wid & 1) ? r[6 * 32] : 0u) | ((wid & 2) ? r[7 * 32] : 0u);
-              hi[1] = hi[0] | r[96];
-              const u32 r4 = r[128], r5 = r[160];
-              hi[2] = hi[0] | r4;
-              hi[3] = hi[1] | r4;
+          for (int i = 0; i < RPT; i++) {
+            const u32 lr = tid + i * kProdBlock, x = av[i][part + w];
+            reinterpret_cast<uint2 *>(sA)[w * MR + lr] =
+                make_uint2(((x & 0xFFu) << 7) | ((x & 0xFF00u) << 15),
+                           ((x >> 9) & 0x7F80u) | ((x >> 1) & 0x7F800000u));
+          }
+        __syncthreads();  // the step's operands and counts
+        if (part + kPart == 8 && s + 1 < k1) {
+          load_a(s + 1);
+          load_b(s + 1, st ^ 1);
+        }
+        u32 any = 0;
 #pragma unroll
-              for (int i = 0; i < 4; i++) hi[4 + i] = hi[i] | r5;
-              u32 *t = tab + ((wid >> 2) * 256 + (wid & 3) * 64) * 32 + lane;
+        for (int w = 0; w < 8; w++) any |= s_cnt[st][w];
+        if (any) {  // (block-uniform)
+          if (part == 0) {
+            u32 m = 0;
 #pragma unroll
-              for (int i = 0; i < 64; i++) t[i * 32] = lo[i & 7] | hi[i >> 3];
-            }
+            for (int j = 0; j < 16; j++)
+              if (__any_sync(0xffffffffu, B[(wid * 16 + j) * 32 + lane] != 0u)) m |= 1u << j;
+            if (lane == 0) s_half[wid] = m;
             __syncthreads();
-            const char *tb = reinterpret_cast<const char *>(tab);
+          }
+          for (int wp = 0; wp < kPart; wp++) {
+            const int w = part + wp;
+            const u32 cnt = s_cnt[st][w];
+            const u32 bm = s_half[2 * w] | (s_half[2 * w + 1] << 16);
+            if (cnt == 0 || bm == 0) continue;  // (block-uniform)
+            if (tid == 0) used += cnt;
+            const u32 *Bw = B + w * 32 * 32 + lane;
+            if (cnt > MR) {
+              {
+                // warp wid: byte wid / 4, the 64 entries with top bits wid % 4
+                const u32 *r = Bw + (wid >> 2) * 8 * 32;
+                u32 lo[8], hi[8];
+                lo[0] = 0;
+                lo[1] = r[0];
+                lo[2] = r[32];
+                lo[3] = lo[1] | lo[2];
+                const u32 r2 = r[64];
 #pragma unroll
-            for (int q = 0; q < RW / 4; q++) {
-              const uint4 x4 = Aw[q];
-              const u32 xs[4] = {x4.x, x4.y, x4.z, x4.w};
+                for (int i = 0; i < 4; i++) lo[4 + i] = lo[i] | r2;
+                hi[0] = ((wid & 1) ? r[6 * 32] : 0u) | ((wid & 2) ? r[7 * 32] : 0u);
+                hi[1] = hi[0] | r[96];
+                const u32 r4 = r[128], r5 = r[160];
+                hi[2] = hi[0] | r4;
+                hi[3] = hi[1] | r4;
 #pragma unroll
-              for (int i = 0; i < 4; i++) {
-                const u32 x = xs[i];
-                if (x) {
-                  const u32 t0 = *(const u32 *)(tb + (((x << 7) & 0x7f80u) | lane4));
-                  const u32 t1 = *(const u32 *)(tb + 32768 + (((x >> 1) & 0x7f80u) | lane4));
-                  const u32 t2 = *(const u32 *)(tb + 65536 + (((x >> 9) & 0x7f80u) | lane4));
-                  const u32 t3 = *(const u32 *)(tb + 98304 + (((x >> 17) & 0x7f80u) | lane4));
-                  acc[q * 4 + i] |= t0 | t1 | t2 | t3;
+                for (int i = 0; i < 4; i++) hi[4 + i] = hi[i] | r5;
+                u32 *t = tab + ((wid >> 2) * 256 + (wid & 3) * 64) * 32 + lane;
+#pragma unroll
+                for (int i = 0; i < 64; i++) t[i * 32] = lo[i & 7] | hi[i >> 3];
+              }
+              __syncthreads();
+              const char *tb = reinterpret_cast<const char *>(tab);
+              const uint4 *Aw = reinterpret_cast<const uint4 *>(sA) + (wp * MR + wid * RW) / 2;
+#pragma unroll
+              for (int q = 0; q < RW / 4; q++) {
+                const uint4 x0 = Aw[2 * q], x1 = Aw[2 * q + 1];
+                if (x0.x | x0.y | x0.z | x0.w | x1.x | x1.y | x1.z | x1.w) {
+                  const u32 xs[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+#pragma unroll
+                  for (int i = 0; i < 4; i++) {
+                    const u32 lo = xs[2 * i], hi = xs[2 * i + 1];
+                    const u32 t0 = *(const u32 *)(tb + ((lo & 0x7F80u) | lane4));
+                    const u32 t1 = *(const u32 *)(tb + 32768 + ((lo >> 16) + lane4));
+                    const u32 t2 = *(const u32 *)(tb + 65536 + ((hi & 0x7F80u) | lane4));
+                    const u32 t3 = *(const u32 *)(tb + 98304 + ((hi >> 16) + lane4));
+                    acc[q * 4 + i] |= t0 | t1 | t2 | t3;
+                  }
+                }
+              }
+              __syncthreads();  // the table is rebuilt for the next word
+            } else {
+              const uint2 *Aw = reinterpret_cast<const uint2 *>(sA) + wp * MR + wid * RW;
+#pragma unroll
+              for (int h = 0; h < RW / 32; h++) {
+                const uint2 mine = Aw[h * 32 + lane];
+                const u32 some = __ballot_sync(0xffffffffu, (mine.x | mine.y) != 0u);
+                if (!some) continue;
+#pragma unroll
+                for (int r = 0; r < 32; r++) {
+                  if (!((some >> r) & 1u)) continue;
+                  const uint2 p = Aw[h * 32 + r];
+                  u32 x = ((p.x >> 7) & 0xFFu) | ((p.x >> 15) & 0xFF00u) |
+                          ((p.y & 0x7F80u) << 9) | ((p.y & 0x7F800000u) << 1);
+                  // (two reads in flight; the last key twice when they are odd)
+                  for (x &= bm; x; ) {
+                    const u32 b0 = __ffs(x) - 1;
+                    x &= x - 1;
+                    const u32 b1 = x ? __ffs(x) - 1 : b0;
+                    x &= x - 1;
+                    acc[h * 32 + r] |= Bw[b0 * 32] | Bw[b1 * 32];
+                  }
                 }
               }
             }
-            __syncthreads();  // the table is rebuilt for the next word
-          } else {
-#pragma unroll
-            for (int q = 0; q < RW / 4; q++) {
-              const uint4 x4 = Aw[q];
-              const u32 xs[4] = {x4.x, x4.y, x4.z, x4.w};
-#pragma unroll
-              for (int i = 0; i < 4; i++)
-                for (u32 x = xs[i] & bm; x; x &= x - 1) acc[q * 4 + i] |= Bw[(__ffs(x) - 1) * 32];
-            }
           }
         }
+        __syncthreads();  // every read of this part's words (and, last, of the inner's rows)
+        if (part + kPart == 8 && tid < 8) s_cnt[st][tid] = 0;  // (next used two steps on)
       }
-      __syncthreads();  // every read of the step's operands, before the next step's stores
     }
     // nonzero words out; units that share rows differ in their keys only
     const u32 col = sl * 32 + lane;
@@ -244,9 +309,225 @@ __global__ void __launch_bounds__(kProdBlock, TAB ? 1 : 2) k_join_product(ProdAr
   // algorithmic bytes: 4 per word of OT, a slice of an inner row per key
   // used, 4 per word reduced into the output
   if (lane == 0) prof_add(a.j.ctl, kPJoinMat, 4 * flushed);
-  if (tid == 0) prof_add(a.j.ctl, kPJoinMat, used * min(128u, 4u << rs));
+  if (tid == 0) prof_add(a.j.ctl, kPJoinMat, used * 128);
   if (launch_rec_finish(a.j.rec) && tid == 0)
     prof_add(a.j.ctl, kPJoinMat, (u64)ids * a.side * 32);
+}
+
+// One warp: output row `row`, the keys of its words [w0, w1) (at most 32
+// words).  RS: rows of 2^RS words, 8 to 64.  With rows shorter than a warp,
+// 32 >> RS keys are read at once, one per group of 2^RS lanes.
+template <int RS>
+__device__ __forceinline__ void product_small_row(const ProdArgs &a, u32 row, u32 w0, u32 w1,
+                                                  u32 *keys_used) {
+  constexpr u32 RWD = 1u << RS;
+  constexpr int LOADS = RS >= 5 ? 4 : 4 >> (5 - RS);  // load instructions per 4 keys
+  const int lane = threadIdx.x & 31;
+  const u32 mine = w0 + lane < w1 ? a.OT[(row << RS) + w0 + lane] : 0u;
+  u32 some = __ballot_sync(0xffffffffu, mine != 0u);
+  if (!some) return;
+  u32 acc0 = 0, acc1 = 0, used = 0;
+  const u32 grp = RS >= 5 ? 0 : (u32)lane >> RS, at = RS >= 5 ? (u32)lane : lane & (RWD - 1);
+  for (; some; some &= some - 1) {
+    const int j = __ffs(some) - 1;
+    u32 x = __shfl_sync(0xffffffffu, mine, j);
+    used += __popc(x);
+    const u32 *base = a.F + ((w0 + j) << (5 + RS)) + at;
+    while (x) {
+      // four keys (the last one repeated when fewer are left)
+      u32 k[4];
+      k[0] = __ffs(x) - 1;
+      x &= x - 1;
+#pragma unroll
+      for (int i = 1; i < 4; i++) {
+        k[i] = x ? __ffs(x) - 1 : k[i - 1];
+        x &= x - 1;
+      }
+#pragma unroll
+      for (int i = 0; i < LOADS; i++) {
+        u32 key = k[i];
+        if (RS == 4) key = grp ? k[2 * i + 1] : k[2 * i];
+        if (RS == 3) key = grp == 0 ? k[0] : grp == 1 ? k[1] : grp == 2 ? k[2] : k[3];
+        acc0 |= base[key << RS];
+        if (RS == 6) acc1 |= base[(key << RS) + 32];
+      }
+    }
+  }
+  if (RS < 5) {
+#pragma unroll
+    for (int o = 16; o >= (int)RWD; o >>= 1) acc0 |= __shfl_xor_sync(0xffffffffu, acc0, o);
+  }
+  const u32 out = (row << RS) + at;
+  if (acc0 && grp == 0) {
+    asm volatile("red.global.or.b32 [%0], %1;" ::"l"(a.G + out), "r"(acc0) : "memory");
+    if (a.dirty) a.dirty[out / kBmChunkWords] = 1;
+  }
+  if (RS == 6 && acc1) {
+    asm volatile("red.global.or.b32 [%0], %1;" ::"l"(a.G + out + 32), "r"(acc1) : "memory");
+    if (a.dirty) a.dirty[out / kBmChunkWords] = 1;  // (rows of one chunk)
+  }
+  *keys_used += used;
+}
+
+// The product over 2^8 .. 2^11 ids by the calling grid's warps (block: the
+// caller's number for this one), both sides non-empty.
+__device__ __forceinline__ void product_small(const ProdArgs &a, u32 block) {
+  const u32 rows = a.side * 256, words = a.side * 8;
+  const u32 per = (words + a.splits - 1) / a.splits;
+  u32 used = 0;
+  const u32 nw = gridDim.x * (blockDim.x >> 5);
+  for (u32 u = (block * blockDim.x + threadIdx.x) >> 5; u < rows * a.splits; u += nw) {
+    const u32 row = u / a.splits, w0 = (u % a.splits) * per, w1 = min(w0 + per, words);
+    switch (a.dk) {
+      case 8: product_small_row<3>(a, row, w0, w1, &used); break;
+      case 9: product_small_row<4>(a, row, w0, w1, &used); break;
+      case 10: product_small_row<5>(a, row, w0, w1, &used); break;
+      default: product_small_row<6>(a, row, w0, w1, &used); break;
+    }
+  }
+  // algorithmic bytes: each word of OT, an inner row per key
+  if (!a.j.ctl) return;  // (the resident loop keeps no account)
+  if ((threadIdx.x & 31) == 0 && used) prof_add(a.j.ctl, kPJoinMat, (u64)used << (a.dk - 3));
+  if (blockIdx.x == 0 && threadIdx.x == 0) prof_add(a.j.ctl, kPJoinMat, (u64)rows * words * 4);
+}
+
+__global__ void __launch_bounds__(256) k_join_product_small(ProdArgs a) {
+  if (ctl_stop(a.j.ctl)) return;
+  u64 n_outer;
+  if (product_empty(a.j, &n_outer)) return;
+  product_small(a, blockIdx.x);
+}
+
+// Warps a row's keys are shared among: about 2,048 warps over all rows, at
+// most 32 words of keys each.
+__host__ __device__ constexpr u32 prod_small_splits(u32 side) {
+  return side >= 8 ? 2 : side >= 4 ? 2 : side == 3 ? 3 : side == 2 ? 4 : 2;
+}
+
+constexpr int kProdRowsBlock = 256;
+constexpr u32 kProdListCap = 4096;  // listed keys per round
+constexpr u32 kProdListTake = kProdListCap / kProdRowsBlock;
+
+// V: 16-byte words of a row per lane, 2^(dk-12).  Lane l holds words
+// j * 32 + l; words past the last id's group are neither read nor written.
+template <int V>
+__global__ void __launch_bounds__(kProdRowsBlock, V <= 8 ? 2 : 1) k_join_product_rows(ProdArgs a) {
+  __shared__ u32 s_list[kProdListCap];  // row of the tile << 16 | key
+  __shared__ u64 s_scan[kProdRowsBlock / 32];
+  __shared__ long long s_tile;
+  if (ctl_stop(a.j.ctl)) return;
+  const u64 n_outer = eff_count(a.j.outer, a.j.outer_vis);
+  // (the launch before this one applied the empty-side rule)
+  if (n_outer == 0 || eff_count(a.j.inner, a.j.inner_vis) == 0) return;
+  if (!prod_lists_keys(a, n_outer)) return;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  constexpr int kRows = kProdRowsBlock / 32;
+  const int rs = a.dk - 5;
+  const u32 n4 = a.side * 2;  // 16-byte words of a row that hold ids
+  const u32 tiles = a.side * 256 / kRows;
+  u64 words_out = 0, keys = 0;
+  while (true) {
+    const long long t = grab_tile(a.rows_rec, &s_tile);
+    if (t >= (long long)tiles) break;
+    const u32 row0 = (u32)t * kRows;
+    u32 w[V * 4];
+    u32 left = 0;
+    {
+      const uint4 *p = reinterpret_cast<const uint4 *>(a.OT + ((u64)(row0 + wid) << rs));
+#pragma unroll
+      for (int j = 0; j < V; j++) {
+        const uint4 x = j * 32 + lane < n4 ? p[j * 32 + lane] : make_uint4(0, 0, 0, 0);
+        w[4 * j] = x.x, w[4 * j + 1] = x.y, w[4 * j + 2] = x.z, w[4 * j + 3] = x.w;
+        left += __popc(x.x) + __popc(x.y) + __popc(x.z) + __popc(x.w);
+      }
+    }
+    while (true) {
+      // all keys that are left, or when they do not fit the list a share of
+      // every thread's
+      u64 total;
+      u64 ex = block_excl_scan<kProdRowsBlock>(left, s_scan, &total);
+      if (total == 0) break;  // (block-uniform)
+      u32 take = left;
+      if (total > kProdListCap) {
+        take = min(left, kProdListTake);
+        ex = block_excl_scan<kProdRowsBlock>(take, s_scan, &total);
+      }
+      left -= take;
+      u32 pos = (u32)ex;
+      const u32 end = pos + take;
+#pragma unroll
+      for (int j = 0; j < V * 4; j++) {
+        const u32 key0 = (((j >> 2) * 32 + lane) * 4 + (j & 3)) * 32;
+        while (w[j] && pos < end) {
+          s_list[pos++] = ((u32)wid << 16) | (key0 + __ffs(w[j]) - 1);
+          w[j] &= w[j] - 1;
+        }
+      }
+      __syncthreads();
+      const u32 n = (u32)total;
+      keys += n;
+      // an equal share of the list a warp, two rows in flight
+      u32 i = (u32)((u64)n * wid / kRows);
+      const u32 iend = (u32)((u64)n * (wid + 1) / kRows);
+      uint4 acc[V];
+      const uint4 none = make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int j = 0; j < V; j++) acc[j] = none;
+      auto row_of = [&](u32 e, uint4 *b) {
+        const uint4 *p = reinterpret_cast<const uint4 *>(a.F + ((u64)(e & 0xFFFFu) << rs));
+#pragma unroll
+        for (int j = 0; j < V; j++) b[j] = j * 32 + lane < n4 ? p[j * 32 + lane] : none;
+      };
+      auto flush = [&](u32 r) {
+        u32 *d = a.G + ((u64)(row0 + r) << rs);
+#pragma unroll
+        for (int j = 0; j < V; j++) {
+          const uint4 v = acc[j];
+          acc[j] = none;
+          if ((v.x | v.y | v.z | v.w) == 0u) continue;
+          u32 *o = d + (j * 32 + lane) * 4;
+          if (v.x) asm volatile("red.global.or.b32 [%0], %1;" ::"l"(o + 0), "r"(v.x) : "memory");
+          if (v.y) asm volatile("red.global.or.b32 [%0], %1;" ::"l"(o + 1), "r"(v.y) : "memory");
+          if (v.z) asm volatile("red.global.or.b32 [%0], %1;" ::"l"(o + 2), "r"(v.z) : "memory");
+          if (v.w) asm volatile("red.global.or.b32 [%0], %1;" ::"l"(o + 3), "r"(v.w) : "memory");
+          if (a.dirty) a.dirty[(o - a.G) / kBmChunkWords] = 1;
+          words_out += 4;
+        }
+      };
+      auto or_in = [&](const uint4 *b) {
+#pragma unroll
+        for (int j = 0; j < V; j++)
+          acc[j].x |= b[j].x, acc[j].y |= b[j].y, acc[j].z |= b[j].z, acc[j].w |= b[j].w;
+      };
+      if (i < iend) {
+        u32 cur = s_list[i] >> 16;
+        for (; i < iend; i += 2) {
+          const u32 e0 = s_list[i], e1 = s_list[min(i + 1, iend - 1)];
+          uint4 b0[V], b1[V];
+          row_of(e0, b0);
+          row_of(e1, b1);
+          if ((e0 >> 16) != cur) {
+            flush(cur);
+            cur = e0 >> 16;
+          }
+          or_in(b0);
+          if ((e1 >> 16) != cur) {
+            flush(cur);
+            cur = e1 >> 16;
+          }
+          or_in(b1);  // (the last entry twice when the share is odd)
+        }
+        flush(cur);
+      }
+      __syncthreads();  // the list is rewritten
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) words_out += __shfl_xor_sync(0xffffffffu, words_out, o);
+  if (lane == 0) prof_add(a.j.ctl, kPJoinMat, 4 * words_out);
+  if (tid == 0) prof_add(a.j.ctl, kPJoinMat, keys * n4 * 16);
+  if (launch_rec_finish(a.rows_rec) && tid == 0)
+    prof_add(a.j.ctl, kPJoinMat, (u64)a.side * 256 * a.side * 32);
 }
 
 }  // namespace gdl

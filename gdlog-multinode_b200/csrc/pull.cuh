@@ -497,7 +497,10 @@ __global__ void __launch_bounds__(kPullBlock, 8) k_join_pull_bm(JoinArgs a, u32 
 // output's NEWT and its transposed twin.
 // ---------------------------------------------------------------------------
 constexpr int kRowsMinBits = 12;   // a bitmap row is at least 32 uint4 (one per lane)
-constexpr unsigned long long kRowsBudget = 256ull << 20;  // |inner| x row bytes, auto mode
+// |inner| x row bytes, auto mode: what the gather reads at 6 TB/s from L2 and
+// HBM.  Same generation over 2^16 ids and 120,000 edges (1 GB a join): 0.16
+// ms a join this way, 0.5 to 6.9 ms in the pull form.
+constexpr unsigned long long kRowsBudget = 4ull << 30;
 
 // In-edges of a sorted key list (k << 32 | y): counts per y.
 __global__ void __launch_bounds__(256) k_inv_count(const DArr *list, u32 *cnt, int dk, Ctl *ctl) {
@@ -586,6 +589,7 @@ struct RowsArgs {
   const u32 *inv_keys;  // in-edge sources, grouped by y
   const u32 *inv_ys;    // the y of each in-edge
   const u32 *inv_off;   // inv_off[2^dk]: the number of in-edges
+  u32 n_edges;          // ... if the caller has it, else 0
   u32 unit;             // in-edges per unit of work (8, 16 or 32)
   u32 *dst;            // output rows y (the output's NEWT or its transposed twin)
   u8 *dirty;           // dirty map of dst, or null
@@ -645,8 +649,37 @@ __device__ __forceinline__ void rows_flush(const RowsArgs &a, u32 y, bool whole,
 }
 
 template <int V>
-__global__ void __launch_bounds__(256) k_join_rows_bm(RowsArgs a) {
-  if (ctl_stop(a.j.ctl)) return;
+__device__ __forceinline__ void join_rows(const RowsArgs &a) {
+  const int lane = threadIdx.x & 31;
+  const int rs = a.dk - 5;
+  // the in-edges actually listed (values outside the domain are skipped by
+  // k_inv_fill and reported by the fixpoint)
+  const u32 n_edges = a.n_edges ? a.n_edges : a.inv_off[1u << a.dk];
+  // Units are runs of U consecutive in-edges (grouped by y, so a unit holds
+  // the in-edges of a few consecutive y's), taken round robin: every warp
+  // reads the same number of rows, kFly at a time, and flushes its
+  // accumulator where y changes.  A y none of whose in-edges lie just
+  // before or just after the unit has them all here: its row is this
+  // warp's alone.  The next unit's ids load while this unit's rows are read.
+  // U follows from the edge count: each warp takes k units of U <= a.unit
+  // edges (k = ceil(edges per warp / a.unit)), so no warp takes one unit
+  // more than the others (that unit would be the launch's tail).  U stays
+  // at least a.unit / 2: shorter units would cut most y's in-edges apart,
+  // and a y split between units is written with reductions.
+  const u32 nw = (gridDim.x * blockDim.x) >> 5;
+  const u32 per_warp = (n_edges + nw - 1) / nw;
+  const u32 k_units = max(1u, (per_warp + a.unit - 1) / a.unit);
+  const u32 U = max(max(1u, a.unit / 2), (per_warp + k_units - 1) / k_units);
+  const u32 n_units = (n_edges + U - 1) / U;
+  const uint4 none = make_uint4(0, 0, 0, 0);
+  constexpr int kFly = V <= 4 ? 4 : 2;
+  u32 u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  u32 my_k = 0, my_y = ~0u;
+  if (u < n_units && u * U + lane < n_edges && lane < (int)U) {
+    my_k = a.inv_keys[u * U + lane];
+    my_y = a.inv_ys[u * U + lane];
+  }
+  // (the first unit's ids are on their way)
   if (eff_count(a.j.inner, a.j.inner_vis) == 0) {
     // src/join.cu:42-45: an empty inner zeroes the outer's count
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -675,36 +708,7 @@ __global__ void __launch_bounds__(256) k_join_rows_bm(RowsArgs a) {
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) *a.j.once_pending = 1;
   }
-  const int lane = threadIdx.x & 31;
-  const int rs = a.dk - 5;
-  // the in-edges actually listed (values outside the domain are skipped by
-  // k_inv_fill and reported by the fixpoint)
-  const u32 n_edges = a.inv_off[1u << a.dk];
   u64 words_out = 0, edges = 0;
-  // Units are runs of U consecutive in-edges (grouped by y, so a unit holds
-  // the in-edges of a few consecutive y's), taken round robin: every warp
-  // reads the same number of rows, kFly at a time, and flushes its
-  // accumulator where y changes.  A y none of whose in-edges lie just
-  // before or just after the unit has them all here: its row is this
-  // warp's alone.  The next unit's ids load while this unit's rows are read.
-  // U follows from the edge count: each warp takes k units of U <= a.unit
-  // edges (k = ceil(edges per warp / a.unit)), so no warp takes one unit
-  // more than the others (that unit would be the launch's tail).  U stays
-  // at least a.unit / 2: shorter units would cut most y's in-edges apart,
-  // and a y split between units is written with reductions.
-  const u32 nw = (gridDim.x * blockDim.x) >> 5;
-  const u32 per_warp = (n_edges + nw - 1) / nw;
-  const u32 k_units = max(1u, (per_warp + a.unit - 1) / a.unit);
-  const u32 U = max(max(1u, a.unit / 2), (per_warp + k_units - 1) / k_units);
-  const u32 n_units = (n_edges + U - 1) / U;
-  const uint4 none = make_uint4(0, 0, 0, 0);
-  constexpr int kFly = V <= 4 ? 4 : 2;
-  u32 u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  u32 my_k = 0, my_y = ~0u;
-  if (u < n_units && u * U + lane < n_edges && lane < (int)U) {
-    my_k = a.inv_keys[u * U + lane];
-    my_y = a.inv_ys[u * U + lane];
-  }
   while (u < n_units) {
     const u32 base = u * U;
     const u32 m = min(U, n_edges - base);
@@ -765,10 +769,15 @@ __global__ void __launch_bounds__(256) k_join_rows_bm(RowsArgs a) {
   for (int o = 16; o > 0; o >>= 1) words_out += __shfl_xor_sync(0xffffffffu, words_out, o);
   // algorithmic bytes: a row of the outer and an (edge, y) pair per
   // in-edge, and each output word written (read and written back)
-  if (lane == 0)
+  if (lane == 0 && a.j.ctl)  // (the resident loop keeps no account)
     prof_add(a.j.ctl, kPJoinMat, edges * ((4ull << rs) + 8) + 8 * words_out);
   if (lane == 0 && words_out && a.j.produced) *a.j.produced = 1;
-  launch_rec_finish(a.j.rec);
+}
+
+template <int V>
+__global__ void __launch_bounds__(256) k_join_rows_bm(RowsArgs a) {
+  if (ctl_stop(a.j.ctl)) return;
+  join_rows<V>(a);
 }
 
 // dst |= transpose(src), src cleared: the transposed output of the joins
