@@ -104,6 +104,11 @@ struct RelDev {
   u32 *bmDT, *bmGT, *bmOT;
   // DELTA's rows as they are, for row-gather joins that read DELTA (pull.cuh)
   u32 *bmDN;
+  // Hash form (hash.cuh): the set of FULL's keys, hmask + 2 slots, and with
+  // dependent columns each slot's position in FULL.
+  u64 *hset;
+  u64 hmask;
+  u32 *hord;
 };
 
 // Loop control of a running fixpoint (one per engine, device memory).

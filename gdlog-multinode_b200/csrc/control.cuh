@@ -73,6 +73,7 @@ __device__ __forceinline__ void begin_iteration(RelDev *rels, LieDev *L, const L
       r.w_full_vis = r.full_vis;
       r.w_delta_vis = r.delta_vis;
       r.newt.n = 0;
+      r.delta_next.n = 0;
     }
     if (i < x.ns) {
       RelDev &r = rels[x.sta[j]];

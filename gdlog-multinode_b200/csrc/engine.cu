@@ -40,6 +40,7 @@
 #include "sort.cuh"
 #include "tma.cuh"
 #include "exchange.cuh"
+#include "hash.cuh"
 
 #include <algorithm>
 #include <condition_variable>
@@ -129,6 +130,8 @@ struct LieHost {
   Counts per_iter;  // launches of one enqueued iteration
   // Resident loop (loop.cuh): the graph's body is one launch that runs every
   // iteration; its steps and update list in device memory.
+  // Hash form of the running fixpoint (hash.cuh).
+  bool hashed = false;
   bool resident = false;
   LoopStep *d_steps = nullptr;
   LoopUpd *d_upd = nullptr;
@@ -1601,6 +1604,98 @@ ProdArgs product_args(gdl_engine *e, LieHost &L, const Plan &plan, size_t oi, co
 bool resident_loop(const gdl_engine *e, const LieHost &L, const Plan &plan) {
   if (!L.dense || e->instances || e->pull_joins != 2 || L.dk < kPullMinBits ||
       L.dk > kLoopMaxBits || L.ops.size() > kMaxOps)
+// Whether this LIE's update relations are deduplicated by hash sets
+// (hash.cuh): no bitmaps, only joins, their inners static and their outers
+// DELTAs, tmp NEWTs or static FULLs, so that no operator reads an update
+// relation's FULL, or a sorted DELTA, during the loop.
+bool hash_form(const gdl_engine *e, const LieHost &L, const Plan &plan) {
+  if (L.dense || e->instances || e->dedup_mode != 0 || L.update.empty()) return false;
+  std::vector<char> is_update(e->rels.size(), 0), is_static(e->rels.size(), 0);
+  for (int r : L.update) is_update[r] = 1;
+  for (int r : L.statics) is_static[r] = 1;
+  for (const OpHost &op : L.ops) {
+    if (op.kind != 0 || op.hook || op.inner_ver == GDL_DELTA || !is_static[op.inner] ||
+        is_update[op.inner])
+      return false;
+    if (op.outer_ver == GDL_FULL && (!is_static[op.outer] || is_update[op.outer])) return false;
+    if (op.outer_ver == GDL_NEWT && is_update[op.outer]) return false;
+    // (with dependent columns no key may be all ones, which looks like an
+    // empty slot: column 0 stays below 2^32 - 1)
+    if (is_update[op.out] && e->rels[op.out].dep &&
+        (e->max_value >= 0xFFFFFFFFull || (op.generic && op.gen.add[0])))
+      return false;
+  }
+  for (int r : L.update)
+    if (plan.full_list[r] || plan.delta_idx[r]) return false;
+  return true;
+}
+
+// The hash set of update relation r, sized for its FULL list's capacity, and
+// filled with its committed rows (`push` must follow when this returns with
+// the set moved, before the fill: `fill` is enqueued by fill_hash).
+gdl_status ensure_hash(gdl_engine *e, int r) {
+  RelDev &h = e->h[r];
+  const u64 slots = next_pow2((h.full.cap + 2) / 3 * 4);
+  const bool dep = e->rels[r].dep != 0;
+  if (!h.hset || h.hmask + 1 < slots) {
+    dfree(e, h.hset);
+    h.hset = nullptr;
+    TRY(dalloc(e, (void **)&h.hset, (slots + 1) * sizeof(u64)));
+    dfree(e, h.hord);
+    h.hord = nullptr;
+    h.hmask = slots - 1;
+  }
+  if (dep && !h.hord) TRY(dalloc(e, (void **)&h.hord, (h.hmask + 2) * sizeof(u32)));
+  return GDL_OK;
+}
+u64 hash_prefix(const gdl_engine *e, int r) { return ~dep_low_mask(e, e->rels[r]); }
+gdl_status fill_hash(gdl_engine *e, int r) {
+  const RelDev &h = e->h[r];
+  CK(e, cudaMemsetAsync(h.hset, 0xFF, (h.hmask + 2) * sizeof(u64), e->s));
+  if (h.hord) CK(e, cudaMemsetAsync(h.hord, 0xFF, (h.hmask + 2) * sizeof(u32), e->s));
+  if (h.full.n) {
+    k_hash_fill<<<grid_for(e, h.full.n, 256, 8), 256, 0, e->s>>>(&e->d_rels[r], hash_prefix(e, r),
+                                                                  e->d_ctl);
+    e->aux_launches++;
+  }
+  CK(e, cudaGetLastError());
+  return GDL_OK;
+}
+
+// Sort a list of n unique keys in place (a DArr in the relation table, whose
+// host mirror is a).
+gdl_status sort_in_place(gdl_engine *e, const DArr *d, const DArr &a) {
+  if (a.n < 2) return GDL_OK;
+  if (e->sort_cap < a.n) {
+    dfree(e, e->sort_buf);
+    e->sort_buf = nullptr;
+    e->sort_cap = a.n;
+    TRY(dalloc(e, (void **)&e->sort_buf, e->sort_cap * sizeof(u64)));
+  }
+  TRY(ensure_scratch(e));  // (tile states for the new capacity)
+  Counts kc;
+  launch_sort(e, d, a.ptr, std::max<u64>(a.n, 1), &kc);
+  e->aux_launches += kc.total;
+  const u64 *at = sorted_location(e, a.ptr);
+  if (at != a.ptr)
+    CK(e, cudaMemcpyAsync(a.ptr, at, a.n * sizeof(u64), cudaMemcpyDeviceToDevice, e->s));
+  CK(e, cudaGetLastError());
+  return GDL_OK;
+}
+
+HashJoinArgs hash_args(gdl_engine *e, const JoinArgs &a, int out, bool hashed) {
+  HashJoinArgs h;
+  memset(&h, 0, sizeof h);
+  memcpy(&h.j, &a, sizeof a);
+  h.out = &e->d_rels[out];
+  h.hashed = hashed;
+  h.prefix = hashed ? hash_prefix(e, out) : ~0ull;
+  h.need_full = need_index(out, kNeedFull);
+  h.need_delta = need_index(out, kNeedDelta);
+  h.need_newt = need_index(out, kNeedNewt);
+  return h;
+}
+
     return false;
   for (size_t oi = 0; oi < L.ops.size(); oi++) {
     const OpHost &op = L.ops[oi];
@@ -1895,6 +1990,22 @@ void enqueue_iteration(gdl_engine *e, LieHost &L, const Plan &plan, Counts *kc, 
       memcpy(&b, &a, sizeof b);
       b.rec = &e->recs[1];
       if (dense && e->dense_join_passes == 1) {
+      if (L.hashed) {
+        bool hashed = false;
+        for (int r : L.update) hashed = hashed || r == op.out;
+        if (plan.static_once[oi]) {
+          a.once = &L.d_lie->jonce[oi];
+          a.once_pending = &L.d_lie->jonce_pending[oi];
+          a.produced = &L.d_lie->produced[oi];
+          a.phantom = &R[op.out].newt_phantom;
+        }
+        HashJoinArgs ha = hash_args(e, a, op.out, hashed);
+        PLAUNCH(kc, kPJoinMat,
+                k_join_hash<<<grid_for(e, outer_cap, 256, 6), 256, 0, s>>>(ha));
+        ha.j.rec = &e->recs[1];
+        PLAUNCH(kc, kPJoinMat, k_join_hash_heavy<<<(int)e->sms * 4, 256, 0, s>>>(ha));
+        continue;
+      }
         const int jb = e->join_block;
         const int jg = grid_for(e, outer_cap, jb, kFuseCtasPerSm * kFuseBlock / jb);
         const int hg = (int)e->sms * 4 * kFuseBlock / jb;
@@ -2090,6 +2201,15 @@ void enqueue_update_step(gdl_engine *e, LieHost &L, const Plan &plan, Counts *kc
       launch_sort(e, &R[r].newt, rh.newt.ptr, rh.newt.cap, kc);
       MergeArgs m;
       memset(&m, 0, sizeof m);
+    if (L.hashed) {
+      if (e->rels[r].dep) {
+        JoinArgs a;
+        memset(&a, 0, sizeof a);
+        a.ctl = e->d_ctl;
+        PLAUNCH(kc, kPMerge, k_hash_aside<<<(int)e->sms * 2, 256, 0, s>>>(hash_args(e, a, r, true)));
+      }
+      continue;
+    }
       m.newt = &R[r].newt;
       m.a = sorted_location(e, rh.newt.ptr);
       m.full = &R[r].full;
@@ -2677,10 +2797,25 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
   mark("scratch");
   TRY(push(e));
   mark("push");
+  L.hashed = hash_form(e, L, plan);
+  if (L.hashed) {
+    // room for a few million tuples before the first growth
+    for (int r : L.update) {
+      RelDev &h = e->h[r];
+      TRY(ensure_arr(e, h.full, std::max<u64>(kHashMinRows, 2 * h.full.n), true));
+      TRY(ensure_arr(e, h.delta, kHashMinRows, true));
+      TRY(ensure_arr(e, h.delta_next, h.delta.cap, false));
+      TRY(ensure_hash(e, r));
+      h.dense = h.full_lazy = 1;  // (the commit only counts FULL's new rows)
+    }
+    for (int r : L.tmps) TRY(ensure_arr(e, e->h[r].newt, kHashMinRows, false));
+  }
   if (L.dense) {
     // FULL's bitmap from its list; NEWT bitmaps empty.
     const u64 words = L.map.words;
     for (int r : L.update) {
+  if (L.hashed)
+    for (int r : L.update) TRY(fill_hash(e, r));
       const RelDev &h = e->h[r];
       CK(e, cudaMemsetAsync(h.bmF, 0, words * 4, e->s));
       CK(e, cudaMemsetAsync(h.bmG, 0, words * 4, e->s));
@@ -3013,6 +3148,14 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
         // The iteration runs again from its start: its NEWT bitmaps must
         // be empty again (emitting relations clear them only on success).
         const u64 words = L.map.words;
+      if (L.hashed) {
+        // the sets again from the committed rows
+        for (int r : L.update) TRY(ensure_hash(e, r));
+        TRY(push(e));
+        TRY(reset_ctl(e));
+        c.generation = e->generation;
+        for (int r : L.update) TRY(fill_hash(e, r));
+      }
         for (auto *v : {&L.update, &L.tmps})
           for (int r : *v) {
             CK(e, cudaMemsetAsync(e->h[r].bmG, 0, words * 4, e->s));
@@ -3206,6 +3349,22 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
   CK(e, cudaEventSynchronize(e->ev1));
   if (listed && (lc->timeout || lc->oob)) {
     e->broken = true;
+  if (L.hashed) {
+    // FULL, and a DELTA that max_iteration left, sorted once
+    const u64 kept_iteration = c.iteration;
+    TRY(pull(e));
+    TRY(reset_ctl(e));
+    for (int r : L.update) {
+      RelDev &h = e->h[r];
+      h.dense = h.full_lazy = 0;
+      TRY(sort_in_place(e, &e->d_rels[r].full, h.full));
+      TRY(sort_in_place(e, &e->d_rels[r].delta, h.delta));
+    }
+    TRY(push(e));
+    CK(e, cudaMemcpyAsync(e->h_ctl, e->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, e->s));
+    listed = true;
+    c.iteration = kept_iteration;
+  }
     return fail(e, GDL_E_TIMEOUT, "listing FULL/DELTA after the loop failed (timeout=%u oob=%u)",
                 lc->timeout, lc->oob);
   }
@@ -3390,6 +3549,8 @@ static void release_program(gdl_engine *e) {
     const RelHost &rh = e->rels[i];
     for (u32 *q : {rh.inv_off, rh.inv_cur, rh.inv_keys, rh.inv_ys})
       dfree(e, q);
+    dfree(e, r.hset);
+    dfree(e, r.hord);
     if (!e->rels[i].raw_is_full) dfree(e, e->rels[i].raw);
   }
   for (LieHost &L : e->lies) {
