@@ -28,6 +28,7 @@
 // state) or to finish.
 #include "../../include/gdlog_b200.h"
 
+#include "closure.cuh"
 #include "common.cuh"
 #include "control.cuh"
 #include "dense.cuh"
@@ -135,6 +136,11 @@ struct LieHost {
   // Resident loop (loop.cuh): the graph's body is one launch that runs every
   // iteration; its steps and update list in device memory.
   bool resident = false;
+  // Linear recursion in one pass an iteration (closure.cuh): the loop's
+  // arguments; its per-row arrays (c_rows of them, c_edges adj entries).
+  bool closure = false;
+  ClosureArgs cargs{};
+  u32 *c_mem = nullptr;
   LoopStep *d_steps = nullptr;
   LoopUpd *d_upd = nullptr;
   int n_steps = 0, n_upd = 0;
@@ -1871,10 +1877,150 @@ gdl_status push_loop(gdl_engine *e, LieHost &L, const Plan &plan) {
   return GDL_OK;
 }
 
+// A LIE of one linear rule over a static relation (closure.cuh).
+bool closure_form(const gdl_engine *e, const LieHost &L) {
+  if (!L.dense || e->pull_joins != 2 || L.ops.size() != 1 || L.update.size() != 1 ||
+      !L.tmps.empty() || L.max_iteration < 2147483647LL || (!e->instances && L.dk < kPullMinBits))
+    return false;
+  const OpHost &op = L.ops[0];
+  bool stat = false;
+  for (int r : L.statics) stat = stat || r == op.inner;
+  return op.kind == 0 && !op.hook && !op.generic && op.pred.kind == 0 && stat &&
+         op.inner_ver != GDL_DELTA && op.inner != op.out && op.outer == L.update[0] &&
+         op.out == L.update[0] && op.outer_ver == GDL_DELTA && op.sel.s0 == 1 && op.sel.s1 == 3;
+}
+
+// The closure form's arrays, before the relation table is uploaded.  Sets
+// L.closure unless some row has too many sources (one read-back).
+gdl_status prepare_closure(gdl_engine *e, LieHost &L) {
+  const int in = L.ops[0].inner, r = L.update[0];
+  const u64 n = e->h[in].full.n;
+  std::vector<u32> first;
+  u64 rows = L.map.seg_shift >= 31 ? square_rows(L.dk, L.side) : 0;
+  if (e->instances)
+    for (const SegInfo &s : e->segs) {
+      first.push_back((u32)rows);
+      rows += s.n;
+    }
+  if (rows >> 32 || L.map.words >> 32 || n >> 32) return GDL_OK;
+  ClosureArgs &a = L.cargs;
+  memset(&a, 0, sizeof a);
+  a.rows = (u32)rows;
+  a.rs = e->instances ? 0 : L.dk - 5;
+  // one block: extents (2 x 2 words a row), and batched: ranges, words and
+  // instances of the rows, adj, the first row of each instance
+  const u64 per_row = e->instances ? 8 : 4;
+  const u64 u32s = rows * per_row + (e->instances ? n + first.size() : 0) + 4;
+  dfree(e, L.c_mem);
+  L.c_mem = nullptr;
+  TRY(dalloc(e, (void **)&L.c_mem, u32s * sizeof(u32)));
+  u32 *p = L.c_mem;
+  a.ext[0] = reinterpret_cast<uint2 *>(p);
+  a.ext[1] = reinterpret_cast<uint2 *>(p + 2 * rows);
+  p += 4 * rows;
+  u32 *maxdeg = p;
+  p += 4;
+  CK(e, cudaMemsetAsync(maxdeg, 0, 2 * sizeof(u32), e->s));  // and the bad-edge flag
+  ClosureRows m{nullptr, nullptr, 1, 31};
+  if (e->instances) {
+    u32 *start = p, *end = p + rows, *word = p + 2 * rows, *inst = p + 3 * rows;
+    u32 *adj = p + 4 * rows, *d_first = adj + n;
+    CK(e, cudaMemcpyAsync(d_first, first.data(), first.size() * sizeof(u32),
+                          cudaMemcpyHostToDevice, e->s));
+    m = ClosureRows{e->d_segs, d_first, (u32)e->segs.size(), e->seg_shift};
+    CK(e, cudaMemsetAsync(start, 0, 2 * rows * sizeof(u32), e->s));
+    k_closure_rows<<<(int)std::min<u64>(first.size(), (u64)e->sms * 8), 256, 0, e->s>>>(m, word,
+                                                                                        inst);
+    e->aux_launches++;
+    if (n) {
+      // the edges by column 1
+      u64 *keys = nullptr;
+      TRY(dalloc(e, (void **)&keys, n * sizeof(u64)));
+      k_closure_swap<<<grid_for(e, n, 256, 8), 256, 0, e->s>>>(&e->d_rels[in].full, keys);
+      e->aux_launches++;
+      const DArr d{keys, n, n};
+      CK(e, cudaMemcpyAsync(e->d_tmp, &d, sizeof d, cudaMemcpyHostToDevice, e->s));
+      TRY(sort_in_place(e, e->d_tmp, d));
+      k_closure_adj<<<grid_for(e, n, 256, 8), 256, 0, e->s>>>(keys, n, m, start, end, adj,
+                                                                    maxdeg + 1);
+      e->aux_launches++;
+      dfree(e, keys);  // stream-ordered
+    }
+    a.start = start;
+    a.end = end;
+    a.adj = adj;
+    a.row_word = word;
+    a.row_inst = inst;
+    a.inst_last = L.d_inst_last;
+  } else {
+    TRY(build_inverse(e, in, L.dk));
+    const RelHost &ih = e->rels[in];
+    a.start = ih.inv_off;
+    a.end = ih.inv_off + 1;
+    a.adj = ih.inv_keys;
+  }
+  k_closure_degree<<<grid_for(e, rows, 256, 4), 256, 0, e->s>>>(a.start, a.end, a.rows, maxdeg);
+  e->aux_launches++;
+  u32 deg[2] = {0, 0};
+  CK(e, cudaMemcpyAsync(deg, maxdeg, sizeof deg, cudaMemcpyDeviceToHost, e->s));
+  CK(e, cudaStreamSynchronize(e->s));
+  if (deg[0] > kClosureMaxDegree || deg[1]) return GDL_OK;
+  RelDev &h = e->h[r];
+  const u64 words = L.map.words;
+  if (!h.bmDN) TRY(dalloc(e, (void **)&h.bmDN, words * 4));
+  if (!h.bmGT) TRY(dalloc(e, (void **)&h.bmGT, words * 4));
+  a.F = h.bmF;
+  a.D[0] = h.bmDN;
+  a.D[1] = h.bmGT;
+  a.rd = &e->d_rels[r];
+  a.loop.rels = e->d_rels;
+  a.loop.lie = L.d_lie;
+  a.loop.ctl = e->d_ctl;
+  // rows a warp looks at: as few as keep every warp of the grid busy
+  const u64 warps = (u64)e->sms * kClosureCtasPerSm * (kLoopBlock / 32);
+  a.chunk = 4;
+  while (a.chunk < 32 && rows / a.chunk > warps) a.chunk *= 2;
+  L.closure = true;
+  return GDL_OK;
+}
+
+// The first DELTA's rows and extents (after the upload of the table).
+gdl_status start_closure(gdl_engine *e, LieHost &L) {
+  const int r = L.update[0];
+  const RelDev &h = e->h[r];
+  const ClosureArgs &a = L.cargs;
+  ClosureRows m{nullptr, nullptr, 1, 31};
+  if (e->instances)
+    m = ClosureRows{e->d_segs, a.adj + e->h[L.ops[0].inner].full.n, (u32)e->segs.size(),
+                    e->seg_shift};
+  k_closure_ext_init<<<grid_for(e, a.rows, 256, 8), 256, 0, e->s>>>(a.ext[0], a.ext[1], a.rows);
+  e->aux_launches++;
+  if (h.delta.n) {
+    const DArr *d = &e->d_rels[r].delta;
+    const int g = grid_for(e, h.delta.n, 256, 8);
+    k_closure_ext<<<g, 256, 0, e->s>>>(d, m, a.ext[0]);
+    k_closure_zero<<<grid_for(e, (u64)a.rows * 32, 256, 8), 256, 0, e->s>>>(a);
+    k_bm_from_list<<<g, 256, 0, e->s>>>(d, a.D[0], L.map, e->d_ctl);
+    e->aux_launches += 3;
+  }
+  CK(e, cudaGetLastError());
+  return GDL_OK;
+}
+
 // The resident loop as the graph body's one launch.  Two blocks an SM at
 // most (all resident); fewer where a domain has less work than that (a
 // barrier's cost grows with its blocks).
 cudaError_t launch_loop(gdl_engine *e, LieHost &L, Counts *kc) {
+  if (L.closure) {
+    ClosureArgs a;
+    memcpy(&a, &L.cargs, sizeof a);
+    const u64 chunks = (a.rows + a.chunk - 1) / a.chunk;
+    const int g = grid_for(e, chunks, kLoopBlock / 32, kClosureCtasPerSm);
+    void *args[] = {&a};
+    kc->add(kPControl);
+    return cudaLaunchCooperativeKernel((const void *)k_closure_loop, dim3(g), dim3(kLoopBlock),
+                                       args, 0, e->s);
+  }
   LoopArgs a;
   memset(&a, 0, sizeof a);
   a.steps = L.d_steps;
@@ -2796,6 +2942,9 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
     }
     TRY(ps);
   }
+  const bool use_graph = getenv("GDLOG_NO_GRAPH") == nullptr && !e->profile;
+  L.closure = false;
+  if (use_graph && closure_form(e, L)) TRY(prepare_closure(e, L));
   mark("dense_alloc");
   L.hashed = hash_form(e, L, plan);
   if (L.hashed) {
@@ -2822,8 +2971,10 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
     for (int r : L.update) {
       const RelDev &h = e->h[r];
       CK(e, cudaMemsetAsync(h.bmF, 0, words * 4, e->s));
-      CK(e, cudaMemsetAsync(h.bmG, 0, words * 4, e->s));
-      CK(e, cudaMemsetAsync(h.bmD, 0, words / kBmChunkWords, e->s));
+      if (!L.closure) {
+        CK(e, cudaMemsetAsync(h.bmG, 0, words * 4, e->s));
+        CK(e, cudaMemsetAsync(h.bmD, 0, words / kBmChunkWords, e->s));
+      }
       if (h.full.n) {
         k_bm_from_list<<<grid_for(e, h.full.n, 256, 8), 256, 0, e->s>>>(
             &e->d_rels[r].full, h.bmF, L.map, e->d_ctl);
@@ -2838,7 +2989,7 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
           e->aux_launches++;
         }
       }
-      if (plan.delta_n[r]) {
+      if (plan.delta_n[r] && !L.closure) {
         // ... and as rows, for the row-gather joins
         CK(e, cudaMemsetAsync(h.bmDN, 0, words * 4, e->s));
         if (h.delta.n) {
@@ -2871,11 +3022,12 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
         e->aux_launches++;
       }
     }
+    if (L.closure) TRY(start_closure(e, L));
     // the in-edges of the static inners of row-gather joins
     std::vector<char> built(e->rels.size(), 0);
     for (size_t oi = 0; oi < L.ops.size(); oi++) {
       const int r = L.ops[oi].inner;
-      if (!plan.rows[oi] || built[r]) continue;
+      if (!plan.rows[oi] || built[r] || L.closure) continue;
       TRY(build_inverse(e, r, L.dk));
       built[r] = 1;
     }
@@ -2975,9 +3127,8 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
   L.graph_launches = 0;
   L.kernels = 0;
   L.graph_dirty = true;
-  const bool use_graph = getenv("GDLOG_NO_GRAPH") == nullptr && !e->profile;
-  L.resident = use_graph && resident_loop(e, L, plan);
-  if (L.resident) TRY(push_loop(e, L, plan));
+  L.resident = L.closure || (use_graph && resident_loop(e, L, plan));
+  if (L.resident && !L.closure) TRY(push_loop(e, L, plan));
   u64 batch = 4;
   bool first_batch = true;
   bool tail_listed = false;
@@ -3561,7 +3712,7 @@ static void release_program(gdl_engine *e) {
     release_graph(e, L);
     // stream-ordered frees (a cudaFree would wait for the whole device)
     for (void *p : {(void *)L.d_trace, (void *)L.d_lie, (void *)L.d_joinrec, (void *)L.d_steps,
-                    (void *)L.d_upd})
+                    (void *)L.d_upd, (void *)L.c_mem})
       dfree(e, p);
     dfree(e, L.d_inst_delta);
     dfree(e, L.d_inst_last);
