@@ -82,6 +82,19 @@ __device__ __forceinline__ u32 transpose32(u32 x, int lane) {
   return x;
 }
 
+// Tile t of a pass over per x per tiles: strips of eight tile rows, down each
+// column of a strip in turn.  Eight consecutive tiles then cover 256
+// consecutive bytes of each row they write transposed, and 32 tiles a whole
+// line of each row they read, while those lines are in L2: walked row by row,
+// the 32-byte pieces of a transposed line are `per` tiles apart.
+constexpr u32 kTileStrip = 8;
+__device__ __forceinline__ void tile_rc(u32 t, u32 per, u32 &tr, u32 &tc) {
+  const u32 s = t / (kTileStrip * per), in = t - s * kTileStrip * per;
+  const u32 h = min(kTileStrip, per - s * kTileStrip);
+  tc = in / h;
+  tr = s * kTileStrip + in % h;
+}
+
 struct TransposeArgs {
   const u32 *g;   // source bitmap
   const u32 *f;   // if set: the source is g & ~f
@@ -104,10 +117,11 @@ __global__ void __launch_bounds__(kTrBlock) k_bm_transpose(TransposeArgs a) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   u64 bits = 0, moved = 0;
   for (u64 t = blockIdx.x; t < tiles; t += gridDim.x) {
-    const u64 tr = t / per, tc = t % per;
+    u32 tr, tc;
+    tile_rc((u32)t, (u32)per, tr, tc);
     // this thread's input row: tile row tr, row threadIdx.x of the tile
     // (warp wid holds rows 32 wid .. 32 wid + 31), words 8 tc .. 8 tc + 7
-    const u64 src = ((tr * 256 + (u64)threadIdx.x) << rs) + tc * 8;
+    const u64 src = (((u64)tr * 256 + threadIdx.x) << rs) + tc * 8;
     u32 v[8];
     load8(a.g + src, v);
     bool any = (v[0] | v[1] | v[2] | v[3] | v[4] | v[5] | v[6] | v[7]) != 0u;
@@ -125,7 +139,7 @@ __global__ void __launch_bounds__(kTrBlock) k_bm_transpose(TransposeArgs a) {
     // (a tile's reads of s_t are ordered before the next tile's writes by
     // the next tile's __syncthreads_or)
     const bool tile_any = __syncthreads_or(any);
-    uint4 *d = reinterpret_cast<uint4 *>(a.dst + ((tc * 256 + (u64)threadIdx.x) << rs) + tr * 8);
+    uint4 *d = reinterpret_cast<uint4 *>(a.dst + (((u64)tc * 256 + threadIdx.x) << rs) + tr * 8);
     if (tile_any) {
 #pragma unroll
       for (int i = 0; i < 8; i++) {

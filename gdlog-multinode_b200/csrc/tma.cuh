@@ -186,7 +186,9 @@ __global__ void __launch_bounds__(kTrBlock, 2)
   const u64 mine = tiles > blockIdx.x ? (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
   auto issue = [&](u64 j) {
     const u64 t = blockIdx.x + j * gridDim.x;
-    const int tr = (int)(t / per), tc = (int)(t % per), st = (int)(j % ns);
+    u32 tr, tc;
+    tile_rc((u32)t, (u32)per, tr, tc);
+    const int st = (int)(j % ns);
     mbar_expect_tx(&s_bar[st], 2 * kTmaTile);
     if (gt)
       tma_load(in_n(st), &m.nsrc, tr * 8, tc * 256, &s_bar[st]);
@@ -202,7 +204,8 @@ __global__ void __launch_bounds__(kTrBlock, 2)
   for (; k < mine; k++) {
     const u64 t = blockIdx.x + k * gridDim.x;
     const int st = (int)(k % ns), slot = (int)(k & 1);
-    const int tr = (int)(t / per), tc = (int)(t % per);
+    u32 tr, tc;
+    tile_rc((u32)t, (u32)per, tr, tc);
     // (stage (k + ns - 1) % ns held tile k - 1, read before the last barrier)
     if (tid == 0 && k + ns - 1 < mine) issue(k + ns - 1);
     const bool ok = mbar_wait(&s_bar[st], (u32)(k / ns) & 1u, limit);
@@ -351,7 +354,9 @@ __global__ void __launch_bounds__(kTrBlock, 2)
   const u64 mine = tiles > blockIdx.x ? (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
   auto issue = [&](u64 j) {
     const u64 t = blockIdx.x + j * gridDim.x;
-    const int tr = (int)(t / per), tc = (int)(t % per), st = (int)(j % ns);
+    u32 tr, tc;
+    tile_rc((u32)t, (u32)per, tr, tc);
+    const int st = (int)(j % ns);
     mbar_expect_tx(&s_bar[st], ni * kTmaTile);
     tma_load(in_s(st), &m.src, tc * 8, tr * 256, &s_bar[st]);
     if (!overwrite) tma_load(in_d(st), &m.dst, tr * 8, tc * 256, &s_bar[st]);
@@ -364,7 +369,8 @@ __global__ void __launch_bounds__(kTrBlock, 2)
   for (; k < mine; k++) {
     const u64 t = blockIdx.x + k * gridDim.x;
     const int st = (int)(k % ns), slot = (int)(k & 1);
-    const int tr = (int)(t / per), tc = (int)(t % per);
+    u32 tr, tc;
+    tile_rc((u32)t, (u32)per, tr, tc);
     if (tid == 0 && k + ns - 1 < mine) issue(k + ns - 1);
     const bool ok = mbar_wait(&s_bar[st], (u32)(k / ns) & 1u, limit);
     u32 v[8], q[8];
