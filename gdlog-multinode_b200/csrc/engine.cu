@@ -297,6 +297,7 @@ struct gdl_engine {
   int row_gather = 2;
   u32 spin_limit = kSpinLimit;  // polls of a bounded device wait
   u32 test_wait = 0;            // gdl_engine_test_timeout (next fixpoint only)
+  u32 *prod_list = nullptr;     // rows of a product's outer (product.cuh)
   u64 *d_pull_count = nullptr;  // bit count of a transposed NEWT (zero between launches)
   // Device memory in bytes, read once at creation: cudaMemGetInfo can take
   // tens of milliseconds on a busy host, so the fixpoint sizes its lists
@@ -1337,10 +1338,8 @@ void launch_rows(gdl_engine *e, const RowsArgs &ra, Counts *kc) {
   }
 }
 
-// A boolean-product join (product.cuh).  With tables, from
-// 2^kProdTableBits ids on, the key range is split until there are four units
-// of work a block: at 20,000 ids 400 row-by-column blocks share 148 SMs
-// unevenly (3 rounds for 2.7), and at 2^12 there are only 16.
+// A boolean-product join (product.cuh): a resident wave of every kernel, the
+// work divided on the device.
 void launch_product(gdl_engine *e, ProdArgs &pa, Counts *kc) {
   const u32 ids = pa.side * 256;
   if (pa.dk < kProdTableBits) {
@@ -1348,13 +1347,8 @@ void launch_product(gdl_engine *e, ProdArgs &pa, Counts *kc) {
             <<<grid_for(e, (u64)ids * pa.splits, 8, 4), 256, 0, e->s>>>(pa));
     return;
   }
-  const u64 blocks = (u64)((ids + kProdRows - 1) / kProdRows) * ((ids + 1023) / 1024);
-  const u64 split =
-      std::min<u64>(pa.side, std::max<u64>(1, ((u64)e->sms * 4 + blocks - 1) / blocks));
-  pa.ksteps = (u32)((pa.side + split - 1) / split);
-  const u64 units = blocks * ((pa.side + pa.ksteps - 1) / pa.ksteps);
-  PLAUNCH(kc, kPJoinMat, k_join_product<<<grid_for(e, units, 1, 1), kProdBlock, kProdSmem, e->s>>>(
-                             pa));
+  PLAUNCH(kc, kPJoinMat, k_prod_rows<<<grid_for(e, pa.side * 8, 1, 4), 256, 0, e->s>>>(pa));
+  PLAUNCH(kc, kPJoinMat, k_join_product<<<(int)e->sms, kProdBlock, kProdSmem, e->s>>>(pa));
   const int gr = (int)e->sms * (pa.dk >= 16 ? 1 : 2);
 #define GDL_PROD_ROWS(V) \
   PLAUNCH(kc, kPJoinMat, k_join_product_rows<V><<<gr, kProdRowsBlock, 0, e->s>>>(pa))
@@ -1602,6 +1596,7 @@ ProdArgs product_args(gdl_engine *e, LieHost &L, const Plan &plan, size_t oi, co
   pa.OT = op.outer_ver == GDL_NEWT ? oh.bmGT : oh.bmDT;
   pa.F = e->h[op.inner].bmF;
   pa.rows_rec = &e->recs[9];
+  pa.list = e->prod_list;
   pa.G = plan.pull_t[oi] ? out.bmOT : out.bmG;
   pa.dirty = plan.pull_t[oi] ? nullptr : out.dirty;
   pa.dk = L.dk;
@@ -3651,6 +3646,8 @@ gdl_status gdl_engine_create(int32_t device, void *stream, gdl_engine **out) {
       bad(cudaMalloc(&e->recs, 16 * sizeof(LaunchRec))) ||
       bad(cudaMalloc(&e->d_tmp, 4 * sizeof(DArr))) || bad(cudaMalloc(&e->d_u64, 4 * sizeof(u64))) ||
       bad(cudaMalloc(&e->d_u32, 4 * sizeof(u32))) ||
+      bad(cudaMalloc(&e->prod_list, ((1u << 16) + 1) * sizeof(u32))) ||
+      bad(cudaMemsetAsync(e->prod_list, 0, sizeof(u32), e->s)) ||
       bad(cudaMalloc(&e->d_pull_count, sizeof(u64))) || bad(cudaEventCreate(&e->ev0)) ||
       bad(cudaEventCreate(&e->ev1)) ||
       bad(cudaEventCreateWithFlags(&e->ev_first, cudaEventDisableTiming)) ||
@@ -3758,6 +3755,7 @@ gdl_status gdl_engine_clear(gdl_engine *e) {
       CK(e, cudaMemsetAsync(e->sort_offsets, 0, kMaxPasses * kMaxRadix * sizeof(u32), e->s));
     CK(e, cudaMemsetAsync(e->d_u32, 0, 4 * sizeof(u32), e->s));
     CK(e, cudaMemsetAsync(e->d_pull_count, 0, sizeof(u64), e->s));
+    CK(e, cudaMemsetAsync(e->prod_list, 0, sizeof(u32), e->s));
     TRY(reset_ctl(e));
     CK(e, cudaStreamSynchronize(e->s));
     e->broken = false;
@@ -3804,7 +3802,7 @@ gdl_status gdl_engine_destroy(gdl_engine *e) {
                   (void *)e->d_segs,
                   (void *)e->d_tile_inst, (void *)e->d_square_seg,
                   (void *)e->recs,
-                  (void *)e->d_tmp, (void *)e->d_u64, (void *)e->d_u32, (void *)e->d_pull_count,
+                  (void *)e->d_tmp, (void *)e->d_u64, (void *)e->d_u32, (void *)e->d_pull_count, (void *)e->prod_list,
                   e->d_count, e->d_part,
                   (void *)e->d_rels,
                   (void *)e->d_ctl})

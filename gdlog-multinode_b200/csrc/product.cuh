@@ -10,7 +10,7 @@
 // ids.  Here no list and no index exist.
 //
 // k_join_product: a block owns MR output rows by a slice of 1024 columns (a
-// word a lane, MR / 16 rows a warp, accumulated in registers) and walks the
+// word a lane, MR / 32 rows a warp, accumulated in registers) and walks the
 // keys 32 at a time.  Per 32 keys (one word of each row of OT), by the bits
 // its rows hold:
 //   * many: the four-Russians method (Arlazarov, Dinic, Kronrod, Faradzev
@@ -29,11 +29,14 @@
 // branch.  The next 256 keys' operands load (cp.async for the inner's rows,
 // registers for the outer's words) while these are used.
 //
-// k_join_product_rows: an outer of few tuples (their inner rows within
-// kProdRowsBytes) would leave that kernel scanning empty words for every
-// slice.  A block takes 8 rows of OT, lists their keys in shared memory and
-// its warps OR equal shares of the listed inner rows, whole rows at a time.
-// Both kernels are launched; the device-side tuple count picks one.
+// k_join_product_rows: a row of few keys would leave that kernel scanning
+// empty words for every slice.  A block takes 8 rows of OT, lists their keys
+// in shared memory and its warps OR equal shares of the listed inner rows,
+// whole rows at a time, at L2's rate (6 TB/s: 0.4 ns a key at 20,000 ids,
+// where a row costs the tables 350 ns however many keys it has).
+// Both run: k_prod_rows counts each row's keys and lists the long ones for
+// k_join_product (points-to relations are reflexive, so half the rows hold a
+// few keys and the others thousands; 20,000 variables: 260 -> 195 ms).
 //
 // product_small: below 2^kProdTableBits ids there are too few rows to fill
 // the GPU with tables.  A warp takes one output row and a share of its keys
@@ -47,16 +50,24 @@
 
 namespace gdl {
 
-constexpr int kProdBlock = 512;
+constexpr int kProdBlock = 1024;
 constexpr int kProdWarps = kProdBlock / 32;
 constexpr int kProdStep = 256;       // keys per staged step: 8 words of a row
 constexpr int kProdTableBits = 12;   // tables from 2^12 ids on
-constexpr int kProdWarpRows = 64;    // output rows per warp
+// Output rows per warp: 32 warps of 32 rows, not 16 of 64 (the same 1024
+// accumulators a lane column), halve the unrolled code a warp runs through
+// (instruction fetch was a tenth of its stalls) and double the warps that
+// hide the reads' latency.
+constexpr int kProdWarpRows = 32;
 constexpr u32 kProdRows = kProdWarps * kProdWarpRows;  // per block
+constexpr u32 kProdUnits = 6;        // units of work a block, at least
 constexpr int kProdPart = 4;         // words of a step staged together
-// inner row bytes below which the outer's keys are listed
-constexpr u64 kProdRowsBytes = 1ull << 30;
-
+// A row is short, its keys listed, below 1 / kProdShort of the ids: a third
+// of what the tables take for it.
+constexpr u32 kProdShort = 64;
+__device__ __forceinline__ bool prod_short(u32 keys, u32 side) {
+  return keys * kProdShort < side * 256;
+}
 // Dynamic shared memory: the tables, two stages of 256 inner row slices, and
 // kProdPart of a step's 8 outer words, as two words each.
 constexpr u32 kProdSmem = 4 * 256 * 128 + 2 * kProdStep * 128 + 2 * kProdPart * kProdRows * 4;
@@ -68,9 +79,9 @@ struct ProdArgs {
   u32 *G;          // output rows: the output's NEWT or its transposed twin
   u8 *dirty;       // dirty map of G, or null
   LaunchRec *rows_rec;  // launch record of k_join_product_rows
+  u32 *list;       // [0]: long rows of OT, then (from [1]) those rows
   int dk;          // rows of 2^(dk-5) words
   u32 side;        // 256-id groups that hold ids
-  u32 ksteps;      // groups per unit of work (the key range is split)
   u32 splits;      // product_small: warps a row's keys are shared among
 };
 
@@ -105,32 +116,69 @@ __device__ __forceinline__ bool product_empty(const JoinArgs &j, u64 *n_outer) {
   return *n_outer == 0;
 }
 
-__device__ __forceinline__ bool prod_lists_keys(const ProdArgs &a, u64 n_outer) {
-  return a.dk >= kProdTableBits && n_outer * a.side * 32 <= kProdRowsBytes;
+// The long rows of OT, listed for k_join_product (which sets the count back
+// to zero), nearly in order: 32 rows a block, one atomic.
+__global__ void __launch_bounds__(256) k_prod_rows(ProdArgs a) {
+  __shared__ u32 s_any[8];
+  __shared__ u32 s_base;
+  if (ctl_stop(a.j.ctl)) return;
+  const u64 n_outer = eff_count(a.j.outer, a.j.outer_vis);
+  if (n_outer == 0 || eff_count(a.j.inner, a.j.inner_vis) == 0) return;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const u32 n4 = a.side * 2;
+  for (u32 g = blockIdx.x; g < a.side * 8; g += gridDim.x) {
+    u32 mask = 0;  // this warp's four rows
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const uint4 *p =
+          reinterpret_cast<const uint4 *>(a.OT + ((u64)(g * 32 + wid * 4 + q) << (a.dk - 5)));
+      u32 keys = 0;
+      for (u32 i = lane; i < n4; i += 32) {
+        const uint4 v = p[i];
+        keys += __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
+      }
+      if (!prod_short(__reduce_add_sync(0xffffffffu, keys), a.side)) mask |= 1u << q;
+    }
+    __syncthreads();
+    if (lane == 0) s_any[wid] = mask;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      const bool on = (s_any[lane >> 2] >> (lane & 3)) & 1u;
+      const u32 b = __ballot_sync(0xffffffffu, on);
+      if (lane == 0) s_base = b ? atomicAdd(&a.list[0], (u32)__popc(b)) : 0u;
+      __syncwarp();
+      if (on) a.list[1 + s_base + __popc(b & ((1u << lane) - 1u))] = g * 32 + lane;
+    }
+  }
 }
 
 __global__ void __launch_bounds__(kProdBlock, 1) k_join_product(ProdArgs a) {
   constexpr int RW = kProdWarpRows;
   constexpr u32 MR = kProdRows;
-  constexpr int RPT = MR / kProdBlock;  // outer rows loaded per thread
+  static_assert(MR == kProdBlock, "a thread loads one outer row");
+  constexpr u32 kNoRow = 0xFFFFFFFFu;
   constexpr int kPart = kProdPart;
   extern __shared__ __align__(128) u32 prod_mem[];
   u32 *tab = prod_mem;
   u32 *sB = tab + 4 * 256 * 32;
   u32 *sA = sB + 2 * kProdStep * 32;
   __shared__ u32 s_cnt[2][8];            // bits of the outer per word of keys
-  __shared__ u32 s_half[kProdWarps];     // inner rows with bits, 16 a warp
+  __shared__ u32 s_rows[8];              // inner rows with bits, per word of keys
   __shared__ long long s_unit;
   if (ctl_stop(a.j.ctl)) return;
   u64 n_outer;
   if (product_empty(a.j, &n_outer)) return;
-  if (prod_lists_keys(a, n_outer)) return;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int rs = a.dk - 5;
   const u32 row_words = 1u << rs;
   const u32 ids = a.side * 256;  // at most 2^dk
-  const u32 n_rb = (ids + MR - 1) / MR, n_sl = (ids + 1023) / 1024;
-  const u32 n_kc = (a.side + a.ksteps - 1) / a.ksteps;
+  const u32 n_rows = *((volatile u32 *)&a.list[0]);
+  const u32 n_rb = (n_rows + MR - 1) / MR, n_sl = (ids + 1023) / 1024;
+  // The key range is split until there are kProdUnits units a block: at 20,000
+  // ids 400 row-by-column blocks share 148 SMs unevenly (3 rounds for 2.7),
+  // and few long rows are few blocks.
+  const u32 ksteps = max(2u, a.side * n_rb * n_sl / (kProdUnits * gridDim.x));
+  const u32 n_kc = (a.side + ksteps - 1) / ksteps;
   const u32 units = n_rb * n_sl * n_kc;
   const u32 lane4 = lane * 4;
   u64 used = 0, flushed = 0;
@@ -140,21 +188,19 @@ __global__ void __launch_bounds__(kProdBlock, 1) k_join_product(ProdArgs a) {
     if (g >= (long long)units) break;
     const u32 u = (u32)g;
     const u32 kc = u % n_kc, sl = (u / n_kc) % n_sl, rb = u / n_kc / n_sl;
-    const u32 k0 = kc * a.ksteps, k1 = min(k0 + a.ksteps, a.side);
+    const u32 k0 = kc * ksteps, k1 = min(k0 + ksteps, a.side);
     u32 acc[RW];
 #pragma unroll
     for (int r = 0; r < RW; r++) acc[r] = 0;
-    u32 av[RPT][8];
+    // this thread's outer row (also lane l's: output row l of the warp)
+    const u32 my_row = rb * MR + tid < n_rows ? a.list[1 + rb * MR + tid] : kNoRow;
+    u32 av[8];
     auto load_a = [&](u32 s) {
+      if (my_row != kNoRow) {
+        load8(a.OT + ((u64)my_row << rs) + s * 8, av);
+      } else {
 #pragma unroll
-      for (int i = 0; i < RPT; i++) {
-        const u32 lr = tid + i * kProdBlock, row = rb * MR + lr;
-        if (row < ids) {
-          load8(a.OT + ((u64)row << rs) + s * 8, av[i]);
-        } else {
-#pragma unroll
-          for (int w = 0; w < 8; w++) av[i][w] = 0;
-        }
+        for (int w = 0; w < 8; w++) av[w] = 0;
       }
     };
     // 256 inner rows of 128 bytes (zeros past the row's end)
@@ -174,10 +220,7 @@ __global__ void __launch_bounds__(kProdBlock, 1) k_join_product(ProdArgs a) {
       const u32 st = (s - k0) & 1;
 #pragma unroll
       for (int w = 0; w < 8; w++) {
-        u32 c = 0;
-#pragma unroll
-        for (int i = 0; i < RPT; i++) c += __popc(av[i][w]);
-        c = __reduce_add_sync(0xffffffffu, c);
+        const u32 c = __reduce_add_sync(0xffffffffu, (u32)__popc(av[w]));
         if (lane == 0 && c) atomicAdd(&s_cnt[st][w], c);
       }
       asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -186,14 +229,12 @@ __global__ void __launch_bounds__(kProdBlock, 1) k_join_product(ProdArgs a) {
       for (int part = 0; part < 8; part += kPart) {
         // the outer's words of this part, as table offsets: bytes 0, 1 (times 128) in one word, bytes 2, 3 in the next
 #pragma unroll
-        for (int w = 0; w < kPart; w++)
-#pragma unroll
-          for (int i = 0; i < RPT; i++) {
-            const u32 lr = tid + i * kProdBlock, x = av[i][part + w];
-            reinterpret_cast<uint2 *>(sA)[w * MR + lr] =
-                make_uint2(((x & 0xFFu) << 7) | ((x & 0xFF00u) << 15),
-                           ((x >> 9) & 0x7F80u) | ((x >> 1) & 0x7F800000u));
-          }
+        for (int w = 0; w < kPart; w++) {
+          const u32 x = av[part + w];
+          reinterpret_cast<uint2 *>(sA)[w * MR + tid] =
+              make_uint2(((x & 0xFFu) << 7) | ((x & 0xFF00u) << 15),
+                         ((x >> 9) & 0x7F80u) | ((x >> 1) & 0x7F800000u));
+        }
         __syncthreads();  // the step's operands and counts
         if (part + kPart == 8 && s + 1 < k1) {
           load_a(s + 1);
@@ -206,23 +247,26 @@ __global__ void __launch_bounds__(kProdBlock, 1) k_join_product(ProdArgs a) {
           if (part == 0) {
             u32 m = 0;
 #pragma unroll
-            for (int j = 0; j < 16; j++)
-              if (__any_sync(0xffffffffu, B[(wid * 16 + j) * 32 + lane] != 0u)) m |= 1u << j;
-            if (lane == 0) s_half[wid] = m;
+            for (int j = 0; j < kProdStep / kProdWarps; j++)
+              if (__any_sync(0xffffffffu,
+                             B[(wid * (kProdStep / kProdWarps) + j) * 32 + lane] != 0u))
+                m |= 1u << j;
+            // (eight rows a warp: byte wid % 4 of word wid / 4)
+            if (lane == 0) reinterpret_cast<u8 *>(s_rows)[wid] = (u8)m;
             __syncthreads();
           }
           for (int wp = 0; wp < kPart; wp++) {
             const int w = part + wp;
             const u32 cnt = s_cnt[st][w];
-            const u32 bm = s_half[2 * w] | (s_half[2 * w + 1] << 16);
+            const u32 bm = s_rows[w];
             if (cnt == 0 || bm == 0) continue;  // (block-uniform)
             if (tid == 0) used += cnt;
             const u32 *Bw = B + w * 32 * 32 + lane;
             if (cnt > MR) {
               {
-                // warp wid: byte wid / 4, the 64 entries with top bits wid % 4
-                const u32 *r = Bw + (wid >> 2) * 8 * 32;
-                u32 lo[8], hi[8];
+                // warp wid: byte wid / 8, the 32 entries with top bits wid % 8
+                const u32 *r = Bw + (wid >> 3) * 8 * 32;
+                u32 lo[8], hi[4];
                 lo[0] = 0;
                 lo[1] = r[0];
                 lo[2] = r[32];
@@ -230,16 +274,15 @@ __global__ void __launch_bounds__(kProdBlock, 1) k_join_product(ProdArgs a) {
                 const u32 r2 = r[64];
 #pragma unroll
                 for (int i = 0; i < 4; i++) lo[4 + i] = lo[i] | r2;
-                hi[0] = ((wid & 1) ? r[6 * 32] : 0u) | ((wid & 2) ? r[7 * 32] : 0u);
+                hi[0] = ((wid & 1) ? r[5 * 32] : 0u) | ((wid & 2) ? r[6 * 32] : 0u) |
+                        ((wid & 4) ? r[7 * 32] : 0u);
                 hi[1] = hi[0] | r[96];
-                const u32 r4 = r[128], r5 = r[160];
+                const u32 r4 = r[128];
                 hi[2] = hi[0] | r4;
                 hi[3] = hi[1] | r4;
+                u32 *t = tab + ((wid >> 3) * 256 + (wid & 7) * 32) * 32 + lane;
 #pragma unroll
-                for (int i = 0; i < 4; i++) hi[4 + i] = hi[i] | r5;
-                u32 *t = tab + ((wid >> 2) * 256 + (wid & 3) * 64) * 32 + lane;
-#pragma unroll
-                for (int i = 0; i < 64; i++) t[i * 32] = lo[i & 7] | hi[i >> 3];
+                for (int i = 0; i < 32; i++) t[i * 32] = lo[i & 7] | hi[i >> 3];
               }
               __syncthreads();
               const char *tb = reinterpret_cast<const char *>(tab);
@@ -296,8 +339,9 @@ __global__ void __launch_bounds__(kProdBlock, 1) k_join_product(ProdArgs a) {
 #pragma unroll
     for (int r = 0; r < RW; r++) {
       const u32 v = acc[r];
+      const u32 row = __shfl_sync(0xffffffffu, my_row, r);
       if (v && col < row_words) {
-        const u64 gw = ((u64)(rb * MR + wid * RW + r) << rs) + col;
+        const u64 gw = ((u64)row << rs) + col;
         asm volatile("red.global.or.b32 [%0], %1;" ::"l"(a.G + gw), "r"(v) : "memory");
         if (a.dirty) a.dirty[gw / kBmChunkWords] = 1;
         flushed++;
@@ -310,8 +354,10 @@ __global__ void __launch_bounds__(kProdBlock, 1) k_join_product(ProdArgs a) {
   // used, 4 per word reduced into the output
   if (lane == 0) prof_add(a.j.ctl, kPJoinMat, 4 * flushed);
   if (tid == 0) prof_add(a.j.ctl, kPJoinMat, used * 128);
-  if (launch_rec_finish(a.j.rec) && tid == 0)
+  if (launch_rec_finish(a.j.rec) && tid == 0) {
+    a.list[0] = 0;
     prof_add(a.j.ctl, kPJoinMat, (u64)ids * a.side * 32);
+  }
 }
 
 // One warp: output row `row`, the keys of its words [w0, w1) (at most 32
@@ -419,7 +465,6 @@ __global__ void __launch_bounds__(kProdRowsBlock, V <= 8 ? 2 : 1) k_join_product
   const u64 n_outer = eff_count(a.j.outer, a.j.outer_vis);
   // (the launch before this one applied the empty-side rule)
   if (n_outer == 0 || eff_count(a.j.inner, a.j.inner_vis) == 0) return;
-  if (!prod_lists_keys(a, n_outer)) return;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   constexpr int kRows = kProdRowsBlock / 32;
   const int rs = a.dk - 5;
@@ -429,17 +474,20 @@ __global__ void __launch_bounds__(kProdRowsBlock, V <= 8 ? 2 : 1) k_join_product
   while (true) {
     const long long t = grab_tile(a.rows_rec, &s_tile);
     if (t >= (long long)tiles) break;
-    const u32 row0 = (u32)t * kRows;
+    // (rows of a tile lie far apart: long rows, often neighbours, go to
+    // different blocks)
+    auto row_no = [&](u32 r) { return (u32)t + r * tiles; };
     u32 w[V * 4];
     u32 left = 0;
     {
-      const uint4 *p = reinterpret_cast<const uint4 *>(a.OT + ((u64)(row0 + wid) << rs));
+      const uint4 *p = reinterpret_cast<const uint4 *>(a.OT + ((u64)row_no(wid) << rs));
 #pragma unroll
       for (int j = 0; j < V; j++) {
         const uint4 x = j * 32 + lane < n4 ? p[j * 32 + lane] : make_uint4(0, 0, 0, 0);
         w[4 * j] = x.x, w[4 * j + 1] = x.y, w[4 * j + 2] = x.z, w[4 * j + 3] = x.w;
         left += __popc(x.x) + __popc(x.y) + __popc(x.z) + __popc(x.w);
       }
+      if (!prod_short(__reduce_add_sync(0xffffffffu, left), a.side)) left = 0;
     }
     while (true) {
       // all keys that are left, or when they do not fit the list a share of
@@ -479,7 +527,7 @@ __global__ void __launch_bounds__(kProdRowsBlock, V <= 8 ? 2 : 1) k_join_product
         for (int j = 0; j < V; j++) b[j] = j * 32 + lane < n4 ? p[j * 32 + lane] : none;
       };
       auto flush = [&](u32 r) {
-        u32 *d = a.G + ((u64)(row0 + r) << rs);
+        u32 *d = a.G + ((u64)row_no(r) << rs);
 #pragma unroll
         for (int j = 0; j < V; j++) {
           const uint4 v = acc[j];
