@@ -120,7 +120,7 @@ __device__ __forceinline__ u32 closure_row(const ClosureArgs &a, bool on, u32 ro
 __global__ void __launch_bounds__(kLoopBlock, kClosureCtasPerSm) k_closure_loop(ClosureArgs a) {
   __shared__ int s_go;
   Ctl *ctl = a.loop.ctl;
-  u32 gen = ctl->bar_word >> 1;
+  u32 gen = ctl->bar_word >> 2;
   bool go = !ctl_stop(ctl);
   const int lane = threadIdx.x & 31;
   const LaneLists lists = lane_lists(a.loop.lie, lane);

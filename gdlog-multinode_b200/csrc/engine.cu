@@ -141,6 +141,7 @@ struct LieHost {
   bool closure = false;
   ClosureArgs cargs{};
   u32 *c_mem = nullptr;
+  HashJoinArgs *d_hops = nullptr;  // hash form: the joins, then relations with asides
   LoopStep *d_steps = nullptr;
   LoopUpd *d_upd = nullptr;
   int n_steps = 0, n_upd = 0;
@@ -319,7 +320,8 @@ struct gdl_engine {
   void *d_count = nullptr;    // gdl_join_count's scratch (CountScratch)
   void *d_part = nullptr;     // gdl_partition_rows: counts and cursors per destination
   u64 *d_u64 = nullptr;       // [4] small device scalars
-  u32 *d_u32 = nullptr;       // [4]: [0] pack check, [3] device checks of async loads (sticky)
+  u64 *h_scalars = nullptr;   // [4] pinned, for their read-back
+  u32 *d_u32 = nullptr;       // [4]: [3] device checks of async loads (sticky)
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // Graph capture runs on its own stream, so that the engine stream can run
   // a loop's first iteration meanwhile; ev_first marks that iteration's end.
@@ -853,22 +855,22 @@ u64 *sorted_location(gdl_engine *e, u64 *buf0) { return (sort_passes(e) & 1) ? e
 gdl_status launch_list(gdl_engine *e, const u32 *bm, u64 words, int rs, DArr *out,
                        int check_n);
 
-gdl_status load_keys(gdl_engine *e, int rel, const u64 *keys_dev, u64 n) {
+// keys_dev (from dalloc) becomes the relation's raw buffer.
+gdl_status load_keys(gdl_engine *e, int rel, u64 *keys_dev, u64 n) {
   RelHost &rh = e->rels[rel];
-  TRY(refresh_rel(e, rel));
+  if (const gdl_status s = refresh_rel(e, rel)) {
+    dfree(e, keys_dev);
+    return s;
+  }
   RelDev &r = e->h[rel];
   rh.bm_valid = false;
   rh.full_resident = false;
   rh.inv_ready = false;
   // raw := keys in load order
   if (rh.raw && !rh.raw_is_full) dfree(e, rh.raw);
-  rh.raw = nullptr;
+  rh.raw = keys_dev;
   rh.raw_n = n;
   rh.raw_is_full = false;
-  if (n) {
-    TRY(dalloc(e, (void **)&rh.raw, n * sizeof(u64)));
-    CK(e, cudaMemcpyAsync(rh.raw, keys_dev, n * sizeof(u64), cudaMemcpyDeviceToDevice, e->s));
-  }
   r.full.n = 0;
   r.delta.n = 0;
   r.newt.n = 0;
@@ -1610,7 +1612,8 @@ ProdArgs product_args(gdl_engine *e, LieHost &L, const Plan &plan, size_t oi, co
 // DELTAs, tmp NEWTs or static FULLs, so that no operator reads an update
 // relation's FULL, or a sorted DELTA, during the loop.
 bool hash_form(const gdl_engine *e, const LieHost &L, const Plan &plan) {
-  if (L.dense || e->instances || e->dedup_mode != 0 || L.update.empty()) return false;
+  if (L.dense || e->instances || e->dedup_mode != 0 || L.update.empty() || L.ops.empty())
+    return false;
   std::vector<char> is_update(e->rels.size(), 0), is_static(e->rels.size(), 0);
   for (int r : L.update) is_update[r] = 1;
   for (int r : L.statics) is_static[r] = 1;
@@ -1695,6 +1698,41 @@ HashJoinArgs hash_args(gdl_engine *e, const JoinArgs &a, int out, bool hashed) {
   h.need_delta = need_index(out, kNeedDelta);
   h.need_newt = need_index(out, kNeedNewt);
   return h;
+}
+
+// Join oi of a LIE in the hash form.
+HashJoinArgs hash_join_args(gdl_engine *e, LieHost &L, const Plan &plan, size_t oi) {
+  const OpHost &op = L.ops[oi];
+  bool hashed = false;
+  for (int r : L.update) hashed = hashed || r == op.out;
+  HashJoinArgs h = hash_args(e, join_args(e, L, plan, oi), op.out, hashed);
+  if (plan.static_once[oi]) {
+    h.j.once = &L.d_lie->jonce[oi];
+    h.j.once_pending = &L.d_lie->jonce_pending[oi];
+    h.j.produced = &L.d_lie->produced[oi];
+    h.j.phantom = &e->d_rels[op.out].newt_phantom;
+  }
+  return h;
+}
+
+// The hash form's resident loop: its joins, then an entry for each update
+// relation with dependent columns.
+gdl_status push_hash_loop(gdl_engine *e, LieHost &L, const Plan &plan) {
+  std::vector<HashJoinArgs> ops;
+  for (size_t oi = 0; oi < L.ops.size(); oi++) ops.push_back(hash_join_args(e, L, plan, oi));
+  for (int r : L.update)
+    if (e->rels[r].dep) {
+      JoinArgs a;
+      memset(&a, 0, sizeof a);
+      a.ctl = e->d_ctl;
+      ops.push_back(hash_args(e, a, r, true));
+    }
+  if (!L.d_hops)
+    TRY(dalloc(e, (void **)&L.d_hops, (kHashLoopOps + kMaxRels) * sizeof(HashJoinArgs)));
+  CK(e, cudaMemcpyAsync(L.d_hops, ops.data(), ops.size() * sizeof(HashJoinArgs),
+                        cudaMemcpyHostToDevice, e->s));
+  L.n_steps = (int)ops.size();
+  return GDL_OK;
 }
 
 // Whether the loop of this LIE runs as one resident kernel (loop.cuh).
@@ -1956,9 +1994,9 @@ gdl_status prepare_closure(gdl_engine *e, LieHost &L) {
   }
   k_closure_degree<<<grid_for(e, rows, 256, 4), 256, 0, e->s>>>(a.start, a.end, a.rows, maxdeg);
   e->aux_launches++;
-  u32 deg[2] = {0, 0};
-  CK(e, cudaMemcpyAsync(deg, maxdeg, sizeof deg, cudaMemcpyDeviceToHost, e->s));
+  CK(e, cudaMemcpyAsync(e->h_scalars, maxdeg, 2 * sizeof(u32), cudaMemcpyDeviceToHost, e->s));
   CK(e, cudaStreamSynchronize(e->s));
+  const u32 *deg = reinterpret_cast<const u32 *>(e->h_scalars);
   if (deg[0] > kClosureMaxDegree || deg[1]) return GDL_OK;
   RelDev &h = e->h[r];
   const u64 words = L.map.words;
@@ -2006,6 +2044,21 @@ gdl_status start_closure(gdl_engine *e, LieHost &L) {
 // most (all resident); fewer where a domain has less work than that (a
 // barrier's cost grows with its blocks).
 cudaError_t launch_loop(gdl_engine *e, LieHost &L, Counts *kc) {
+  if (L.hashed) {
+    HashLoopArgs a;
+    memset(&a, 0, sizeof a);
+    a.ops = L.d_hops;
+    a.n_ops = (int)L.ops.size();
+    a.n_all = L.n_steps;
+    a.rels = e->d_rels;
+    a.lie = L.d_lie;
+    a.ctl = e->d_ctl;
+    void *args[] = {&a};
+    kc->add(kPControl);
+    return cudaLaunchCooperativeKernel((const void *)k_hash_loop,
+                                       dim3((int)e->sms * kHashLoopCtasPerSm), dim3(256), args, 0,
+                                       e->s);
+  }
   if (L.closure) {
     ClosureArgs a;
     memcpy(&a, &L.cargs, sizeof a);
@@ -2132,15 +2185,7 @@ void enqueue_iteration(gdl_engine *e, LieHost &L, const Plan &plan, Counts *kc, 
       u64 outer_cap = std::max({oh.delta.cap, oh.delta_next.cap, oh.full.cap, oh.full_next.cap,
                                 oh.newt.cap});
       if (L.hashed) {
-        bool hashed = false;
-        for (int r : L.update) hashed = hashed || r == op.out;
-        if (plan.static_once[oi]) {
-          a.once = &L.d_lie->jonce[oi];
-          a.once_pending = &L.d_lie->jonce_pending[oi];
-          a.produced = &L.d_lie->produced[oi];
-          a.phantom = &R[op.out].newt_phantom;
-        }
-        HashJoinArgs ha = hash_args(e, a, op.out, hashed);
+        HashJoinArgs ha = hash_join_args(e, L, plan, oi);
         PLAUNCH(kc, kPJoinMat,
                 k_join_hash<<<grid_for(e, outer_cap, 256, 6), 256, 0, s>>>(ha));
         ha.j.rec = &e->recs[1];
@@ -3124,6 +3169,10 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
   L.graph_dirty = true;
   L.resident = L.closure || (use_graph && resident_loop(e, L, plan));
   if (L.resident && !L.closure) TRY(push_loop(e, L, plan));
+  if (use_graph && L.hashed && L.ops.size() <= (size_t)kHashLoopOps) {
+    L.resident = true;
+    TRY(push_hash_loop(e, L, plan));
+  }
   u64 batch = 4;
   bool first_batch = true;
   bool tail_listed = false;
@@ -3301,6 +3350,8 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
         TRY(reset_ctl(e));
         c.generation = e->generation;
         for (int r : L.update) TRY(fill_hash(e, r));
+        // (the scratch the joins write pieces to may have moved)
+        if (L.resident) TRY(push_hash_loop(e, L, plan));
       }
       if (L.dense && !resume) {
         // The iteration runs again from its start: its NEWT bitmaps must
@@ -3641,6 +3692,7 @@ gdl_status gdl_engine_create(int32_t device, void *stream, gdl_engine **out) {
       bad(cudaMalloc(&e->d_rels, kMaxRels * sizeof(RelDev))) ||
       bad(cudaMalloc(&e->d_ctl, sizeof(Ctl))) || bad(cudaMallocHost(&e->h_ctl, sizeof(Ctl))) ||
       bad(cudaMallocHost(&e->h_ctl2, sizeof(Ctl))) ||
+      bad(cudaMallocHost(&e->h_scalars, 4 * sizeof(u64))) ||
       bad(cudaMallocHost(&e->h_trace, kTraceRows * kMaxRels * 3 * sizeof(u64))) ||
       bad(cudaMallocHost(&e->h_rels_pin, kMaxRels * sizeof(RelDev))) ||
       bad(cudaMalloc(&e->recs, 16 * sizeof(LaunchRec))) ||
@@ -3709,7 +3761,7 @@ static void release_program(gdl_engine *e) {
     release_graph(e, L);
     // stream-ordered frees (a cudaFree would wait for the whole device)
     for (void *p : {(void *)L.d_trace, (void *)L.d_lie, (void *)L.d_joinrec, (void *)L.d_steps,
-                    (void *)L.d_upd, (void *)L.c_mem})
+                    (void *)L.d_upd, (void *)L.c_mem, (void *)L.d_hops})
       dfree(e, p);
     dfree(e, L.d_inst_delta);
     dfree(e, L.d_inst_last);
@@ -3811,6 +3863,7 @@ gdl_status gdl_engine_destroy(gdl_engine *e) {
   if (e->h_ctl2) cudaFreeHost(e->h_ctl2);
   if (e->h_trace) cudaFreeHost(e->h_trace);
   if (e->h_rels_pin) cudaFreeHost(e->h_rels_pin);
+  if (e->h_scalars) cudaFreeHost(e->h_scalars);
   if (e->pin_keys) cudaFreeHost(e->pin_keys);
   if (e->ev0) cudaEventDestroy(e->ev0);
   if (e->ev1) cudaEventDestroy(e->ev1);
@@ -3900,9 +3953,7 @@ static gdl_status load_common(gdl_engine *e, int32_t rel, const uint64_t *rows, 
     CK(e, cudaMemcpyAsync(dk, keys.data(), n * sizeof(u64), cudaMemcpyHostToDevice, e->s));
     e->max_value = std::max(e->max_value, m01);
     e->kbits = std::max(e->kbits, bits_for(e->max_value));
-    gdl_status s = load_keys(e, rel, dk, n);
-    dfree(e, dk);  // stream-ordered behind the load
-    return s;
+    return load_keys(e, rel, dk, n);
   }
   u64 *d_rows = nullptr, *d_keys = nullptr;
   u64 maxv = 0;
@@ -3921,14 +3972,16 @@ static gdl_status load_common(gdl_engine *e, int32_t rel, const uint64_t *rows, 
     CK(e, cudaMemcpyAsync(d_rows, rows, n * 2 * sizeof(u64), cudaMemcpyHostToDevice, e->s));
   }
   TRY(dalloc(e, (void **)&d_keys, n * sizeof(u64)));
-  CK(e, cudaMemsetAsync(e->d_u64, 0, sizeof(u64), e->s));
-  CK(e, cudaMemsetAsync(e->d_u32, 0, sizeof(u32), e->s));
-  k_pack_rows<<<grid_for(e, n, 256, 8), 256, 0, e->s>>>(d_rows, n, d_keys, e->d_u64, e->d_u32);
+  // largest value and range check, side by side: one clear, one read-back
+  CK(e, cudaMemsetAsync(e->d_u64, 0, 2 * sizeof(u64), e->s));
+  k_pack_rows<<<grid_for(e, n, 256, 8), 256, 0, e->s>>>(d_rows, n, d_keys, e->d_u64,
+                                                        reinterpret_cast<u32 *>(e->d_u64 + 1));
   CK(e, cudaGetLastError());
   if (on_device) {
-    CK(e, cudaMemcpyAsync(&maxv, e->d_u64, sizeof maxv, cudaMemcpyDeviceToHost, e->s));
-    CK(e, cudaMemcpyAsync(&badv, e->d_u32, sizeof badv, cudaMemcpyDeviceToHost, e->s));
+    CK(e, cudaMemcpyAsync(e->h_scalars, e->d_u64, 2 * sizeof(u64), cudaMemcpyDeviceToHost, e->s));
     CK(e, cudaStreamSynchronize(e->s));
+    maxv = e->h_scalars[0];
+    badv = (u32)e->h_scalars[1];
   }
   if (!on_device) dfree(e, d_rows);
   if (badv) {
@@ -3942,9 +3995,7 @@ static gdl_status load_common(gdl_engine *e, int32_t rel, const uint64_t *rows, 
   }
   e->max_value = std::max(e->max_value, maxv);
   e->kbits = std::max(e->kbits, bits_for(e->max_value));
-  gdl_status s = load_keys(e, rel, d_keys, n);
-  dfree(e, d_keys);
-  return s;
+  return load_keys(e, rel, d_keys, n);
 }
 
 gdl_status gdl_relation_load(gdl_engine *e, int32_t rel, const uint64_t *rows, uint64_t n) {

@@ -16,7 +16,8 @@
 //     reference does;
 //   * after the loop FULL is sorted once by the radix sort.
 // A candidate costs one random 8-byte access (an L2 hit while the set is
-// below 100 MB), whatever |FULL| is.
+// below 100 MB), whatever |FULL| is.  The iterations run in one resident
+// launch (k_hash_loop, as loop.cuh): a barrier an operator.
 //
 // Dependent columns (src/lie.cu:131-138): a tuple is new only if no FULL
 // tuple has its other columns, and tuples of one iteration that differ in
@@ -32,6 +33,7 @@
 #include "dense.cuh"
 #include "index.cuh"
 #include "join.cuh"
+#include "loop.cuh"
 
 namespace gdl {
 
@@ -167,11 +169,14 @@ __device__ __forceinline__ void hash_emit(const HashJoinArgs &a, WarpOut &w, u32
 // A join's candidates into a hash set or a tmp list: probe and expand as
 // k_join_bm (dense.cuh), 32 candidates of a warp's 32 outer rows a step; runs
 // longer than kHeavyRun are cut into pieces for k_join_hash_heavy.
-__global__ void __launch_bounds__(256) k_join_hash(HashJoinArgs a) {
-  __shared__ FuseSmem<256> sm;
-  __shared__ WarpOut s_out[8];
+struct HashSmem {
+  FuseSmem<256> fuse;
+  WarpOut out[8];
+};
+__device__ __forceinline__ void hash_join(const HashJoinArgs &a, HashSmem &hs) {
+  FuseSmem<256> &sm = hs.fuse;
+  WarpOut *s_out = hs.out;
   const JoinArgs &j = a.j;
-  if (ctl_stop(j.ctl)) return;
   const u64 n_outer = eff_count(j.outer, j.outer_vis);
   const u64 n_inner = eff_count(j.inner, j.inner_vis);
   if (n_outer == 0 || n_inner == 0) {
@@ -252,17 +257,15 @@ __global__ void __launch_bounds__(256) k_join_hash(HashJoinArgs a) {
   if (lane == 0) prof_add(j.ctl, kPJoinMat, cand * 16);
   if (blockIdx.x == 0 && threadIdx.x == 0) prof_add(j.ctl, kPJoinMat, n_outer * 24);
 }
+__global__ void __launch_bounds__(256) k_join_hash(HashJoinArgs a) {
+  __shared__ HashSmem sm;
+  if (ctl_stop(a.j.ctl)) return;
+  hash_join(a, sm);
+}
 
-// The pieces of long runs, a block per piece; the last block empties the
-// piece list.  (An overflow may be raised while blocks of this launch are
-// still starting: every block comes to the end.)
-__global__ void __launch_bounds__(256) k_join_hash_heavy(HashJoinArgs a) {
-  __shared__ int s_stop;
-  __shared__ WarpOut s_out[8];
+// The first np pieces of long runs, a block per piece.
+__device__ __forceinline__ void hash_heavy(const HashJoinArgs &a, u64 np, WarpOut *s_out) {
   const JoinArgs &j = a.j;
-  if (threadIdx.x == 0) s_stop = ctl_stop(j.ctl);
-  __syncthreads();
-  const u64 np = s_stop ? 0 : min(j.op->nc, j.crow_cap);
   const u64 *inner = j.inner->ptr;
   u64 cand = 0;
   bool emitted = false;
@@ -290,15 +293,22 @@ __global__ void __launch_bounds__(256) k_join_hash_heavy(HashJoinArgs a) {
     if (j.produced) *j.produced = 1;
   }
   if (threadIdx.x == 0) prof_add(j.ctl, kPJoinMat, cand * 16);
-  if (launch_rec_finish(j.rec) && threadIdx.x == 0) j.op->nc = 0;
+}
+// (The last block empties the piece list.  An overflow may be raised while
+// blocks of this launch are still starting: every block comes to the end.)
+__global__ void __launch_bounds__(256) k_join_hash_heavy(HashJoinArgs a) {
+  __shared__ int s_stop;
+  __shared__ WarpOut s_out[8];
+  if (threadIdx.x == 0) s_stop = ctl_stop(a.j.ctl);
+  __syncthreads();
+  hash_heavy(a, s_stop ? 0 : min(a.j.op->nc, a.j.crow_cap), s_out);
+  if (launch_rec_finish(a.j.rec) && threadIdx.x == 0) a.j.op->nc = 0;
 }
 
 // The candidates put aside: new unless a tuple of their prefix was in FULL
 // when the iteration began; each kept once.  (A slot taken by this launch or
 // the joins has an ordinal from FULL's count on, or none yet.)
-__global__ void __launch_bounds__(256) k_hash_aside(HashJoinArgs a) {
-  __shared__ WarpOut s_out[8];
-  if (ctl_stop(a.j.ctl)) return;
+__device__ __forceinline__ void hash_aside(const HashJoinArgs &a, WarpOut *s_out) {
   RelDev *r = a.out;
   u32 waiting = 0;
   const u64 n = min(r->newt.n, r->newt.cap);
@@ -329,6 +339,92 @@ __global__ void __launch_bounds__(256) k_hash_aside(HashJoinArgs a) {
     hash_put(a, true, s_out[threadIdx.x >> 5], waiting, is_new, k, slot);
   }
   hash_flush(a, true, s_out[threadIdx.x >> 5], waiting);
+}
+__global__ void __launch_bounds__(256) k_hash_aside(HashJoinArgs a) {
+  __shared__ WarpOut s_out[8];
+  if (ctl_stop(a.j.ctl)) return;
+  hash_aside(a, s_out);
+}
+
+constexpr int kHashLoopOps = 16;
+constexpr int kHashLoopCtasPerSm = 4;
+
+struct HashLoopArgs {
+  const HashJoinArgs *ops;  // n_ops joins, then (to n_all) the relations whose
+  int n_ops, n_all;         // candidates may be put aside
+  RelDev *rels;
+  LieDev *lie;
+  Ctl *ctl;
+};
+
+// Every iteration of a LIE.  A join's barrier tells whether it left pieces of
+// long runs, the last join's whether candidates were put aside; when neither,
+// that barrier commits.  An overflow ends the loop uncommitted.
+__global__ void __launch_bounds__(256, kHashLoopCtasPerSm) k_hash_loop(HashLoopArgs a) {
+  __shared__ HashSmem sm;
+  __shared__ int s_go;
+  Ctl *ctl = a.ctl;
+  u32 gen = ctl->bar_word >> 2;
+  u32 flags = ctl_stop(ctl) ? 1u : 0u;
+  auto aside_left = [&]() {
+    bool any = false;
+    for (int i = a.n_ops; i < a.n_all; i++) any |= *((volatile u64 *)&a.ops[i].out->newt.n) != 0;
+    return any;
+  };
+  // (every lane of the warp sees the same words)
+  auto finish = [&](int lane) -> u32 {
+    return commit_iteration(a.rels, a.lie, ctl, 1, lane) ? 1u : 0u;
+  };
+  while (!(flags & 1u)) {
+    bool committed = false;
+    for (int i = 0; i < a.n_ops && !(flags & 1u); i++) {
+      const HashJoinArgs &op = a.ops[i];
+      const bool last = i == a.n_ops - 1;
+      hash_join(op, sm);
+      // bit 1: more to do before the next join (or the commit)
+      flags = loop_barrier_flags(ctl, gen, &s_go, [&](int lane) -> u32 {
+        if (*((volatile u32 *)&ctl->overflow)) return 1u;
+        if (*((volatile u64 *)&op.j.op->nc)) return 2u;
+        if (!last) return 0u;
+        return aside_left() ? 2u : finish(lane);
+      });
+      if (flags & 1u) break;
+      if (!(flags & 2u)) {
+        committed = last;
+        continue;
+      }
+      const u64 np = min(*((volatile u64 *)&op.j.op->nc), op.j.crow_cap);
+      if (np) {
+        hash_heavy(op, np, sm.out);
+        flags = loop_barrier_flags(ctl, gen, &s_go, [&](int lane) -> u32 {
+          if (lane == 0) op.j.op->nc = 0;
+          if (*((volatile u32 *)&ctl->overflow)) return 1u;
+          if (!last) return 0u;
+          return aside_left() ? 2u : finish(lane);
+        });
+        if (flags & 1u) break;
+        if (!(flags & 2u)) {
+          committed = last;
+          continue;
+        }
+      }
+    }
+    if ((flags & 1u) || committed) continue;
+    for (int i = a.n_ops; i < a.n_all && !(flags & 1u); i++) {
+      hash_aside(a.ops[i], sm.out);
+      const bool end = i == a.n_all - 1;
+      flags = loop_barrier_flags(ctl, gen, &s_go, [&](int lane) -> u32 {
+        if (*((volatile u32 *)&ctl->overflow)) return 1u;
+        return end ? finish(lane) : 0u;
+      });
+    }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (*((volatile u32 *)&ctl->overflow))  // (pieces of an iteration that runs again)
+      for (int i = 0; i < a.n_ops; i++) a.ops[i].j.op->nc = 0;
+    if (ctl->cond_set)
+      cudaGraphSetConditional((cudaGraphConditionalHandle)ctl->cond_handle, 0u);
+  }
 }
 
 // The set of FULL's committed rows (the set is all empty when this starts;

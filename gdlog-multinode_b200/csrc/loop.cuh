@@ -82,12 +82,12 @@ struct LoopArgs {
 };
 
 // Grid barrier, all threads of all blocks.  The last block's first warp runs
-// fin(lane), which returns whether the loop stops.  One round trip to count
-// arrivals and one to see the word the last block releases, which carries
-// the barrier's number and the stop bit.  False when the loop stops (its
-// end, or a wait that gave up).
+// fin(lane), which returns flags every block gets: bit 0 stops the loop, bit 1
+// is the caller's.  One round trip to count arrivals and one to see the word
+// the last block releases, which carries the barrier's number and the flags.
+// A wait that gives up returns the stop bit.
 template <class Fin>
-__device__ __forceinline__ bool loop_barrier(Ctl *ctl, u32 &gen, int *s_go, Fin fin) {
+__device__ __forceinline__ u32 loop_barrier_flags(Ctl *ctl, u32 &gen, int *s_go, Fin fin) {
   __syncthreads();
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
@@ -101,13 +101,14 @@ __device__ __forceinline__ bool loop_barrier(Ctl *ctl, u32 &gen, int *s_go, Fin 
       last = before == gridDim.x - 1;
     }
     last = __shfl_sync(0xffffffffu, last, 0);
+    __syncwarp();
     u32 word = 0;
     if (last) {
-      const bool stop = fin(lane);
+      const u32 flags = fin(lane);
       __syncwarp();
       if (lane == 0) {
         ctl->bar_count = 0;
-        word = ((gen + 1) << 1) | (stop ? 1u : 0u);
+        word = ((gen + 1) << 2) | flags;
         asm volatile("st.release.gpu.u32 [%0], %1;" ::"l"(&ctl->bar_word),
                      "r"(word)
                      : "memory");
@@ -116,7 +117,7 @@ __device__ __forceinline__ bool loop_barrier(Ctl *ctl, u32 &gen, int *s_go, Fin 
       const u32 limit = ctl->spin_limit;
       for (u32 polls = 0;; polls++) {
         asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(word) : "l"(&ctl->bar_word) : "memory");
-        if ((word >> 1) != gen) break;
+        if ((word >> 2) != gen) break;
         if ((polls & 63u) == 63u && *((volatile u32 *)&ctl->timeout)) {
           word = 1;
           break;
@@ -128,11 +129,16 @@ __device__ __forceinline__ bool loop_barrier(Ctl *ctl, u32 &gen, int *s_go, Fin 
         }
       }
     }
-    if (lane == 0) *s_go = !(word & 1u);
+    if (lane == 0) *s_go = (int)(word & 3u);
   }
   __syncthreads();
-  gen = (gen + 1) & 0x7FFFFFFFu;
-  return *s_go != 0;
+  gen = (gen + 1) & 0x3FFFFFFFu;
+  return (u32)*s_go;
+}
+// ... with fin returning whether the loop stops; false when it does.
+template <class Fin>
+__device__ __forceinline__ bool loop_barrier(Ctl *ctl, u32 &gen, int *s_go, Fin fin) {
+  return !(loop_barrier_flags(ctl, gen, s_go, [&](int lane) { return fin(lane) ? 1u : 0u; }) & 1u);
 }
 
 // k_commit's bookkeeping (control.cuh) for relations kept as bitmaps with
@@ -377,7 +383,7 @@ __global__ void __launch_bounds__(kLoopBlock, 2) k_lie_loop(LoopArgs a) {
   __shared__ LoopUpd s_upd[kLoopMaxUpd];
   __shared__ int s_go;
   Ctl *ctl = a.ctl;
-  u32 gen = ctl->bar_word >> 1;  // (it cannot change before this block arrives)
+  u32 gen = ctl->bar_word >> 2;  // (it cannot change before this block arrives)
   bool go = !ctl_stop(ctl);
   const int rs = a.dk - 5;
   const LaneLists lists = lane_lists(a.lie, threadIdx.x & 31);
