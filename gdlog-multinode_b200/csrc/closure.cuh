@@ -181,7 +181,9 @@ __global__ void __launch_bounds__(kLoopBlock, kClosureCtasPerSm) k_closure_loop(
       atomicAdd((unsigned long long *)&a.rd->scan.total_a, (unsigned long long)n_new);
     if (__any_sync(0xffffffffu, found) && lane == 0) a.rd->scan.pop_g = 1;  // NEWT is not empty
     go = loop_barrier(ctl, gen, &s_go,
-                      [&](int ln) { return loop_commit(a.loop, lists, ln); });
+                      [&](int ln) {
+                        return loop_commit<false>(a.loop.rels, a.loop.lie, ctl, lists, ln);
+                      });
   }
   if (blockIdx.x == 0 && threadIdx.x == 0 && ctl->cond_set)
     cudaGraphSetConditional((cudaGraphConditionalHandle)ctl->cond_handle, 0u);

@@ -362,31 +362,42 @@ struct HashLoopArgs {
 // that barrier commits.  An overflow ends the loop uncommitted.
 __global__ void __launch_bounds__(256, kHashLoopCtasPerSm) k_hash_loop(HashLoopArgs a) {
   __shared__ HashSmem sm;
+  __shared__ HashJoinArgs s_op[kHashLoopOps];
   __shared__ int s_go;
+  for (u32 i = threadIdx.x; i < a.n_ops * sizeof(HashJoinArgs) / 4; i += 256)
+    reinterpret_cast<u32 *>(s_op)[i] = reinterpret_cast<const u32 *>(a.ops)[i];
+  __syncthreads();
   Ctl *ctl = a.ctl;
   u32 gen = ctl->bar_word >> 2;
   u32 flags = ctl_stop(ctl) ? 1u : 0u;
-  auto aside_left = [&]() {
-    bool any = false;
-    for (int i = a.n_ops; i < a.n_all; i++) any |= *((volatile u64 *)&a.ops[i].out->newt.n) != 0;
-    return any;
-  };
-  // (every lane of the warp sees the same words)
+  const LaneLists lists = lane_lists(a.lie, threadIdx.x & 31);
+  // the asides' counts, a relation a lane
+  const u64 *aside_n = nullptr;
+  if ((int)(threadIdx.x & 31) < a.n_all - a.n_ops)
+    aside_n = &a.ops[a.n_ops + (threadIdx.x & 31)].out->newt.n;
   auto finish = [&](int lane) -> u32 {
-    return commit_iteration(a.rels, a.lie, ctl, 1, lane) ? 1u : 0u;
+    return loop_commit<true>(a.rels, a.lie, ctl, lists, lane) ? 1u : 0u;
+  };
+  // What the last block decides after a join: 1 an overflow ends the loop, 2
+  // pieces (nc) or, after the last join, asides are left, else it may commit.
+  // One round trip: every word is loaded before one is looked at.
+  auto decide = [&](int lane, const u64 *nc, bool last) -> u32 {
+    const u64 left = nc ? *((volatile const u64 *)nc) : 0;
+    const u64 put = aside_n ? *((volatile const u64 *)aside_n) : 0;
+    if (*((volatile u32 *)&ctl->overflow)) return 1u;
+    if (left) return 2u;
+    if (!last) return 0u;
+    return __any_sync(0xffffffffu, put != 0) ? 2u : finish(lane);
   };
   while (!(flags & 1u)) {
     bool committed = false;
     for (int i = 0; i < a.n_ops && !(flags & 1u); i++) {
-      const HashJoinArgs &op = a.ops[i];
+      const HashJoinArgs &op = s_op[i];
       const bool last = i == a.n_ops - 1;
       hash_join(op, sm);
       // bit 1: more to do before the next join (or the commit)
       flags = loop_barrier_flags(ctl, gen, &s_go, [&](int lane) -> u32 {
-        if (*((volatile u32 *)&ctl->overflow)) return 1u;
-        if (*((volatile u64 *)&op.j.op->nc)) return 2u;
-        if (!last) return 0u;
-        return aside_left() ? 2u : finish(lane);
+        return decide(lane, &op.j.op->nc, last);
       });
       if (flags & 1u) break;
       if (!(flags & 2u)) {
@@ -398,9 +409,7 @@ __global__ void __launch_bounds__(256, kHashLoopCtasPerSm) k_hash_loop(HashLoopA
         hash_heavy(op, np, sm.out);
         flags = loop_barrier_flags(ctl, gen, &s_go, [&](int lane) -> u32 {
           if (lane == 0) op.j.op->nc = 0;
-          if (*((volatile u32 *)&ctl->overflow)) return 1u;
-          if (!last) return 0u;
-          return aside_left() ? 2u : finish(lane);
+          return decide(lane, nullptr, last);
         });
         if (flags & 1u) break;
         if (!(flags & 2u)) {

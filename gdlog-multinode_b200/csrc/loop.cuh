@@ -143,20 +143,26 @@ __device__ __forceinline__ bool loop_barrier(Ctl *ctl, u32 &gen, int *s_go, Fin 
 
 // k_commit's bookkeeping (control.cuh) for relations kept as bitmaps with
 // the fused update step, then the next iteration's opening.  One warp; every
-// load of a lane is issued before any of them is used.  DELTA's lists are
-// not written during the loop, so nothing is swapped: only counts change.
-__device__ __forceinline__ bool loop_commit(const LoopArgs &a, const LaneLists &x, int lane) {
-  Ctl *ctl = a.ctl;
+// load of a lane is issued before any of them is used.  With bitmaps DELTA's
+// lists are not written during the loop and only counts change; the hash
+// form (hash.cuh) swaps its two DELTA lists.
+template <bool HASH>
+__device__ __forceinline__ bool loop_commit(RelDev *rels, LieDev *lie, Ctl *ctl,
+                                            const LaneLists &x, int lane) {
   const u64 it = ctl->iteration, trace_base = ctl->trace_base, trace_rows = ctl->trace_rows;
   const u64 max_it = ctl->max_iteration, stop_at = ctl->stop_at;
-  u64 *trace = a.lie->trace;
+  u64 *trace = lie->trace;
   bool grew = false;
 #pragma unroll
   for (int j = 0; j < kListPerLane; j++) {
     const int i = lane + 32 * j;
     if (i < x.nu) {
-      RelDev &r = a.rels[x.upd[j]];
-      const u64 nd = r.scan.total_a, nn = r.scan.pop_g, nf = r.full.n;
+      RelDev &r = rels[x.upd[j]];
+      const u64 nd = HASH ? r.delta_next.n : r.scan.total_a;
+      const u64 nn = HASH ? r.c_newt_n : r.scan.pop_g, nf = r.full.n;
+      u64 *dp = nullptr, *np = nullptr;
+      u64 dc = 0, nc = 0;
+      if (HASH) dp = r.delta.ptr, dc = r.delta.cap, np = r.delta_next.ptr, nc = r.delta_next.cap;
       const u32 ph = r.newt_phantom, wv = r.w_full_vis;
       const u64 row = it - trace_base;
       u64 *tr = (trace && row < trace_rows) ? trace + (row * x.nu + i) * 3 : nullptr;
@@ -173,29 +179,35 @@ __device__ __forceinline__ bool loop_commit(const LoopArgs &a, const LaneLists &
         tr[1] = dn;
         tr[2] = nf + dn;
       }
-      r.scan.total_a = 0;
-      r.scan.pop_g = 0;
+      if (HASH) {
+        if (!none) r.delta.ptr = np, r.delta.cap = nc, r.delta_next.ptr = dp, r.delta_next.cap = dc;
+        r.delta_next.n = 0;
+        r.c_newt_n = 0;
+      } else {
+        r.scan.total_a = 0;
+        r.scan.pop_g = 0;
+      }
       r.newt.n = 0;
       r.newt_phantom = 0;
     }
     if (i < x.ns) {
-      RelDev &r = a.rels[x.sta[j]];
+      RelDev &r = rels[x.sta[j]];
       const u32 f = r.w_full_vis, d = r.w_delta_vis;
       r.full_vis = f;
       r.delta_vis = d;
     }
     if (i < x.nt) {
-      RelDev &r = a.rels[x.tmp[j]];
+      RelDev &r = rels[x.tmp[j]];
       const u32 f = r.full_vis, d = r.delta_vis;
       r.newt.n = 0;  // src/lie.cu:85-87
       r.w_full_vis = f;
       r.w_delta_vis = d;
     }
     if (i < x.no) {
-      const u32 p = a.lie->jonce_pending[i];
+      const u32 p = lie->jonce_pending[i];
       if (p) {
-        a.lie->jonce[i] |= p;
-        a.lie->jonce_pending[i] = 0;
+        lie->jonce[i] |= p;
+        lie->jonce_pending[i] = 0;
       }
     }
   }
@@ -505,7 +517,7 @@ __global__ void __launch_bounds__(kLoopBlock, 2) k_lie_loop(LoopArgs a) {
         if (nn) atomicAdd((unsigned long long *)&u.rd->scan.pop_g, (unsigned long long)nn);
       }
     }
-    go = loop_barrier(ctl, gen, &s_go, [&](int lane) { return loop_commit(a, lists, lane); });
+    go = loop_barrier(ctl, gen, &s_go, [&](int lane) { return loop_commit<false>(a.rels, a.lie, ctl, lists, lane); });
   }
   if (blockIdx.x == 0 && threadIdx.x == 0 && ctl->cond_set)
     cudaGraphSetConditional((cudaGraphConditionalHandle)ctl->cond_handle, 0u);
