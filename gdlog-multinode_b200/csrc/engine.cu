@@ -1652,6 +1652,21 @@ gdl_status ensure_hash(gdl_engine *e, int r) {
   if (dep && !h.hord) TRY(dalloc(e, (void **)&h.hord, (h.hmask + 2) * sizeof(u32)));
   return GDL_OK;
 }
+// Lists and sets of a LIE in the hash form: room for a few million tuples
+// before the first growth.
+gdl_status prepare_hash(gdl_engine *e, LieHost &L) {
+  for (int r : L.update) {
+    RelDev &h = e->h[r];
+    TRY(ensure_arr(e, h.full, std::max<u64>(kHashMinRows, std::min<u64>(2 * h.full.n, kMaxRows)),
+                   true));
+    TRY(ensure_arr(e, h.delta, kHashMinRows, true));
+    TRY(ensure_arr(e, h.delta_next, h.delta.cap, false));
+    TRY(ensure_hash(e, r));
+    h.dense = h.full_lazy = 1;  // (the commit only counts FULL's new rows)
+  }
+  for (int r : L.tmps) TRY(ensure_arr(e, e->h[r].newt, kHashMinRows, false));
+  return GDL_OK;
+}
 u64 hash_prefix(const gdl_engine *e, int r) { return ~dep_low_mask(e, e->rels[r]); }
 gdl_status fill_hash(gdl_engine *e, int r) {
   const RelDev &h = e->h[r];
@@ -2984,20 +2999,24 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
   }
   const bool use_graph = getenv("GDLOG_NO_GRAPH") == nullptr && !e->profile;
   L.closure = false;
-  if (use_graph && closure_form(e, L)) TRY(prepare_closure(e, L));
+  if (use_graph && closure_form(e, L)) {
+    const gdl_status cs = prepare_closure(e, L);
+    if (cs == GDL_E_NOMEM)
+      cudaGetLastError();  // (no room for its arrays: the general path)
+    else
+      TRY(cs);
+  }
   mark("dense_alloc");
   L.hashed = hash_form(e, L, plan);
   if (L.hashed) {
-    // room for a few million tuples before the first growth
-    for (int r : L.update) {
-      RelDev &h = e->h[r];
-      TRY(ensure_arr(e, h.full, std::max<u64>(kHashMinRows, 2 * h.full.n), true));
-      TRY(ensure_arr(e, h.delta, kHashMinRows, true));
-      TRY(ensure_arr(e, h.delta_next, h.delta.cap, false));
-      TRY(ensure_hash(e, r));
-      h.dense = h.full_lazy = 1;  // (the commit only counts FULL's new rows)
+    const gdl_status hs = prepare_hash(e, L);
+    if (hs == GDL_E_NOMEM) {
+      cudaGetLastError();  // (no room for the sets: sorted lists)
+      L.hashed = false;
+      for (int r : L.update) e->h[r].dense = e->h[r].full_lazy = 0;
+    } else {
+      TRY(hs);
     }
-    for (int r : L.tmps) TRY(ensure_arr(e, e->h[r].newt, kHashMinRows, false));
   }
   TRY(ensure_scratch(e));
   mark("scratch");
@@ -3215,6 +3234,11 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
                           cudaMemcpyDeviceToHost, e->s));
     return GDL_OK;
   };
+  // A resident loop's blocks wait for one another, so all of them must be on
+  // the GPU: engines of one process run such loops one at a time per device
+  // (each fills the GPU anyhow).
+  static std::mutex resident_mu[64];
+  std::unique_lock<std::mutex> resident_lock(resident_mu[e->device & 63], std::defer_lock);
   while (true) {
     c.pause = 0;
     c.stop_at = c.iteration + (use_graph ? std::min<u64>(trace_rows, 1u << 20) : batch);
@@ -3270,6 +3294,7 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
       k_begin<<<1, 32, 0, e->s>>>(e->d_rels, L.d_lie, e->d_ctl);
       L.kernels++;
       e->prof_launches[kPControl]++;
+      if (L.resident) resident_lock.lock();
       CK(e, cudaGraphLaunch(L.gexec, e->s));
       L.graph_launches++;
     } else if (!use_graph) {
@@ -3289,6 +3314,7 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
     }
     TRY(enqueue_tail(it0, c.stop_at));
     CK(e, cudaStreamSynchronize(e->s));
+    if (resident_lock.owns_lock()) resident_lock.unlock();
     prof_collect(e);
     c = *e->h_ctl;
     e->generation = c.generation;

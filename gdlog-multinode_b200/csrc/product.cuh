@@ -444,10 +444,10 @@ __global__ void __launch_bounds__(256) k_join_product_small(ProdArgs a) {
   product_small(a, blockIdx.x);
 }
 
-// Warps a row's keys are shared among: about 2,048 warps over all rows, at
-// most 32 words of keys each.
+// Warps a row's keys are shared among: 8 words of keys (256) each from 2^10
+// ids on, 4 below, so that a full row is at most 64 rounds of four reads.
 __host__ __device__ constexpr u32 prod_small_splits(u32 side) {
-  return side >= 8 ? 2 : side >= 4 ? 2 : side == 3 ? 3 : side == 2 ? 4 : 2;
+  return side >= 4 ? side : 2 * side;
 }
 
 constexpr int kProdRowsBlock = 256;
