@@ -990,6 +990,9 @@ struct Plan {
   std::vector<char> twin_zero;
   // per op: pull form computed as a boolean product (product.cuh)
   std::vector<char> product;
+  // per op: a product over a tmp NEWT whose tuples mostly repeat from one
+  // iteration to the next (product.cuh)
+  std::vector<char> repeats;
   // per op: a row-gather join writing an update relation's NEWT directly,
   // first of the iteration's ops to write that relation (the update step
   // leaves NEWT zero, so its rows are zero when the join starts)
@@ -1021,6 +1024,7 @@ Plan make_plan(gdl_engine *e, const LieHost &L) {
   p.twin_zero.assign(L.ops.size(), 0);
   p.g_zero.assign(L.ops.size(), 0);
   p.product.assign(L.ops.size(), 0);
+  p.repeats.assign(L.ops.size(), 0);
   {
     std::vector<char> is_static(n, 0), is_update(n, 0), newt_read(n, 0);
     for (int r : L.statics) is_static[r] = 1;
@@ -1165,6 +1169,33 @@ void plan_pull(const gdl_engine *e, const LieHost &L, Plan &p) {
     if (op.kind == 0 && op.inner_ver != GDL_DELTA && !p.product[oi] && !p.rows[oi])
       p.full_idx[op.inner] = 1;
   }
+  // Products over a tmp NEWT that leave out what the iteration before joined:
+  // the output is an update relation whose NEWT nothing reads (a tuple that
+  // is in its FULL need not appear there again), the tmp has this one reader,
+  // the inner keeps its DELTA transposed, and no join can hide the inner's
+  // FULL for an iteration (src/join.cu:42-45 zeroes an outer's count).
+  if (L.dk >= kProdTableBits)
+    for (size_t oi = 0; oi < L.ops.size(); oi++) {
+      const OpHost &op = L.ops[oi];
+      if (!p.product[oi] || op.outer_ver != GDL_NEWT || !is_update[op.inner] || !is_update[op.out] ||
+          p.acopy_src[op.out] || !p.fused[op.inner] || !p.fused[op.out])
+        continue;
+      int readers = 0;
+      bool ok = true, delta_t = false;
+      for (size_t oj = 0; oj < L.ops.size(); oj++) {
+        const OpHost &q = L.ops[oj];
+        if (q.kind == 0 && q.outer_ver == GDL_NEWT && q.outer == op.outer) readers++;
+        if (q.kind != 0 && q.inner == op.outer) ok = false;
+        if (q.kind == 0 && q.outer_ver == GDL_NEWT && q.outer == op.out) ok = false;
+        if (q.kind == 1 && q.inner_ver == GDL_NEWT && q.inner == op.out) ok = false;
+        if (q.kind == 0 && q.outer_ver == GDL_FULL && q.outer == op.inner) ok = false;
+        if (p.pull[oj] && !p.rows[oj] && q.outer_ver == GDL_DELTA && q.outer == op.inner)
+          delta_t = true;
+      }
+      p.repeats[oi] = ok && readers == 1 && delta_t;
+      // (its second product writes the other orientation)
+      if (p.repeats[oi]) p.out_t[op.out] = 1;
+    }
   // Which orientations of DELTA and NEWT the joins read.  A fused update
   // step keeps DELTA as rows when nothing reads it transposed (the record
   // from which the list is written if max_iteration leaves a DELTA).
@@ -1186,7 +1217,7 @@ void plan_pull(const gdl_engine *e, const LieHost &L, Plan &p) {
       continue;
     bool only_t = true;
     for (size_t oi = 0; oi < L.ops.size(); oi++)
-      if (L.ops[oi].out == r && !p.out_twin[oi]) only_t = false;
+      if (L.ops[oi].out == r && (!p.out_twin[oi] || p.repeats[oi])) only_t = false;
     p.fold_late[r] = only_t;
   }
   // A transposed twin is zero when the op that writes it starts: folded
@@ -1228,8 +1259,11 @@ void plan_pull(const gdl_engine *e, const LieHost &L, Plan &p) {
 }
 
 // Transposed bitmaps of the relations pull-form joins read.
-gdl_status ensure_tbitmaps(gdl_engine *e, const Plan &p, int r, u64 words) {
+gdl_status ensure_tbitmaps(gdl_engine *e, const LieHost &L, const Plan &p, int r, u64 words) {
   RelDev &h = e->h[r];
+  for (size_t oi = 0; oi < L.ops.size(); oi++)  // the fresh part of a repeated NEWT
+    if (p.repeats[oi] && L.ops[oi].outer == r && !h.bmDT)
+      TRY(dalloc(e, (void **)&h.bmDT, words * 4));
   if (p.delta_n[r] && !h.bmDN) TRY(dalloc(e, (void **)&h.bmDN, words * 4));
   if (p.delta_t[r] && !h.bmDT) TRY(dalloc(e, (void **)&h.bmDT, words * 4));
   if (p.newt_t[r] && !h.bmGT) TRY(dalloc(e, (void **)&h.bmGT, words * 4));
@@ -2168,6 +2202,10 @@ void enqueue_iteration(gdl_engine *e, LieHost &L, const Plan &plan, Counts *kc, 
           TransposeArgs t = transpose_args(oh.bmG, nullptr, oh.bmGT, L.dk, L.side,
                                            &R[op.outer].newt, e->d_pull_count, &e->recs[7],
                                            e->d_ctl);
+          if (plan.repeats[oi]) {
+            t.diff = oh.bmDT;
+            t.diff_n = &R[op.outer].scan.total_a;  // (and total_b)
+          }
           PLAUNCH(kc, kPBitmap, k_bm_transpose<<<grid_for(e, (u64)L.side * L.side, 1, 8), kTrBlock,
                                                  0, s>>>(t));
           OT = oh.bmGT;
@@ -2177,6 +2215,33 @@ void enqueue_iteration(gdl_engine *e, LieHost &L, const Plan &plan, Counts *kc, 
           // the inner is a FULL kept as a bitmap: a boolean product
           const RelDev &out = e->h[op.out];
           ProdArgs pa = product_args(e, L, plan, oi, a);
+          if (plan.repeats[oi]) {
+            pa.part = 1;
+            pa.OT_fresh = oh.bmDT;
+            pa.n_fresh = &R[op.outer].scan.total_b;
+            pa.newt = &R[op.outer].newt;
+            pa.delta = &R[op.inner].delta;
+            launch_product(e, pa, kc);
+            PLAUNCH(kc, kPJoinMat, k_prod_repeats<<<(int)e->sms, 256, 0, s>>>(
+                                       pa, &R[op.out].newt_phantom));
+            // the whole NEWT with the inner's DELTA, the other way round
+            ProdArgs pb;
+            memcpy(&pb, &pa, sizeof pa);
+            pb.part = 2;
+            pb.OT = e->h[op.inner].bmDT;
+            pb.F = oh.bmG;
+            pb.G = plan.pull_t[oi] ? out.bmG : out.bmOT;
+            pb.dirty = plan.pull_t[oi] ? out.dirty : nullptr;
+            pb.j.outer = &R[op.inner].delta;
+            pb.j.inner = &R[op.outer].newt;
+            pb.j.outer_vis = nullptr;
+            pb.j.inner_vis = nullptr;
+            pb.j.outer_bm = nullptr;
+            launch_product(e, pb, kc);
+            launch_fold(e, out.bmOT, out.bmG, out.dirty, L.dk, L.side,
+                        plan.fold_over[oi] && !out.dirty, kc, s);
+            continue;
+          }
           launch_product(e, pa, kc);
           if (plan.pull_t[oi] && !plan.fold_late[op.out])
             launch_fold(e, out.bmOT, out.bmG, out.dirty, L.dk, L.side,
@@ -2799,8 +2864,10 @@ gdl_status validate_rel(gdl_engine *e, int r) {
 gdl_status presize_lists(gdl_engine *e, LieHost &L, const Plan &plan, u64 cap) {
   for (int r : L.update) {
     RelDev &h = e->h[r];
-    TRY(ensure_arr(e, h.delta, cap, true));
-    TRY(ensure_arr(e, h.delta_next, cap, false));
+    if (!plan.fused[r]) {  // (a fused update step keeps DELTA as bitmaps)
+      TRY(ensure_arr(e, h.delta, cap, true));
+      TRY(ensure_arr(e, h.delta_next, cap, false));
+    }
     if (plan.newt_list[r] || plan.acopy_src[r]) TRY(ensure_arr(e, h.newt, cap, false));
     if (plan.full_list[r]) {
       TRY(ensure_arr(e, h.full, cap, true));
@@ -2819,7 +2886,8 @@ gdl_status presize_lists(gdl_engine *e, LieHost &L, const Plan &plan, u64 cap) {
       TRY(ensure_index(e, h.delta_idx_next, h.delta_next.cap));
     }
   }
-  for (int r : L.tmps) TRY(ensure_arr(e, e->h[r].newt, cap, false));
+  for (int r : L.tmps)
+    if (plan.newt_list[r] || plan.acopy_src[r]) TRY(ensure_arr(e, e->h[r].newt, cap, false));
   return GDL_OK;
 }
 
@@ -2954,7 +3022,7 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
       e->h[r].dense = 1;
     }
     for (auto *v : {&L.update, &L.tmps})
-      for (int r : *v) TRY(ensure_tbitmaps(e, plan, r, words));
+      for (int r : *v) TRY(ensure_tbitmaps(e, L, plan, r, words));
     // (before the relation table is uploaded: a later read-back of the table
     // replaces the host mirror)
     for (size_t oi = 0; oi < L.ops.size(); oi++) {
@@ -2981,9 +3049,9 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
     // does not fit, retry within a quarter of the memory actually free.
     u64 lists = 0;
     for (int r : L.update)
-      lists += 2 + ((plan.newt_list[r] || plan.acopy_src[r]) ? 1 : 0) +
+      lists += (plan.fused[r] ? 0 : 2) + ((plan.newt_list[r] || plan.acopy_src[r]) ? 1 : 0) +
                (plan.full_list[r] ? 2 : (e->instances ? 0 : 1));
-    lists += L.tmps.size();
+    for (int r : L.tmps) lists += plan.newt_list[r] || plan.acopy_src[r];
     const u64 domain = words * 32;
     const u64 cap = std::min<u64>(
         {domain, e->total_mem / 4 / std::max<u64>(lists, 1) / 8, kMaxRows});
@@ -3390,6 +3458,9 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
             // (and the transposed twins, zero between their uses)
             if (e->h[r].bmOT) CK(e, cudaMemsetAsync(e->h[r].bmOT, 0, words * 4, e->s));
           }
+        // (a repeated NEWT is compared with a committed iteration's)
+        for (int r : L.tmps)
+          if (plan.newt_t[r]) CK(e, cudaMemsetAsync(e->h[r].bmGT, 0, words * 4, e->s));
       }
       if (resume) {
         tail_listed = false;

@@ -38,6 +38,15 @@
 // k_join_product (points-to relations are reflexive, so half the rows hold a
 // few keys and the others thousands; 20,000 variables: 260 -> 195 ms).
 //
+// A tmp NEWT outer (points-to's two-step rule) is derived anew in every
+// iteration, mostly the tuples of the iteration before: joined with all of
+// FULL then, and their results are in the output's FULL now.  So with few
+// fresh tuples only those are joined with FULL, and the whole NEWT with the
+// inner's DELTA (as the product the other way round: its few rows against
+// NEWT's), semi-naive within the rule.  The transpose that makes OT keeps the
+// last one's to compare with; the device decides by the counts.  Late
+// iterations at 20,000 variables: 6.5 -> 0.5 to 1.2 ms a product.
+//
 // product_small: below 2^kProdTableBits ids there are too few rows to fill
 // the GPU with tables.  A warp takes one output row and a share of its keys
 // and ORs the inner's rows straight from L1 / L2, four keys' loads in flight
@@ -82,6 +91,13 @@ struct ProdArgs {
   u32 *list;       // [0]: long rows of OT, then (from [1]) those rows
   int dk;          // rows of 2^(dk-5) words
   u32 side;        // 256-id groups that hold ids
+  // Repeated outer: the fresh part of OT and its size; part 1 takes it in
+  // place of OT when it is small, part 2 (OT the inner's DELTA, F NEWT's rows)
+  // runs in that case only.  0: neither.
+  int part;
+  const u32 *OT_fresh;
+  const u64 *n_fresh;
+  const DArr *newt, *delta;  // the outer, and the inner's DELTA
   u32 splits;      // product_small: warps a row's keys are shared among
 };
 
@@ -96,6 +112,20 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src, u32 bytes
 // block calls this; a NEWT outer's bitmap is cleared too).  Returns whether
 // there is nothing to join.  The inner is looked at first: no block reads
 // the outer's count while block 0 may be zeroing it.
+// The two parts against the whole: by their tuples, with room for what they
+// cost beyond that (at 20,000 variables: 8.2 ms for 6.6 where a tenth of NEWT
+// was fresh or DELTA, 1.2 for 6.6 at a fiftieth).
+__device__ __forceinline__ bool prod_few_fresh(const ProdArgs &a) {
+  return a.part && (*a.n_fresh + a.delta->n) * 16 <= a.newt->n;
+}
+// The outer a launch reads, null when there is nothing for it to do.
+__device__ __forceinline__ const u32 *prod_outer(const ProdArgs &a) {
+  if (a.part == 0) return a.OT;
+  const bool few = prod_few_fresh(a);
+  if (a.part == 1) return few ? a.OT_fresh : a.OT;
+  return few && a.j.outer->n && a.j.inner->n ? a.OT : nullptr;
+}
+
 __device__ __forceinline__ bool product_empty(const JoinArgs &j, u64 *n_outer) {
   if (eff_count(j.inner, j.inner_vis) == 0) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -124,6 +154,8 @@ __global__ void __launch_bounds__(256) k_prod_rows(ProdArgs a) {
   if (ctl_stop(a.j.ctl)) return;
   const u64 n_outer = eff_count(a.j.outer, a.j.outer_vis);
   if (n_outer == 0 || eff_count(a.j.inner, a.j.inner_vis) == 0) return;
+  const u32 *OT = prod_outer(a);
+  if (!OT) return;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const u32 n4 = a.side * 2;
   for (u32 g = blockIdx.x; g < a.side * 8; g += gridDim.x) {
@@ -131,7 +163,7 @@ __global__ void __launch_bounds__(256) k_prod_rows(ProdArgs a) {
 #pragma unroll
     for (int q = 0; q < 4; q++) {
       const uint4 *p =
-          reinterpret_cast<const uint4 *>(a.OT + ((u64)(g * 32 + wid * 4 + q) << (a.dk - 5)));
+          reinterpret_cast<const uint4 *>(OT + ((u64)(g * 32 + wid * 4 + q) << (a.dk - 5)));
       u32 keys = 0;
       for (u32 i = lane; i < n4; i += 32) {
         const uint4 v = p[i];
@@ -167,7 +199,9 @@ __global__ void __launch_bounds__(kProdBlock, 1) k_join_product(ProdArgs a) {
   __shared__ long long s_unit;
   if (ctl_stop(a.j.ctl)) return;
   u64 n_outer;
-  if (product_empty(a.j, &n_outer)) return;
+  if (a.part != 2 && product_empty(a.j, &n_outer)) return;
+  const u32 *OT = prod_outer(a);
+  if (!OT) return;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int rs = a.dk - 5;
   const u32 row_words = 1u << rs;
@@ -197,7 +231,7 @@ __global__ void __launch_bounds__(kProdBlock, 1) k_join_product(ProdArgs a) {
     u32 av[8];
     auto load_a = [&](u32 s) {
       if (my_row != kNoRow) {
-        load8(a.OT + ((u64)my_row << rs) + s * 8, av);
+        load8(OT + ((u64)my_row << rs) + s * 8, av);
       } else {
 #pragma unroll
         for (int w = 0; w < 8; w++) av[w] = 0;
@@ -360,6 +394,36 @@ __global__ void __launch_bounds__(kProdBlock, 1) k_join_product(ProdArgs a) {
   }
 }
 
+// A product that leaves the repeated tuples out still counts as having found
+// theirs (NEWT is not empty, src/lie.cu:114-121): *phantom is set when some
+// key of OT has an inner row with bits.  Warps stop at the first such key, as
+// a rule at once.
+__global__ void __launch_bounds__(256) k_prod_repeats(ProdArgs a, u32 *phantom) {
+  if (ctl_stop(a.j.ctl) || !prod_few_fresh(a)) return;
+  if (a.newt->n == 0 || eff_count(a.j.inner, a.j.inner_vis) == 0) return;
+  const int lane = threadIdx.x & 31;
+  const u32 words = a.side * 8, rows = a.side * 256;
+  for (u32 r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows;
+       r += (gridDim.x * blockDim.x) >> 5) {
+    for (u32 w0 = 0; w0 < words; w0 += 32) {
+      if (*((volatile u32 *)phantom)) return;
+      const u32 mine = w0 + lane < words ? a.OT[((u64)r << (a.dk - 5)) + w0 + lane] : 0u;
+      for (u32 some = __ballot_sync(0xffffffffu, mine != 0u); some; some &= some - 1) {
+        const int j = __ffs(some) - 1;
+        for (u32 x = __shfl_sync(0xffffffffu, mine, j); x; x &= x - 1) {
+          const u32 *row = a.F + ((u64)((w0 + j) * 32 + __ffs(x) - 1) << (a.dk - 5));
+          u32 any = 0;
+          for (u32 i = lane; i < words; i += 32) any |= row[i];
+          if (__any_sync(0xffffffffu, any != 0u)) {
+            if (lane == 0) *phantom = 1;
+            return;
+          }
+        }
+      }
+    }
+  }
+}
+
 // One warp: output row `row`, the keys of its words [w0, w1) (at most 32
 // words).  RS: rows of 2^RS words, 8 to 64.  With rows shorter than a warp,
 // 32 >> RS keys are read at once, one per group of 2^RS lanes.
@@ -465,6 +529,8 @@ __global__ void __launch_bounds__(kProdRowsBlock, V <= 8 ? 2 : 1) k_join_product
   const u64 n_outer = eff_count(a.j.outer, a.j.outer_vis);
   // (the launch before this one applied the empty-side rule)
   if (n_outer == 0 || eff_count(a.j.inner, a.j.inner_vis) == 0) return;
+  const u32 *OT = prod_outer(a);
+  if (!OT) return;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   constexpr int kRows = kProdRowsBlock / 32;
   const int rs = a.dk - 5;
@@ -480,7 +546,7 @@ __global__ void __launch_bounds__(kProdRowsBlock, V <= 8 ? 2 : 1) k_join_product
     u32 w[V * 4];
     u32 left = 0;
     {
-      const uint4 *p = reinterpret_cast<const uint4 *>(a.OT + ((u64)row_no(wid) << rs));
+      const uint4 *p = reinterpret_cast<const uint4 *>(OT + ((u64)row_no(wid) << rs));
 #pragma unroll
       for (int j = 0; j < V; j++) {
         const uint4 x = j * 32 + lane < n4 ? p[j * 32 + lane] : make_uint4(0, 0, 0, 0);

@@ -103,6 +103,10 @@ struct TransposeArgs {
   u32 side;       // 256 x 256-bit tiles per side that hold ids
   DArr *count_to; // if set: receives the number of bits as its n
   u64 *count_acc; // zero between launches
+  // if set: the bits that dst did not hold before (it keeps what the last
+  // launch wrote), their number added to diff_n[0] and published in diff_n[1]
+  u32 *diff;
+  u64 *diff_n;
   LaunchRec *lrec;
   Ctl *ctl;
 };
@@ -116,6 +120,7 @@ __global__ void __launch_bounds__(kTrBlock) k_bm_transpose(TransposeArgs a) {
   const u64 tiles = per * per;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   u64 bits = 0, moved = 0;
+  u32 fresh = 0;
   for (u64 t = blockIdx.x; t < tiles; t += gridDim.x) {
     u32 tr, tc;
     tile_rc((u32)t, (u32)per, tr, tc);
@@ -139,7 +144,10 @@ __global__ void __launch_bounds__(kTrBlock) k_bm_transpose(TransposeArgs a) {
     // (a tile's reads of s_t are ordered before the next tile's writes by
     // the next tile's __syncthreads_or)
     const bool tile_any = __syncthreads_or(any);
-    uint4 *d = reinterpret_cast<uint4 *>(a.dst + (((u64)tc * 256 + threadIdx.x) << rs) + tr * 8);
+    const u64 dw = (((u64)tc * 256 + threadIdx.x) << rs) + tr * 8;
+    uint4 *d = reinterpret_cast<uint4 *>(a.dst + dw);
+    u32 old[8];
+    if (a.diff) load8(a.dst + dw, old);
     if (tile_any) {
 #pragma unroll
       for (int i = 0; i < 8; i++) {
@@ -151,11 +159,30 @@ __global__ void __launch_bounds__(kTrBlock) k_bm_transpose(TransposeArgs a) {
       const u32 *q = s_t[threadIdx.x];
       d[0] = make_uint4(q[0], q[1], q[2], q[3]);
       d[1] = make_uint4(q[4], q[5], q[6], q[7]);
+      if (a.diff) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          old[i] = q[i] & ~old[i];
+          fresh += __popc(old[i]);
+        }
+      }
     } else {
       d[0] = make_uint4(0, 0, 0, 0);
       d[1] = make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int i = 0; i < 8; i++) old[i] = 0;
     }
     moved += 32;
+    if (a.diff) {
+      uint4 *o = reinterpret_cast<uint4 *>(a.diff + dw);
+      o[0] = make_uint4(old[0], old[1], old[2], old[3]);
+      o[1] = make_uint4(old[4], old[5], old[6], old[7]);
+      moved += 64;
+    }
+  }
+  if (a.diff) {
+    fresh = __reduce_add_sync(0xffffffffu, fresh);
+    if (lane == 0 && fresh) atomicAdd((unsigned long long *)&a.diff_n[0], (unsigned long long)fresh);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -172,6 +199,10 @@ __global__ void __launch_bounds__(kTrBlock) k_bm_transpose(TransposeArgs a) {
   if (launch_rec_finish(a.lrec) && threadIdx.x == 0) {
     a.count_to->n = *a.count_acc;
     *a.count_acc = 0;
+    if (a.diff) {
+      a.diff_n[1] = a.diff_n[0];
+      a.diff_n[0] = 0;
+    }
   }
 }
 
