@@ -18,7 +18,9 @@
 //                                in the graph, open the next iteration)
 //
 // (In the dense form the per-relation dedup is a bitmap scan instead, and
-// joins set bits: dense.cuh.)
+// joins set bits: dense.cuh, or are row unions and boolean products: pull.cuh,
+// product.cuh.  Small domains, linear recursion and hash sets run the whole
+// loop in one resident launch: loop.cuh, closure.cuh, hash.cuh.)
 //
 // That sequence is captured once into a CUDA graph as the body of a
 // conditional while-node; k_commit sets the node's condition, so a whole
@@ -137,7 +139,7 @@ struct LieHost {
   // iteration; its steps and update list in device memory.
   bool resident = false;
   // Linear recursion in one pass an iteration (closure.cuh): the loop's
-  // arguments; its per-row arrays (c_rows of them, c_edges adj entries).
+  // arguments; one allocation for its per-row arrays and edges.
   bool closure = false;
   ClosureArgs cargs{};
   u32 *c_mem = nullptr;
@@ -298,7 +300,7 @@ struct gdl_engine {
   int row_gather = 2;
   u32 spin_limit = kSpinLimit;  // polls of a bounded device wait
   u32 test_wait = 0;            // gdl_engine_test_timeout (next fixpoint only)
-  u32 *prod_list = nullptr;     // rows of a product's outer (product.cuh)
+  u32 *prod_list = nullptr;     // rows of a product's outer (product.cuh), behind d_u32
   u64 *d_pull_count = nullptr;  // bit count of a transposed NEWT (zero between launches)
   // Device memory in bytes, read once at creation: cudaMemGetInfo can take
   // tens of milliseconds on a busy host, so the fixpoint sizes its lists
@@ -320,7 +322,7 @@ struct gdl_engine {
   void *d_count = nullptr;    // gdl_join_count's scratch (CountScratch)
   void *d_part = nullptr;     // gdl_partition_rows: counts and cursors per destination
   u64 *d_u64 = nullptr;       // [4] small device scalars
-  u64 *h_scalars = nullptr;   // [4] pinned, for their read-back
+  u64 *h_scalars = nullptr;   // [4] for their read-back, behind h_rels_pin
   u32 *d_u32 = nullptr;       // [4]: [3] device checks of async loads (sticky)
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // Graph capture runs on its own stream, so that the engine stream can run
@@ -1646,7 +1648,7 @@ ProdArgs product_args(gdl_engine *e, LieHost &L, const Plan &plan, size_t oi, co
 // DELTAs, tmp NEWTs or static FULLs, so that no operator reads an update
 // relation's FULL, or a sorted DELTA, during the loop.
 bool hash_form(const gdl_engine *e, const LieHost &L, const Plan &plan) {
-  if (L.dense || e->instances || e->dedup_mode != 0 || L.update.empty() || L.ops.empty())
+  if (L.dense || e->instances || e->dedup_mode == 1 || L.update.empty() || L.ops.empty())
     return false;
   std::vector<char> is_update(e->rels.size(), 0), is_static(e->rels.size(), 0);
   for (int r : L.update) is_update[r] = 1;
@@ -1668,9 +1670,9 @@ bool hash_form(const gdl_engine *e, const LieHost &L, const Plan &plan) {
   return true;
 }
 
-// The hash set of update relation r, sized for its FULL list's capacity, and
-// filled with its committed rows (`push` must follow when this returns with
-// the set moved, before the fill: `fill` is enqueued by fill_hash).
+// The hash set of update relation r, sized for its FULL list's capacity.  Its
+// address is in RelDev, so the table is pushed before fill_hash puts the
+// committed rows into it.
 gdl_status ensure_hash(gdl_engine *e, int r) {
   RelDev &h = e->h[r];
   const u64 slots = next_pow2((h.full.cap + 2) / 3 * 4);
@@ -3789,14 +3791,11 @@ gdl_status gdl_engine_create(int32_t device, void *stream, gdl_engine **out) {
       bad(cudaMalloc(&e->d_rels, kMaxRels * sizeof(RelDev))) ||
       bad(cudaMalloc(&e->d_ctl, sizeof(Ctl))) || bad(cudaMallocHost(&e->h_ctl, sizeof(Ctl))) ||
       bad(cudaMallocHost(&e->h_ctl2, sizeof(Ctl))) ||
-      bad(cudaMallocHost(&e->h_scalars, 4 * sizeof(u64))) ||
       bad(cudaMallocHost(&e->h_trace, kTraceRows * kMaxRels * 3 * sizeof(u64))) ||
-      bad(cudaMallocHost(&e->h_rels_pin, kMaxRels * sizeof(RelDev))) ||
+      bad(cudaMallocHost(&e->h_rels_pin, kMaxRels * sizeof(RelDev) + 4 * sizeof(u64))) ||
       bad(cudaMalloc(&e->recs, 16 * sizeof(LaunchRec))) ||
       bad(cudaMalloc(&e->d_tmp, 4 * sizeof(DArr))) || bad(cudaMalloc(&e->d_u64, 4 * sizeof(u64))) ||
-      bad(cudaMalloc(&e->d_u32, 4 * sizeof(u32))) ||
-      bad(cudaMalloc(&e->prod_list, ((1u << 16) + 1) * sizeof(u32))) ||
-      bad(cudaMemsetAsync(e->prod_list, 0, sizeof(u32), e->s)) ||
+      bad(cudaMalloc(&e->d_u32, (4 + (1u << 16) + 1) * sizeof(u32))) ||
       bad(cudaMalloc(&e->d_pull_count, sizeof(u64))) || bad(cudaEventCreate(&e->ev0)) ||
       bad(cudaEventCreate(&e->ev1)) ||
       bad(cudaEventCreateWithFlags(&e->ev_first, cudaEventDisableTiming)) ||
@@ -3806,12 +3805,14 @@ gdl_status gdl_engine_create(int32_t device, void *stream, gdl_engine **out) {
       bad(cudaMemcpyAsync(&e->d_ctl->spin_limit, &e->spin_limit, sizeof(u32),
                           cudaMemcpyHostToDevice, e->s)) ||
       bad(cudaMemsetAsync(e->recs, 0, 16 * sizeof(LaunchRec), e->s)) ||
-      bad(cudaMemsetAsync(e->d_u32, 0, 4 * sizeof(u32), e->s)) ||
+      bad(cudaMemsetAsync(e->d_u32, 0, 5 * sizeof(u32), e->s)) ||
       bad(cudaMemsetAsync(e->d_pull_count, 0, sizeof(u64), e->s)) ||
       bad(cudaStreamSynchronize(e->s))) {
     gdl_engine_destroy(e);
     return GDL_E_CUDA;
   }
+  e->h_scalars = reinterpret_cast<u64 *>(e->h_rels_pin + kMaxRels);
+  e->prod_list = e->d_u32 + 4;
   // TMA passes: the driver's tensor-map encoder, and their shared memory
   if (!getenv("GDLOG_NO_TMA")) {
     cudaDriverEntryPointQueryResult q;
@@ -3951,7 +3952,7 @@ gdl_status gdl_engine_destroy(gdl_engine *e) {
                   (void *)e->d_segs,
                   (void *)e->d_tile_inst, (void *)e->d_square_seg,
                   (void *)e->recs,
-                  (void *)e->d_tmp, (void *)e->d_u64, (void *)e->d_u32, (void *)e->d_pull_count, (void *)e->prod_list,
+                  (void *)e->d_tmp, (void *)e->d_u64, (void *)e->d_u32, (void *)e->d_pull_count,
                   e->d_count, e->d_part,
                   (void *)e->d_rels,
                   (void *)e->d_ctl})
@@ -3960,7 +3961,6 @@ gdl_status gdl_engine_destroy(gdl_engine *e) {
   if (e->h_ctl2) cudaFreeHost(e->h_ctl2);
   if (e->h_trace) cudaFreeHost(e->h_trace);
   if (e->h_rels_pin) cudaFreeHost(e->h_rels_pin);
-  if (e->h_scalars) cudaFreeHost(e->h_scalars);
   if (e->pin_keys) cudaFreeHost(e->pin_keys);
   if (e->ev0) cudaEventDestroy(e->ev0);
   if (e->ev1) cudaEventDestroy(e->ev1);

@@ -116,7 +116,10 @@ gdl_status gdl_engine_test_timeout(gdl_engine *e, int32_t polls);
  * DENSE: when 2 * bits(largest column value) <= dense_max_bits (at most 32,
  * the default), relations are kept as bitmaps over the key domain during the
  * loop and NEWT is deduplicated by setting bits.  AUTO (default): DENSE
- * where the domain allows, else SORT.  Results are identical in all modes.
+ * where the domain allows, else SORT.  Where a LIE's domain is too wide for
+ * bitmaps and no operator reads an update relation's FULL during the loop,
+ * AUTO and DENSE keep a hash set of each FULL and sort it once at the end.
+ * Results are identical in all modes.
  * dense_max_bits == 0 keeps the current bound.  The environment variables
  * GDLOG_DEDUP=auto|sort|dense and GDLOG_DENSE_MAX_BITS set the defaults.
  * No reference counterpart. */
@@ -146,15 +149,16 @@ typedef struct gdl_tuning {
   int32_t pull_joins;          /* joins into bitmaps whose output is (outer
                                   column 1, inner column 1) over a DELTA or
                                   tmp NEWT outer: 1 = push form (outer in key
-                                  order), 2 = pull form (gathered by output
-                                  row from the transposed outer) when ids
-                                  reach 2^10 (default), 3 = pull form from
-                                  2^8 ids */
+                                  order), 2 = boolean products where the inner
+                                  FULL is a bitmap, else the pull form
+                                  (gathered by output row from the transposed
+                                  outer) when ids reach 2^10 (default), 3 =
+                                  pull form from 2^8 ids */
   int32_t row_gather;          /* those joins over a static inner when ids reach
                                   2^12: 1 = off, 2 = gather the outer's bitmap
                                   rows along the inner's in-edges when the
                                   inner is small enough (|inner| x row bytes
-                                  <= 256 MB; default), 3 = whenever possible */
+                                  <= 4 GB; default), 3 = whenever possible */
   int32_t spin_limit_log2;     /* a bounded device-side wait (look-back of a scan)
                                   gives up after 2^this polls and the call
                                   returns GDL_E_TIMEOUT (default 22; 1..30) */

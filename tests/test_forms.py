@@ -143,6 +143,7 @@ def test_hash_sets_equal_sorted_lists(name):
     prog, args = WIDE[name]
     want = outcome(prog, args, "sort")
     assert outcome(prog, args) == want
+    assert outcome(prog, args, "dense") == want  # (too wide for bitmaps: sets as well)
     assert outcome(prog, args, no_graph=True) == want
 
 
