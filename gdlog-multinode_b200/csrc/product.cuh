@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(kProdBlock, 1) k_join_product(ProdArgs a) {
   const u32 n_kc = (a.side + ksteps - 1) / ksteps;
   const u32 units = n_rb * n_sl * n_kc;
   const u32 lane4 = lane * 4;
-  u64 used = 0, flushed = 0;
+  u64 flushed = 0;
   while (true) {
     if (tid < 16) s_cnt[tid >> 3][tid & 7] = 0;
     const long long g = grab_tile(a.j.rec, &s_unit);
@@ -294,7 +294,6 @@ __global__ void __launch_bounds__(kProdBlock, 1) k_join_product(ProdArgs a) {
             const u32 cnt = s_cnt[st][w];
             const u32 bm = s_rows[w];
             if (cnt == 0 || bm == 0) continue;  // (block-uniform)
-            if (tid == 0) used += cnt;
             const u32 *Bw = B + w * 32 * 32 + lane;
             if (cnt > MR) {
               {
@@ -384,10 +383,9 @@ __global__ void __launch_bounds__(kProdBlock, 1) k_join_product(ProdArgs a) {
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) flushed += __shfl_xor_sync(0xffffffffu, flushed, o);
-  // algorithmic bytes: 4 per word of OT, a slice of an inner row per key
-  // used, 4 per word reduced into the output
+  // algorithmic bytes of both kernels together: OT and the inner once, 4 per
+  // word reduced into the output
   if (lane == 0) prof_add(a.j.ctl, kPJoinMat, 4 * flushed);
-  if (tid == 0) prof_add(a.j.ctl, kPJoinMat, used * 128);
   if (launch_rec_finish(a.j.rec) && tid == 0) {
     a.list[0] = 0;
     prof_add(a.j.ctl, kPJoinMat, (u64)ids * a.side * 32);
@@ -536,7 +534,7 @@ __global__ void __launch_bounds__(kProdRowsBlock, V <= 8 ? 2 : 1) k_join_product
   const int rs = a.dk - 5;
   const u32 n4 = a.side * 2;  // 16-byte words of a row that hold ids
   const u32 tiles = a.side * 256 / kRows;
-  u64 words_out = 0, keys = 0;
+  u64 words_out = 0;
   while (true) {
     const long long t = grab_tile(a.rows_rec, &s_tile);
     if (t >= (long long)tiles) break;
@@ -579,7 +577,6 @@ __global__ void __launch_bounds__(kProdRowsBlock, V <= 8 ? 2 : 1) k_join_product
       }
       __syncthreads();
       const u32 n = (u32)total;
-      keys += n;
       // an equal share of the list a warp, two rows in flight
       u32 i = (u32)((u64)n * wid / kRows);
       const u32 iend = (u32)((u64)n * (wid + 1) / kRows);
@@ -639,7 +636,6 @@ __global__ void __launch_bounds__(kProdRowsBlock, V <= 8 ? 2 : 1) k_join_product
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) words_out += __shfl_xor_sync(0xffffffffu, words_out, o);
   if (lane == 0) prof_add(a.j.ctl, kPJoinMat, 4 * words_out);
-  if (tid == 0) prof_add(a.j.ctl, kPJoinMat, keys * n4 * 16);
   if (launch_rec_finish(a.rows_rec) && tid == 0)
     prof_add(a.j.ctl, kPJoinMat, (u64)a.side * 256 * a.side * 32);
 }
