@@ -416,7 +416,9 @@ gdl_status dalloc(gdl_engine *e, void **p, size_t bytes) {
   auto rp = e->replay.find(bytes);
   if (rp != e->replay.end() && j < rp->second.size()) {
     auto at = e->spare_at.find(rp->second[j]);
-    if (at != e->spare_at.end()) *p = take_spare(e, at->second);
+    // (a block that went back to the pool may have come again at the same
+    // address with another size)
+    if (at != e->spare_at.end() && at->second->first >= bytes) *p = take_spare(e, at->second);
   }
   if (!*p) {
     auto it = e->spare.lower_bound(bytes);
@@ -430,6 +432,7 @@ gdl_status dalloc(gdl_engine *e, void **p, size_t bytes) {
       drop_spare(e);
       r = cudaMallocAsync(p, bytes, e->s);
     }
+    if (r != cudaSuccess) cudaGetLastError();  // (not for a later launch's check to find)
     CK(e, r);
     e->alloc_size[*p] = bytes;
   }
