@@ -124,7 +124,7 @@ struct Ctl {
   u32 spin_limit;  // polls a bounded wait makes before it gives up (timeout)
   u32 test_wait;   // nonzero: k_begin waits this many polls on `never` (tests)
   u32 never;       // a flag no kernel sets
-  u32 pad_ctl2;
+  u32 hash_long;   // a probe chain of a hash set passed its bound (hash.cuh)
   u32 bar_count, bar_word;  // grid barrier of the resident loop (loop.cuh)
   u64 iteration;     // iteration_counter of the reference loop
   u64 stop_at;       // pause when iteration reaches this

@@ -1741,6 +1741,33 @@ gdl_status sort_in_place(gdl_engine *e, const DArr *d, const DArr &a) {
   return GDL_OK;
 }
 
+// FULL and DELTA of a LIE in the hash form, as the sorted lists that the other
+// forms keep (the table is uploaded after this).
+gdl_status sort_hash_lists(gdl_engine *e, LieHost &L) {
+  for (int r : L.update) {
+    RelDev &h = e->h[r];
+    h.dense = h.full_lazy = 0;
+    TRY(sort_in_place(e, &e->d_rels[r].full, h.full));
+    TRY(sort_in_place(e, &e->d_rels[r].delta, h.delta));
+  }
+  return GDL_OK;
+}
+// The rest of the loop on sorted lists, from the last committed iteration
+// (the host mirror and the table hold it).
+gdl_status leave_hash(gdl_engine *e, LieHost &L) {
+  L.hashed = L.resident = false;
+  TRY(sort_hash_lists(e, L));
+  for (int r : L.update) {
+    RelDev &h = e->h[r];
+    TRY(ensure_arr(e, h.full_next, h.full.cap, false));
+    TRY(ensure_arr(e, h.newt, h.delta.cap, false));
+    h.newt.n = h.delta_next.n = 0;
+    h.c_newt_n = 0;
+  }
+  TRY(ensure_scratch(e));
+  return push(e);
+}
+
 HashJoinArgs hash_args(gdl_engine *e, const JoinArgs &a, int out, bool hashed) {
   HashJoinArgs h;
   memset(&h, 0, sizeof h);
@@ -3437,12 +3464,20 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
       TRY(grow_after_overflow(e, c));
       L.grow_ms += host_ms_since(tg);
       const bool resume = L.dense && c.overflow_stage == 1;
+      bool grew = false;
+      for (u64 x : c.need) grew = grew || x != 0;
+      const bool to_lists = L.hashed && c.hash_long && !grew;
+      c.hash_long = 0;
       c.overflow = 0;
       c.overflow_stage = 0;
       memset(c.need, 0, sizeof c.need);
       L.retries++;
       L.graph_dirty = true;
-      if (L.hashed) {
+      if (to_lists) {
+        TRY(reset_ctl(e));
+        c.generation = e->generation;
+        TRY(leave_hash(e, L));
+      } else if (L.hashed) {
         // the sets again from the committed rows
         for (int r : L.update) TRY(ensure_hash(e, r));
         TRY(push(e));
@@ -3653,12 +3688,7 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
     const u64 kept_iteration = c.iteration;
     TRY(pull(e));
     TRY(reset_ctl(e));
-    for (int r : L.update) {
-      RelDev &h = e->h[r];
-      h.dense = h.full_lazy = 0;
-      TRY(sort_in_place(e, &e->d_rels[r].full, h.full));
-      TRY(sort_in_place(e, &e->d_rels[r].delta, h.delta));
-    }
+    TRY(sort_hash_lists(e, L));
     TRY(push(e));
     CK(e, cudaMemcpyAsync(e->h_ctl, e->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, e->s));
     listed = true;

@@ -8,7 +8,7 @@
 // FULL as a list during the loop (every inner is a static relation, DELTA and
 // a tmp NEWT are only outers), order is needed once, at the end.  Then:
 //   * FULL is an unsorted list plus a set of its keys: open addressing, 8-byte
-//     slots, at most three quarters full, ~0 empty;
+//     slots, at most three quarters full when an iteration commits, ~0 empty;
 //   * a join probes, expands and inserts in one pass (k_join_hash): a
 //     candidate that takes an empty slot is new and is appended to FULL and to
 //     the next DELTA, any other is dropped, most of them by a plain load;
@@ -27,6 +27,14 @@
 // otherwise unused here) and k_hash_aside decides it after the joins, when
 // each slot's ordinal in FULL (`hord`) says whether its tuple was there when
 // the iteration began.
+//
+// A key takes its slot before the list's counter counts it, so an iteration
+// may pass the three quarters before the overflow is seen: up to 224 keys a
+// warp wait uncounted, and a warp looks at the overflow flag once a step.  A
+// set may even fill up.  Probe chains are therefore bounded (kHashMaxProbe):
+// past the bound the iteration ends uncommitted and runs again, from a larger
+// set where the rows counted ask for one, else (the chain is the tuples of one
+// prefix, which no larger set shortens) on sorted lists.
 #pragma once
 
 #include "common.cuh"
@@ -51,8 +59,19 @@ struct HashJoinArgs {
   int need_full, need_delta, need_newt;  // need slots of out
 };
 
+// Slots a probe looks at.  The longest chain of random keys in a set three
+// quarters full is about ln(slots) / 0.038 slots (Knuth vol. 3, 6.4): 420 of
+// 2^23, 570 of 2^31.
+constexpr u32 kHashMaxProbe = 2048;
+
+// The iteration cannot be committed with this set.
+__device__ __forceinline__ void hash_chain_long(Ctl *ctl) {
+  ctl->hash_long = 1;
+  atomicExch(&ctl->overflow, 1u);
+}
+
 // One candidate: 0 known, 1 new (its slot in *slot), 2 its prefix is present
-// with another dependent part.
+// with another dependent part, 3 its probe chain is too long.
 __device__ __forceinline__ int hash_insert(u64 *set, u64 mask, u64 prefix, u64 k, u64 *slot) {
   if (k == kHashEmpty) {
     // the one key that looks like an empty slot has a slot of its own
@@ -60,7 +79,7 @@ __device__ __forceinline__ int hash_insert(u64 *set, u64 mask, u64 prefix, u64 k
     return atomicCAS((unsigned long long *)&set[mask + 1], kHashEmpty, 0ull) == kHashEmpty;
   }
   u64 h = mix64(k & prefix) & mask;
-  for (u64 step = 0; step <= mask; step++) {
+  for (u32 step = 0; step < kHashMaxProbe; step++) {
     u64 s = *((volatile u64 *)&set[h]);
     if (s == kHashEmpty) {
       s = atomicCAS((unsigned long long *)&set[h], kHashEmpty, k);
@@ -73,7 +92,7 @@ __device__ __forceinline__ int hash_insert(u64 *set, u64 mask, u64 prefix, u64 k
     if (((s ^ k) & prefix) == 0) return 2;
     h = (h + 1) & mask;
   }
-  return 0;  // (a set always has an empty slot)
+  return 3;
 }
 
 // A warp's new keys wait in shared memory until kOutCap - 32 are there, so
@@ -154,6 +173,7 @@ __device__ __forceinline__ void hash_emit(const HashJoinArgs &a, WarpOut &w, u32
   u64 slot = 0;
   const int st = valid ? hash_insert(a.out->hset, a.out->hmask, a.prefix, k, &slot) : 0;
   hash_put(a, true, w, n, st == 1, k, slot);
+  if (st == 3) hash_chain_long(a.j.ctl);
   if (st == 2) {
     RelDev *r = a.out;
     const u64 pos = atomicAdd((unsigned long long *)&r->newt.n, 1ull);
@@ -200,7 +220,8 @@ __device__ __forceinline__ void hash_join(const HashJoinArgs &a, HashSmem &hs) {
   bool emitted = false;
   u32 waiting = 0;
   for (u64 c = (u64)blockIdx.x * 8 + wid; c < chunks; c += nw) {
-    if (*((volatile u32 *)&j.ctl->overflow)) break;
+    u32 over = *((volatile u32 *)&j.ctl->overflow);
+    if (__any_sync(0xffffffffu, over != 0)) break;
     const u64 i = c * 32 + lane;
     u64 row = 0;
     u32 s = 0, l = 0;
@@ -232,6 +253,9 @@ __device__ __forceinline__ void hash_join(const HashJoinArgs &a, HashSmem &hs) {
     sm.excl[wid][lane] = inc - l;
     __syncwarp();
     for (u64 base = 0; base < total; base += 32) {
+      // (a chunk may hold thousands of candidates; the load is under way with
+      // the step's others)
+      over = *((volatile u32 *)&j.ctl->overflow);
       const u64 p = base + lane;
       u64 t = 0;
       bool ok = false;
@@ -245,6 +269,7 @@ __device__ __forceinline__ void hash_join(const HashJoinArgs &a, HashSmem &hs) {
       }
       emitted |= ok;
       hash_emit(a, s_out[wid], waiting, t, ok);
+      if (__any_sync(0xffffffffu, over != 0)) break;
     }
     __syncwarp();
     cand += total;
@@ -271,10 +296,10 @@ __device__ __forceinline__ void hash_heavy(const HashJoinArgs &a, u64 np, WarpOu
   bool emitted = false;
   u32 waiting = 0;
   for (u64 k = blockIdx.x; k < np; k += gridDim.x) {
-    if (*((volatile u32 *)&j.ctl->overflow)) break;
     const u64 row = j.crow_key[k];
     const u32 s = j.crow_start[k], l = j.crow_len[k];
     for (u32 j0 = threadIdx.x & ~31u; j0 < l; j0 += blockDim.x) {  // (warp-uniform)
+      const u32 over = *((volatile u32 *)&j.ctl->overflow);
       const u32 q = j0 + (threadIdx.x & 31);
       u64 t = 0;
       bool ok = false;
@@ -284,6 +309,7 @@ __device__ __forceinline__ void hash_heavy(const HashJoinArgs &a, u64 np, WarpOu
       }
       emitted |= ok;
       hash_emit(a, s_out[threadIdx.x >> 5], waiting, t, ok);
+      if (__any_sync(0xffffffffu, over != 0)) break;
     }
     cand += l;
   }
@@ -316,12 +342,14 @@ __device__ __forceinline__ void hash_aside(const HashJoinArgs &a, WarpOut *s_out
   const int lane = threadIdx.x & 31;
   for (u64 i0 = ((u64)blockIdx.x * blockDim.x + threadIdx.x) & ~31ull; i0 < n;
        i0 += (u64)gridDim.x * blockDim.x) {
+    if (__any_sync(0xffffffffu, *((volatile u32 *)&a.j.ctl->overflow) != 0)) break;
     bool is_new = false;
     u64 k = 0, slot = 0;
     if (i0 + lane < n) {
       k = r->newt.ptr[i0 + lane];
       u64 h = mix64(k & a.prefix) & mask;
-      for (u64 step = 0; step <= mask; step++) {
+      u32 step = 0;
+      for (; step < kHashMaxProbe; step++) {
         u64 s = *((volatile u64 *)&r->hset[h]);
         if (s == kHashEmpty) {
           s = atomicCAS((unsigned long long *)&r->hset[h], kHashEmpty, k);
@@ -335,6 +363,7 @@ __device__ __forceinline__ void hash_aside(const HashJoinArgs &a, WarpOut *s_out
         if (((s ^ k) & a.prefix) == 0 && *((volatile u32 *)&r->hord[h]) < full_n) break;
         h = (h + 1) & mask;
       }
+      if (step == kHashMaxProbe) hash_chain_long(a.j.ctl);
     }
     hash_put(a, true, s_out[threadIdx.x >> 5], waiting, is_new, k, slot);
   }

@@ -1,0 +1,67 @@
+"""The hash form (csrc/hash.cuh) where its sets and lists run out: iterations
+that pass the first set by millions of tuples, and probe chains that no larger
+set shortens.  Contents, loop passes and traces are whole numbers and equal the
+sorted lists'."""
+import numpy as np
+import pytest
+
+import programs as P
+import workloads as W
+from gdlog_b200 import DELTA, FULL, INNER, OUTER, PLUS, Engine
+
+pytestmark = pytest.mark.gpu
+
+BASE = 1 << 20  # ids beyond the bitmaps
+
+
+def layered(layers, width, degree, seed):
+    """Every node has `degree` sources in the layer before its own; edges in
+    the order of the layers."""
+    rng = np.random.default_rng(seed)
+    dst = np.repeat(np.arange(width, layers * width), degree)
+    src = (dst // width - 1) * width + rng.integers(0, width, len(dst))
+    return np.unique(np.stack([src, dst], axis=1), axis=0).astype(np.uint64) + np.uint64(BASE)
+
+
+def outcome(prog, args, mode=None):
+    with Engine("gpu", dedup=mode) as g:
+        r = prog(g, *args)
+        return ({k: (v.size(), v.digest()) for k, v in r.relations.items()}, r.iterations,
+                {k: lie.trace().tolist() for k, lie in r.lies.items()})
+
+
+@pytest.mark.parametrize("degree,width", [(8, 125000), (30, 9000), (100, 3200)])
+@pytest.mark.parametrize("prog", ["tc", "path_length"])
+def test_first_iteration_passes_the_first_set(prog, degree, width):
+    """The first set holds 6.3 million tuples; the first iteration derives
+    more than that, nearly all of them new, from runs of `degree` tuples."""
+    edges = layered(3, width, degree, degree)
+    got = outcome(getattr(P, prog), (edges,))
+    assert max(size for size, _ in got[0].values()) - len(edges) > 6_000_000
+    assert got == outcome(getattr(P, prog), (edges,), "sort")
+
+
+def lengths_of_one_pair(eng, n):
+    """path(b, y, l + 1) :- edge(a, b), path(a, y, l) from n lengths of one
+    pair: every iteration derives n tuples of one prefix."""
+    edge = eng.relation("edge")
+    path = eng.relation("path", arity=3, dependent_column_size=1, index_flag=False)
+    first = np.stack([np.full(n, 3), np.full(n, 60), 2 * np.arange(n)], axis=1)
+    eng.load(path, first.astype(np.uint64))
+    eng.load(edge, np.array([[3, 4], [4, 5], [4, 6], [6, 7]], dtype=np.uint64))
+    lie = eng.lie()
+    lie.add_relations(edge, True)
+    lie.add_relations(path, False)
+    lie.add_join(edge, FULL, path, DELTA, path, (INNER(1), OUTER(1), PLUS(OUTER(2), 1)))
+    it = lie.fixpoint()
+    return it, path.size(), path.digest(), lie.trace().tolist()
+
+
+@pytest.mark.parametrize("n", [2047, 2049, 5000])
+def test_many_tuples_of_one_prefix_in_one_iteration(n):
+    got = []
+    for mode in (None, "sort"):
+        with Engine("gpu", dedup=mode) as g:
+            got.append(lengths_of_one_pair(g, n))
+    assert got[0] == got[1]
+    assert got[0][1] == 5 * n  # (four nodes are reached from the pair's first)
