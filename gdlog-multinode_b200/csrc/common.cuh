@@ -109,6 +109,7 @@ struct RelDev {
   u64 *hset;
   u64 hmask;
   u32 *hord;
+  u32 hlong;  // a chain passed its bound when the set was filled
 };
 
 // Loop control of a running fixpoint (one per engine, device memory).

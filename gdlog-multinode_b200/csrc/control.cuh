@@ -110,7 +110,16 @@ __global__ void k_begin(RelDev *rels, LieDev *L, Ctl *ctl) {
     }
   }
   if (!__shfl_sync(0xffffffffu, ok, 0)) return;
-  begin_iteration(rels, L, lane_lists(L, lane), lane);
+  const LaneLists x = lane_lists(L, lane);
+  u32 hlong = 0;  // (a hash set that could not be filled, hash.cuh)
+#pragma unroll
+  for (int j = 0; j < kListPerLane; j++)
+    if (lane + 32 * j < x.nu) hlong |= rels[x.upd[j]].hlong;
+  begin_iteration(rels, L, x, lane);
+  if (__any_sync(0xffffffffu, hlong != 0) && lane == 0) {
+    ctl->hash_long = 1;
+    ctl->overflow = 1;
+  }
 }
 
 template <class T>

@@ -1688,6 +1688,7 @@ gdl_status ensure_hash(gdl_engine *e, int r) {
     h.hord = nullptr;
     h.hmask = slots - 1;
   }
+  h.hlong = 0;
   if (dep && !h.hord) TRY(dalloc(e, (void **)&h.hord, (h.hmask + 2) * sizeof(u32)));
   return GDL_OK;
 }
@@ -1763,6 +1764,7 @@ gdl_status leave_hash(gdl_engine *e, LieHost &L) {
     TRY(ensure_arr(e, h.newt, h.delta.cap, false));
     h.newt.n = h.delta_next.n = 0;
     h.c_newt_n = 0;
+    h.hlong = 0;
   }
   TRY(ensure_scratch(e));
   return push(e);
@@ -2987,6 +2989,7 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
     rh.delta_sorted = rh.raw_is_full;
     h.newt.n = 0;
     h.newt_phantom = 0;
+    h.hlong = 0;
   }
   for (int r : L.tmps) {
     RelDev &h = e->h[r];
@@ -3122,8 +3125,6 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
   mark("scratch");
   TRY(push(e));
   mark("push");
-  if (L.hashed)
-    for (int r : L.update) TRY(fill_hash(e, r));
   if (L.dense) {
     // FULL's bitmap from its list; NEWT bitmaps empty.
     const u64 words = L.map.words;
@@ -3248,6 +3249,10 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
       CK(e, cudaGetLastError());
     }
   }
+  // (after the table's last upload before the loop: a fill that meets too long
+  // a chain says so in it)
+  if (L.hashed)
+    for (int r : L.update) TRY(fill_hash(e, r));
   mark("indexes");
   // Device LIE description: the header and the trace buffer (the copy-once
   // flags stay as the device has them).

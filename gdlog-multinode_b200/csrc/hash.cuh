@@ -466,7 +466,9 @@ __global__ void __launch_bounds__(256, kHashLoopCtasPerSm) k_hash_loop(HashLoopA
 }
 
 // The set of FULL's committed rows (the set is all empty when this starts;
-// rows of one prefix are entries of their own).
+// rows of one prefix are entries of their own).  Rows past the chains' bound
+// are left out: the iteration that opens next (k_begin) ends the loop, which
+// goes on on sorted lists.
 __global__ void __launch_bounds__(256) k_hash_fill(RelDev *r, u64 prefix, Ctl *ctl) {
   if (ctl_stop(ctl)) return;
   const u64 n = r->full.n, mask = r->hmask;
@@ -479,9 +481,15 @@ __global__ void __launch_bounds__(256) k_hash_fill(RelDev *r, u64 prefix, Ctl *c
       r->hset[h] = 0;
     } else {
       h = mix64(k & prefix) & mask;
-      for (u64 step = 0; step <= mask; step++) {
+      u32 step = 0;
+      for (; step < kHashMaxProbe; step++) {
         if (atomicCAS((unsigned long long *)&r->hset[h], kHashEmpty, k) == kHashEmpty) break;
+        if ((step & 255u) == 255u && *((volatile u32 *)&r->hlong)) return;
         h = (h + 1) & mask;
+      }
+      if (step == kHashMaxProbe) {
+        r->hlong = 1;
+        continue;
       }
     }
     if (r->hord) r->hord[h] = (u32)i;

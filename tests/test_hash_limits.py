@@ -65,3 +65,27 @@ def test_many_tuples_of_one_prefix_in_one_iteration(n):
             got.append(lengths_of_one_pair(g, n))
     assert got[0] == got[1]
     assert got[0][1] == 5 * n  # (four nodes are reached from the pair's first)
+
+
+@pytest.mark.parametrize("n", [2048, 2049, 200000])
+def test_many_rows_of_one_prefix_loaded(n):
+    """FULL's rows of one pair share a probe chain when the set is filled."""
+    got = []
+    for mode in (None, "sort"):
+        with Engine("gpu", dedup=mode) as g:
+            got.append(lengths_of_one_pair(g, n))
+    assert got[0] == got[1]
+    assert got[0][1] == 5 * n
+
+
+def test_form_left_in_one_program_is_taken_in_the_next():
+    """A loop that went on on sorted lists leaves nothing behind."""
+    e = W.grid_edges(20, 20)
+    with Engine("gpu") as g:
+        want = P.path_length(g, e).relations["path"].digest()
+        g.clear()
+        lengths_of_one_pair(g, 5000)
+        g.clear()
+        assert P.path_length(g, e).relations["path"].digest() == want
+        g.clear()
+        assert P.tc(g, e).output.size() == W.grid_tc_size(20, 20)
