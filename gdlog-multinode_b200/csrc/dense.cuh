@@ -1086,6 +1086,16 @@ constexpr int kFuseBlock = 256;
 constexpr int kFuseCtasPerSm = 6;
 constexpr u32 kHeavyRun = 128;
 constexpr u32 kHeavyPiece = 2048;
+// Room for the np pieces of one run in the record buffer: where they go, or ~0
+// when they do not fit.  A reservation that reaches past the buffer's end
+// leaves its entries before the end empty, since the pass over the pieces
+// takes every entry below the count.
+__device__ __forceinline__ u64 reserve_pieces(const JoinArgs &a, u32 np) {
+  const u64 pos = atomicAdd(reinterpret_cast<unsigned long long *>(&a.op->nc), (u64)np);
+  if (pos + np <= a.crow_cap) return pos;
+  for (u64 k = pos; k < a.crow_cap; k++) a.crow_len[k] = 0;
+  return ~0ull;
+}
 // Row-OR pieces: a run at least as long as its row has words (one reduction
 // per word then replaces one per candidate, and the row is 4 bytes a word
 // instead of 8 per candidate) is ORed from the inner's FULL bitmap in
@@ -1163,8 +1173,8 @@ __global__ void __launch_bounds__(BLOCK, kFuseCtasPerSm * kFuseBlock / BLOCK)
         }
       }
       const u32 np = rw ? (rw + kRowPiece - 1) / kRowPiece : (l + kHeavyPiece - 1) / kHeavyPiece;
-      const u64 pos = atomicAdd(reinterpret_cast<unsigned long long *>(&a.op->nc), (u64)np);
-      if (pos + np <= a.crow_cap) {
+      const u64 pos = reserve_pieces(a, np);
+      if (pos != ~0ull) {
         for (u32 k = 0; k < np; k++) {
           if (rw) {
             a.crow_key[pos + k] = xw + (u64)k * kRowPiece;

@@ -231,8 +231,8 @@ __device__ __forceinline__ void hash_join(const HashJoinArgs &a, HashSmem &hs) {
     }
     if (l > kHeavyRun) {
       const u32 np = (l + kHeavyPiece - 1) / kHeavyPiece;
-      const u64 pos = atomicAdd(reinterpret_cast<unsigned long long *>(&j.op->nc), (u64)np);
-      if (pos + np <= j.crow_cap) {
+      const u64 pos = reserve_pieces(j, np);
+      if (pos != ~0ull) {
         for (u32 k = 0; k < np; k++) {
           j.crow_key[pos + k] = row;
           j.crow_start[pos + k] = s + k * kHeavyPiece;

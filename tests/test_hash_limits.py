@@ -89,3 +89,25 @@ def test_form_left_in_one_program_is_taken_in_the_next():
         assert P.path_length(g, e).relations["path"].digest() == want
         g.clear()
         assert P.tc(g, e).output.size() == W.grid_tc_size(20, 20)
+
+
+def test_pieces_past_the_record_buffer():
+    """2.2 million outer rows meet a run of 6,145 tuples, four pieces each:
+    more than the record buffer holds.  The run's reservation that straddles
+    the buffer's end is expanded by its own warp, like those past it."""
+    n, run, hub = 2_200_002, 6145, 5
+    rows = np.stack([np.full(n, hub), np.arange(n) + 100000], axis=1).astype(np.uint64)
+    run_rows = np.stack([np.full(run, hub), 3_000_000 + 2 * np.arange(run)],
+                        axis=1).astype(np.uint64)
+    with Engine("gpu") as g:
+        edge = g.relation("edge")
+        out = g.relation("out", index_flag=False)
+        g.load(out, rows)
+        g.load(edge, run_rows)
+        lie = g.lie()
+        lie.add_relations(edge, True)
+        lie.add_relations(out, False)
+        lie.add_join(edge, FULL, out, DELTA, out, (INNER(1), INNER(0)))
+        assert lie.fixpoint() == 2
+        got = out.rows()
+    assert np.array_equal(got, np.concatenate([rows, run_rows[:, ::-1]]))
