@@ -1163,6 +1163,8 @@ void plan_pull(const gdl_engine *e, const LieHost &L, Plan &p) {
     const u64 bytes = e->h[op.inner].full.n * (4ull << (L.dk - 5));
     if (e->row_gather != 3 && bytes > kRowsBudget) continue;
     if (op.outer_ver == GDL_DELTA && !fused_update(p, op.outer)) continue;
+    // (a transposed output goes to NEWT's rows, which are this join's input)
+    if (op.outer_ver == GDL_NEWT && op.outer == op.out && p.pull_t[oi]) continue;
     p.rows[oi] = 1;
     p.product[oi] = 0;
   }
@@ -1662,6 +1664,10 @@ bool hash_form(const gdl_engine *e, const LieHost &L, const Plan &plan) {
       return false;
     if (op.outer_ver == GDL_FULL && (!is_static[op.outer] || is_update[op.outer])) return false;
     if (op.outer_ver == GDL_NEWT && is_update[op.outer]) return false;
+    // (a join that appends to the NEWT it reads: probe, expansion and append
+    // are one pass here, whose blocks would see each other's tuples, or rows
+    // counted and not yet stored)
+    if (op.outer_ver == GDL_NEWT && op.outer == op.out) return false;
     // (with dependent columns no key may be all ones, which looks like an
     // empty slot: column 0 stays below 2^32 - 1)
     if (is_update[op.out] && e->rels[op.out].dep &&

@@ -1,0 +1,52 @@
+"""Programs at the edges of the rules that pick a fixpoint's form (hash sets,
+row gathers, resident loops, linear recursion), against the CPU oracle."""
+import numpy as np
+import pytest
+
+import programs as P
+import workloads as W
+from gdlog_b200 import DELTA, FULL, INNER, NEWT, OUTER, PLUS, Engine
+
+pytestmark = pytest.mark.gpu
+
+
+def both(prog, *args, mode=None):
+    with Engine("gpu", dedup=mode) as g:
+        got = prog(g, *args)
+    with Engine("oracle") as o:
+        want = prog(o, *args)
+    assert got == want
+    return got
+
+
+def state(lie, *rels):
+    return [(r.size(), r.digest()) for r in rels] + [lie.trace().tolist()]
+
+
+def tmp_joined_into_itself(eng, edges, sel):
+    """tmp :- edge, tmp: the join reads the NEWT that it appends to, as it was
+    when the join began."""
+    edge = eng.relation("edge")
+    out = eng.relation("out", index_flag=False)
+    tmp = eng.relation("tmp", index_flag=False, tmp_flag=True)
+    eng.load(edge, edges)
+    eng.load(out, edges[::3])
+    eng.load(tmp, None)
+    lie = eng.lie()
+    lie.add_relations(edge, True)
+    lie.add_relations(out, False)
+    lie.add_tmp_relation(tmp)
+    lie.add_join(edge, FULL, out, DELTA, tmp, (OUTER(1), INNER(1)))
+    lie.add_join(edge, FULL, tmp, NEWT, tmp, sel)
+    lie.add_join(edge, FULL, tmp, NEWT, out, (OUTER(1), INNER(1)))
+    return [lie.fixpoint()] + state(lie, out)
+
+
+@pytest.mark.parametrize("sel", [(OUTER(1), INNER(1)), (INNER(1), OUTER(1))])
+@pytest.mark.parametrize("base,mode", [(0, None), (0, "dense_rows"), (70000, None),
+                                       (70000, "sort")])
+def test_tmp_joined_into_itself(base, mode, sel):
+    """Ids below 2^13 (bitmaps) and from 70,000 on (lists)."""
+    edges = W.rmat_edges(13, 3000, seed=8) + np.uint64(base)
+    got = both(tmp_joined_into_itself, edges, sel, mode=mode)
+    assert got[0] > 2
