@@ -1804,20 +1804,25 @@ HashJoinArgs hash_join_args(gdl_engine *e, LieHost &L, const Plan &plan, size_t 
   return h;
 }
 
-// The hash form's resident loop: its joins, then an entry for each update
-// relation with dependent columns.
+// The hash form's resident loop: its joins, then an entry for each relation
+// whose candidates they may put aside, an update relation with dependent
+// columns that one of them derives (at most one a join: the loop's last block
+// looks at their counts a lane each).
+static_assert(kHashLoopOps <= 32, "asides, a lane each");
 gdl_status push_hash_loop(gdl_engine *e, LieHost &L, const Plan &plan) {
   std::vector<HashJoinArgs> ops;
   for (size_t oi = 0; oi < L.ops.size(); oi++) ops.push_back(hash_join_args(e, L, plan, oi));
-  for (int r : L.update)
-    if (e->rels[r].dep) {
+  for (int r : L.update) {
+    bool derived = false;
+    for (const OpHost &op : L.ops) derived = derived || op.out == r;
+    if (e->rels[r].dep && derived) {
       JoinArgs a;
       memset(&a, 0, sizeof a);
       a.ctl = e->d_ctl;
       ops.push_back(hash_args(e, a, r, true));
     }
-  if (!L.d_hops)
-    TRY(dalloc(e, (void **)&L.d_hops, (kHashLoopOps + kMaxRels) * sizeof(HashJoinArgs)));
+  }
+  if (!L.d_hops) TRY(dalloc(e, (void **)&L.d_hops, 2 * kHashLoopOps * sizeof(HashJoinArgs)));
   CK(e, cudaMemcpyAsync(L.d_hops, ops.data(), ops.size() * sizeof(HashJoinArgs),
                         cudaMemcpyHostToDevice, e->s));
   L.n_steps = (int)ops.size();

@@ -50,3 +50,36 @@ def test_tmp_joined_into_itself(base, mode, sel):
     edges = W.rmat_edges(13, 3000, seed=8) + np.uint64(base)
     got = both(tmp_joined_into_itself, edges, sel, mode=mode)
     assert got[0] > 2
+
+
+def many_path_relations(eng, n, edges, first):
+    """n relations with a dependent column in one LIE; the last is derived."""
+    edge = eng.relation("edge")
+    paths = [eng.relation(f"path{i}", arity=3, dependent_column_size=1, index_flag=False)
+             for i in range(n)]
+    for i, p in enumerate(paths):
+        eng.load(p, first[i % 3::3])
+    eng.load(edge, W.reverse(edges))
+    lie = eng.lie()
+    lie.add_relations(edge, True)
+    for p in paths:
+        lie.add_relations(p, False)
+    last = paths[-1]
+    lie.add_join(edge, FULL, last, DELTA, last, (INNER(1), OUTER(1), PLUS(OUTER(2), 1)))
+    return [lie.fixpoint()] + state(lie, *paths)
+
+
+@pytest.mark.parametrize("n", [31, 33, 40])
+def test_asides_of_many_relations(n):
+    """Tuples that differ in a dependent column only are put aside until the
+    joins are done, whatever the relation's place in the LIE."""
+    rng = np.random.default_rng(n)
+    edges = W.layered_dag(7, 9, 3)
+    first = np.stack([rng.integers(0, 63, 600), rng.integers(0, 8, 600),
+                      rng.integers(1, 6, 600)], axis=1).astype(np.uint64)
+    got = []
+    for mode in (None, "sort"):
+        with Engine("gpu", dedup=mode) as g:
+            got.append(many_path_relations(g, n, edges, first))
+    assert got[0] == got[1]
+    assert got[0][n][0] > 2 * 200  # (the derived relation grew)
