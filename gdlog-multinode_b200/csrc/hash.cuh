@@ -388,7 +388,8 @@ struct HashLoopArgs {
 
 // Every iteration of a LIE.  A join's barrier tells whether it left pieces of
 // long runs, the last join's whether candidates were put aside; when neither,
-// that barrier commits.  An overflow ends the loop uncommitted.
+// that barrier commits.  An overflow ends the loop uncommitted, at the first
+// barrier after it.
 __global__ void __launch_bounds__(256, kHashLoopCtasPerSm) k_hash_loop(HashLoopArgs a) {
   __shared__ HashSmem sm;
   __shared__ HashJoinArgs s_op[kHashLoopOps];
@@ -398,7 +399,9 @@ __global__ void __launch_bounds__(256, kHashLoopCtasPerSm) k_hash_loop(HashLoopA
   __syncthreads();
   Ctl *ctl = a.ctl;
   u32 gen = ctl->bar_word >> 2;
-  u32 flags = ctl_stop(ctl) ? 1u : 0u;
+  // (not the overflow flag: a block may start after another has raised it, and
+  // each of them arrives at the first barrier or none does)
+  u32 flags = (ctl->done | ctl->pause | ctl->timeout) ? 1u : 0u;
   const LaneLists lists = lane_lists(a.lie, threadIdx.x & 31);
   // the asides' counts, a relation a lane
   const u64 *aside_n = nullptr;
