@@ -1883,6 +1883,7 @@ gdl_status push_loop(gdl_engine *e, LieHost &L, const Plan &plan) {
     LoopStep st;
     memset(&st, 0, sizeof st);
     st.kind = kind;
+    st.delta_rel = -1;
     return st;
   };
   std::vector<char> twin_full(e->rels.size(), 0);  // twin written and not folded yet
@@ -1915,7 +1916,7 @@ gdl_status push_loop(gdl_engine *e, LieHost &L, const Plan &plan) {
     st.inner_vis = a.inner_vis;
     st.outer_bm = a.outer_bm;
     st.outer_words = a.outer_bm_words;
-    st.outer_rel = op.outer;
+    st.op = (int)oi;
     if (plan.rows[oi]) {
       if (plan.out_twin[oi]) fold(op.out);  // (it may expect a zero twin)
       const RowsArgs ra = rows_args(e, L, plan, oi, a);
@@ -1948,8 +1949,9 @@ gdl_status push_loop(gdl_engine *e, LieHost &L, const Plan &plan) {
       st.src = pa.OT;
       st.F = pa.F;
       st.dst = pa.G;
-      // (a DELTA outer zeroed by an empty inner: in operator order within a
-      // level, published at its end)
+      // (a DELTA outer zeroed by an empty inner is no use: LoopStep::before
+      // holds the operators' order)
+      st.delta_rel = op.outer_ver == GDL_DELTA ? op.outer : -1;
       Use u{{st.src, st.F, st.inner, st.inner_vis}, {st.dst}, {}};
       if (!st.outer_vis) u.writes = {st.outer, st.outer_bm};
       add(st, u);
@@ -1971,6 +1973,10 @@ gdl_status push_loop(gdl_engine *e, LieHost &L, const Plan &plan) {
     L.resident = false;
     return GDL_OK;
   }
+  for (LoopStep &st : steps)
+    for (size_t k = 0; k < steps.size(); k++)
+      if (st.delta_rel >= 0 && steps[k].delta_rel == st.delta_rel && steps[k].op < st.op)
+        st.before |= 1ull << k;
   std::vector<LoopUpd> upd;
   for (int r : L.update) {
     const RelDev &h = e->h[r];

@@ -46,7 +46,10 @@ struct LoopStep {
   const u32 *inner_vis;
   u32 *outer_bm;         // NEWT outer: its bitmap and words
   u64 outer_words;
-  int outer_rel;
+  int op;                // place in the LIE
+  int delta_rel;         // product: relation whose DELTA is the outer, else -1
+  u64 before;            // product: the steps (by number) of operators before
+                         // this one with the same DELTA as their outer
   // product: OT, F -> dst; rows: O -> dst; transpose and fold: src -> dst
   const u32 *src, *F;
   u32 *dst;
@@ -408,25 +411,37 @@ __global__ void __launch_bounds__(kLoopBlock, 2) k_lie_loop(LoopArgs a) {
   // work do not all fall to the first blocks)
   auto block_for = [&](u32 i) { return (blockIdx.x + i * 61u) % gridDim.x; };
   while (go) {
+    // Products whose inner is empty, by step.  Inners are FULLs that only the
+    // commit changes, so the iteration's first level looks at all of them.  An
+    // empty inner zeroes its outer's DELTA for the operators after its own
+    // (src/join.cu:42-45): levels reorder steps, so each step knows which
+    // operators those are (LoopStep::before).
+    u64 no_inner = 0;
     for (int i = 0; i < a.n_steps && go;) {
-      // the steps of one level; lane k looks at the sides of the k-th (their
+      // the steps of one level; lane k looks at the outer of the k-th (the
       // loads take one round trip together)
       const int i0 = i, i1 = s_step[i0].level_end;
-      u32 no_inner = 0, no_outer = 0;
+      u32 no_outer = 0;
       if (V == 0) {
-        bool ni = false, no = false;
-        if (i0 + (int)(threadIdx.x & 31) < i1) {
-          const LoopStep &st = s_step[i0 + (threadIdx.x & 31)];
-          if (st.kind == kLoopProduct) {
-            const u64 x = eff_count(st.inner, st.inner_vis), y = eff_count(st.outer, st.outer_vis);
-            ni = x == 0;
-            no = y == 0;
+        const int lane = threadIdx.x & 31;
+        bool ni[2] = {false, false}, no = false;
+        if (i0 == 0) {
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            const LoopStep &st = s_step[lane + 32 * h];
+            if (lane + 32 * h < a.n_steps && st.kind == kLoopProduct)
+              ni[h] = eff_count(st.inner, st.inner_vis) == 0;
           }
         }
-        no_inner = __ballot_sync(0xffffffffu, ni);
+        if (i0 + lane < i1) {
+          const LoopStep &st = s_step[i0 + lane];
+          if (st.kind == kLoopProduct) no = eff_count(st.outer, st.outer_vis) == 0;
+        }
+        if (i0 == 0)
+          no_inner = __ballot_sync(0xffffffffu, ni[0]) |
+                     ((u64)__ballot_sync(0xffffffffu, ni[1]) << 32);
         no_outer = __ballot_sync(0xffffffffu, no);
       }
-      u64 zeroed = 0;  // relations whose DELTA an empty inner zeroed (src/join.cu:42-45)
       for (; i < i1; i++) {
         const LoopStep &st = s_step[i];
         if (st.kind == kLoopRows) {
@@ -462,14 +477,9 @@ __global__ void __launch_bounds__(kLoopBlock, 2) k_lie_loop(LoopArgs a) {
           }
         } else if (st.kind == kLoopProduct) {
           if (V == 0) {
-            if ((no_inner >> (i - i0)) & 1u) {
-              // (written by the barrier: blocks of this level still read it)
-              if (st.outer_vis)
-                zeroed |= 1ull << st.outer_rel;
-              else
-                loop_clear(st);
-            } else if (!((no_outer >> (i - i0)) & 1u) &&
-                       !(st.outer_vis && ((zeroed >> st.outer_rel) & 1ull))) {
+            if ((no_inner >> i) & 1ull) {
+              if (!st.outer_vis) loop_clear(st);  // (its count: by the barrier)
+            } else if (!((no_outer >> (i - i0)) & 1u) && !(no_inner & st.before)) {
               ProdArgs pa;
               pa.j.ctl = nullptr;
               pa.OT = st.src;
@@ -496,7 +506,7 @@ __global__ void __launch_bounds__(kLoopBlock, 2) k_lie_loop(LoopArgs a) {
             st.count_to->n = *st.count_acc;
             *st.count_acc = 0;
           }
-          if ((no_inner >> (k - i0)) & 1u) loop_empty_inner(st);
+          if (((no_inner >> k) & 1ull) && !st.outer_vis) loop_empty_inner(st);
         }
         return false;
       });

@@ -83,3 +83,49 @@ def test_asides_of_many_relations(n):
             got.append(many_path_relations(g, n, edges, first))
     assert got[0] == got[1]
     assert got[0][n][0] > 2 * 200  # (the derived relation grew)
+
+
+def hidden_delta(eng, ids, order):
+    """Operators around one whose inner is empty, which zeroes its outer's
+    DELTA for the operators after it in the LIE and for no others."""
+    rng = np.random.default_rng(ids)
+    rel = {k: eng.relation(k, index_flag=False) for k in "abc"}
+    rel["t"] = eng.relation("t", index_flag=False, tmp_flag=True)
+    for k in "efz":
+        rel[k] = eng.relation(k)
+    for k, n in dict(a=ids // 4, b=ids // 8, c=ids // 8, e=ids, f=ids).items():
+        rows = rng.integers(0, ids, size=(n, 2))
+        rows[0] = ids - 1
+        eng.load(rel[k], rows.astype(np.uint64))
+    for k in "zt":
+        eng.load(rel[k], None)
+    lie = eng.lie()
+    for k in "efz":
+        lie.add_relations(rel[k], True)
+    for k in "abc":
+        lie.add_relations(rel[k], False)
+    lie.add_tmp_relation(rel["t"])
+    for rule in order.split():
+        out, outer, inner = rule
+        lie.add_join(rel[inner], FULL, rel[outer], NEWT if outer == "t" else DELTA, rel[out],
+                     (OUTER(1), INNER(1)))
+    lie.max_iteration = 6
+    return [lie.fixpoint()] + state(lie, rel["a"], rel["b"], rel["c"])
+
+
+@pytest.mark.parametrize("ids", [300, 700, 1500, 3000])
+@pytest.mark.parametrize("order", [
+    "tae bte taf cte caz abe",   # the empty inner last, of a step without a conflict
+    "tae bte taz caf abe",       # ... in the middle, an operator without a conflict after it
+    "caz tae bte abe",           # ... first
+    "tae btz cte caf abe",       # a tmp outer emptied before its second reader
+])
+def test_empty_inner_hides_a_delta_in_operator_order(ids, order):
+    both(hidden_delta, ids, order)
+    both(hidden_delta, ids, order, mode="dense_push")
+
+
+@pytest.mark.parametrize("quirks", ["pull_quirks", "rows_quirks", "static_outer_quirks"])
+def test_quirks_in_the_default_forms(quirks):
+    import test_pull
+    both(getattr(test_pull, quirks))
