@@ -1900,7 +1900,7 @@ gdl_status push_loop(gdl_engine *e, LieHost &L, const Plan &plan) {
     const RelDev &out = e->h[op.out];
     if (op.kind == 2) {
       fold(op.inner);
-      twin_full[op.out] = 0;  // (the copy replaces NEWT)
+      fold(op.out);  // (the copy replaces NEWT: nothing of it stays in the twin)
       LoopStep st = blank(kLoopTranspose);
       st.src = e->h[op.inner].bmG;
       st.dst = out.bmG;

@@ -129,3 +129,34 @@ def test_empty_inner_hides_a_delta_in_operator_order(ids, order):
 def test_quirks_in_the_default_forms(quirks):
     import test_pull
     both(getattr(test_pull, quirks))
+
+
+def copied_over(eng, ids, again):
+    """A column-swapping ACopy into a relation whose NEWT a join with a
+    transposed output wrote before: the copy replaces that NEWT."""
+    rng = np.random.default_rng(ids)
+    x, y, a = (eng.relation(k, index_flag=False) for k in "xya")
+    e = eng.relation("e")
+    for r, n in ((x, 9), (y, ids // 8), (a, ids // 4), (e, ids)):
+        rows = rng.integers(0, ids, size=(n, 2))
+        rows[0] = ids - 1
+        eng.load(r, rows.astype(np.uint64))
+    lie = eng.lie()
+    lie.add_relations(e, True)
+    for r in (x, y, a):
+        lie.add_relations(r, False)
+    lie.add_join(e, FULL, y, DELTA, y, (OUTER(1), INNER(1)))
+    lie.add_join(e, FULL, a, DELTA, x, (INNER(1), OUTER(1)))
+    lie.add_acopy(y, x, P.CP_SWAP)
+    if again:
+        lie.add_join(e, FULL, x, DELTA, x, (INNER(1), OUTER(1)))
+        lie.add_join(e, FULL, x, DELTA, a, (OUTER(1), INNER(1)))
+    lie.max_iteration = 6
+    return [lie.fixpoint()] + state(lie, x, y, a)
+
+
+@pytest.mark.parametrize("again", [False, True])
+@pytest.mark.parametrize("ids", [300, 700, 1500, 3000, 5000])
+def test_acopy_replaces_what_a_transposed_output_wrote(ids, again):
+    both(copied_over, ids, again)
+    both(copied_over, ids, again, mode="dense_push")
