@@ -2016,8 +2016,10 @@ bool closure_form(const gdl_engine *e, const LieHost &L) {
       !L.tmps.empty() || L.max_iteration < 2147483647LL || (!e->instances && L.dk < kPullMinBits))
     return false;
   const OpHost &op = L.ops[0];
+  // (a static relation that was the outer of an empty inner in an earlier LIE
+  // counts as empty, src/join.cu:42-45; the edges here come from its rows)
   bool stat = false;
-  for (int r : L.statics) stat = stat || r == op.inner;
+  for (int r : L.statics) stat = stat || (r == op.inner && e->h[r].full_vis);
   return op.kind == 0 && !op.hook && !op.generic && op.pred.kind == 0 && stat &&
          op.inner_ver != GDL_DELTA && op.inner != op.out && op.outer == L.update[0] &&
          op.out == L.update[0] && op.outer_ver == GDL_DELTA && op.sel.s0 == 1 && op.sel.s1 == 3;

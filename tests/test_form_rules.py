@@ -160,3 +160,51 @@ def copied_over(eng, ids, again):
 def test_acopy_replaces_what_a_transposed_output_wrote(ids, again):
     both(copied_over, ids, again)
     both(copied_over, ids, again, mode="dense_push")
+
+
+def closure_of_a_hidden_relation(eng, edges, shift):
+    """A first LIE zeroes edge's count (it is the outer of an empty inner,
+    src/join.cu:42-45); the closure over it then derives nothing."""
+    edge = eng.relation("edge")
+    none = eng.relation("none")
+    other = eng.relation("other", index_flag=False)
+    path = eng.relation("path", index_flag=False)
+    rows = np.concatenate([edges, edges | np.uint64(1 << shift)]) if shift else edges
+    eng.load(edge, W.reverse(rows))
+    eng.load(path, rows)
+    eng.load(none, None)
+    eng.load(other, None)
+    first = eng.lie()
+    first.add_relations(none, True)
+    first.add_relations(edge, True)
+    first.add_relations(other, False)
+    first.add_join(none, FULL, edge, FULL, other, (OUTER(1), INNER(1)))
+    it0 = first.fixpoint()
+    lie = eng.lie()
+    lie.add_relations(edge, True)
+    lie.add_relations(path, False)
+    lie.add_join(edge, FULL, path, DELTA, path, P.REORDER_PATH)
+    it = [it0, lie.fixpoint()]
+    if shift:
+        return it + [path.instance_stats(2)[0].tolist()]
+    return it + state(lie, path)
+
+
+def test_closure_over_a_relation_that_counts_as_empty():
+    e = W.grid_edges(17, 23)
+    got = both(closure_of_a_hidden_relation, e, 0)
+    assert got[2][0] == len(e)
+    both(closure_of_a_hidden_relation, e, 0, mode="dense_push")
+
+
+def test_batched_closure_over_a_relation_that_counts_as_empty(monkeypatch):
+    e = W.grid_edges(5, 8)
+    got = []
+    for no_graph in (False, True):
+        if no_graph:
+            monkeypatch.setenv("GDLOG_NO_GRAPH", "1")
+        with Engine("gpu") as g:
+            shift = g.set_instances([40, 40])
+            got.append(closure_of_a_hidden_relation(g, e, shift))
+    assert got[0] == got[1]
+    assert got[0][2] == [len(e), len(e)]
