@@ -258,6 +258,20 @@ __global__ void __launch_bounds__(256) k_closure_degree(const u32 *start, const 
   if ((threadIdx.x & 31) == 0 && m) atomicMax(max_degree, m);
 }
 
+// Whether both columns lie in one instance.
+__device__ __forceinline__ bool closure_inside(const ClosureRows &m, u64 k) {
+  return !m.row_first || (((key_c0(k) ^ key_c1(k)) >> m.shift) == 0 &&
+                          closure_row_of(m, key_c0(k)) != kNoWord &&
+                          closure_row_of(m, key_c1(k)) != kNoWord);
+}
+// The first DELTA's tuples out of the instances or between two: as bad edges.
+__global__ void __launch_bounds__(256) k_closure_check(const u64 *keys, u64 n, ClosureRows m,
+                                                       u32 *bad) {
+  for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (u64)gridDim.x * blockDim.x)
+    if (!closure_inside(m, keys[i])) *bad = 1;
+}
+
 // The first DELTA: extents of its rows, those words zeroed, then the bits
 // set (k_bm_from_list).
 __global__ void __launch_bounds__(256) k_closure_ext(const DArr *list, ClosureRows m, uint2 *ext) {
@@ -265,8 +279,8 @@ __global__ void __launch_bounds__(256) k_closure_ext(const DArr *list, ClosureRo
   for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (u64)gridDim.x * blockDim.x) {
     const u64 k = list->ptr[i];
+    if (!closure_inside(m, k)) continue;  // (no extent past its row)
     const u32 r = closure_row_of(m, key_c0(k));
-    if (r == kNoWord || (m.row_first && closure_row_of(m, key_c1(k)) == kNoWord)) continue;
     const u32 c = m.row_first ? key_c1(k) & ((1u << m.shift) - 1u) : key_c1(k);
     atomicMin(&ext[r].x, c >> 5);
     atomicMax(&ext[r].y, (c >> 5) + 1);

@@ -2055,7 +2055,7 @@ gdl_status prepare_closure(gdl_engine *e, LieHost &L) {
   p += 4 * rows;
   u32 *maxdeg = p;
   p += 4;
-  CK(e, cudaMemsetAsync(maxdeg, 0, 2 * sizeof(u32), e->s));  // and the bad-edge flag
+  CK(e, cudaMemsetAsync(maxdeg, 0, 2 * sizeof(u32), e->s));  // and the flag of bad tuples
   ClosureRows m{nullptr, nullptr, 1, 31};
   if (e->instances) {
     u32 *start = p, *end = p + rows, *word = p + 2 * rows, *inst = p + 3 * rows;
@@ -2080,6 +2080,11 @@ gdl_status prepare_closure(gdl_engine *e, LieHost &L) {
                                                                     maxdeg + 1);
       e->aux_launches++;
       dfree(e, keys);  // stream-ordered
+    }
+    if (e->h[r].delta.n) {
+      k_closure_check<<<grid_for(e, e->h[r].delta.n, 256, 8), 256, 0, e->s>>>(
+          e->h[r].delta.ptr, e->h[r].delta.n, m, maxdeg + 1);
+      e->aux_launches++;
     }
     a.start = start;
     a.end = end;

@@ -5,7 +5,7 @@ import pytest
 
 import programs as P
 import workloads as W
-from gdlog_b200 import DELTA, FULL, INNER, NEWT, OUTER, PLUS, Engine
+from gdlog_b200 import DELTA, FULL, INNER, NEWT, OUTER, PLUS, Engine, GdlError
 
 pytestmark = pytest.mark.gpu
 
@@ -208,3 +208,36 @@ def test_batched_closure_over_a_relation_that_counts_as_empty(monkeypatch):
             got.append(closure_of_a_hidden_relation(g, e, shift))
     assert got[0] == got[1]
     assert got[0][2] == [len(e), len(e)]
+
+
+@pytest.mark.parametrize("bad,refused", [
+    (((1 << 10) | 3, 599), True), (((1 << 10) | 7, 599), True), ((31, (1 << 10) | 7), True),
+    ((599, 600), True), ((1 << 10, 599), False), ((0, (1 << 10) | 8), False)])
+def test_first_tuples_out_of_their_instance(bad, refused, monkeypatch):
+    """A batched closure whose path holds a tuple between instances, or past
+    an instance's nodes (the edges do not): what the general path does, which
+    refuses the tuples derived from it."""
+    def run():
+        with Engine("gpu") as g:
+            assert g.set_instances([600, 8]) == 10
+            small = W.grid_edges(2, 4)
+            edges = np.concatenate([W.grid_edges(20, 30), small | np.uint64(1 << 10)])
+            edge = g.relation("edge")
+            path = g.relation("path", index_flag=False)
+            g.load(edge, W.reverse(edges))
+            g.load(path, np.concatenate([edges, np.array([bad], dtype=np.uint64)]))
+            lie = g.lie()
+            lie.add_relations(edge, True)
+            lie.add_relations(path, False)
+            lie.add_join(edge, FULL, path, DELTA, path, P.REORDER_PATH)
+            try:
+                lie.fixpoint()
+            except GdlError as err:
+                return err.code
+            sizes, digests = path.instance_stats(2)
+            return sizes.tolist(), digests.tolist()
+
+    got = run()
+    assert isinstance(got, int) == refused
+    monkeypatch.setenv("GDLOG_NO_GRAPH", "1")
+    assert got == run()
