@@ -43,6 +43,7 @@
 #include "sort.cuh"
 #include "tma.cuh"
 #include "exchange.cuh"
+#include "export.cuh"
 #include "hash.cuh"
 
 #include <algorithm>
@@ -57,7 +58,6 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
-#include <system_error>
 #include <tuple>
 #include <mutex>
 #include <vector>
@@ -4228,82 +4228,48 @@ gdl_status gdl_relation_size(gdl_engine *e, int32_t rel, int32_t ver, uint64_t *
   return GDL_OK;
 }
 
-// A sorted version's keys to the caller's rows.  The keys come over in
-// pieces through a pinned buffer that the engine keeps, and threads unpack
-// each piece as it lands: the caller's pages are mostly untouched before
-// (one thread spent 25 of 35 ms on faulting them in for 4.3 M rows of three
-// columns).
-constexpr u64 kExportPiece = 1ull << 18;    // keys
-constexpr u64 kExportPinned = 1ull << 23;   // keys the pinned buffer holds at most
-static gdl_status export_keys(gdl_engine *e, const u64 *p, u64 n, int ar, uint64_t *rows) {
-  const u64 want = std::min(n, kExportPinned);
-  if (e->pin_cap < want) {
-    if (e->pin_keys) cudaFreeHost(e->pin_keys);
-    e->pin_keys = nullptr;
-    e->pin_cap = 0;
-    CK(e, cudaMallocHost(&e->pin_keys, want * sizeof(u64)));
-    e->pin_cap = want;
-  }
-  const int k2 = e->k2;
-  const unsigned hc = std::thread::hardware_concurrency();
-  const int nt = (int)std::min<u64>(std::min<u64>(hc ? hc : 1, 8), n / kExportPiece + 1);
+// The engine's side of export_pieces (export.cuh).
+struct ExportApi {
+  gdl_engine *e;
   std::vector<cudaEvent_t> evs;
-  gdl_status st = GDL_OK;
-  for (u64 base = 0; base < n && st == GDL_OK; base += e->pin_cap) {
-    const u64 m = std::min(n - base, e->pin_cap);
-    const u64 pieces = (m + kExportPiece - 1) / kExportPiece;
-    while (evs.size() < pieces) {
+  std::atomic<int> err{cudaSuccess};
+  explicit ExportApi(gdl_engine *eng) : e(eng) {}
+  ~ExportApi() {
+    for (cudaEvent_t ev : evs) e->ev_pool.push_back(ev);
+  }
+  bool ok(cudaError_t r) {
+    if (r != cudaSuccess) err = r;
+    return r == cudaSuccess;
+  }
+  u64 *buffer(u64 keys, u64 *cap) {
+    if (e->pin_cap < keys) {
+      if (e->pin_keys) cudaFreeHost(e->pin_keys);
+      e->pin_keys = nullptr;
+      e->pin_cap = 0;
+      if (!ok(cudaMallocHost(&e->pin_keys, keys * sizeof(u64)))) {
+        e->pin_keys = nullptr;
+        return nullptr;
+      }
+      e->pin_cap = keys;
+    }
+    *cap = e->pin_cap;
+    return e->pin_keys;
+  }
+  bool marks(u64 n) {
+    while (evs.size() < n) {
       cudaEvent_t ev = take_event(e);
-      if (!ev) return fail(e, GDL_E_CUDA, "cudaEventCreate failed");
+      if (!ev) return false;
       evs.push_back(ev);
     }
-    for (u64 q = 0; q < pieces; q++) {
-      const u64 o = q * kExportPiece, c = std::min(kExportPiece, m - o);
-      cudaMemcpyAsync(e->pin_keys + o, p + base + o, c * sizeof(u64), cudaMemcpyDeviceToHost, e->s);
-      cudaEventRecord(evs[q], e->s);
-    }
-    std::atomic<u64> next{0};
-    std::atomic<bool> bad{false};
-    const int dev = e->device;
-    auto work = [&, dev] {
-      cudaSetDevice(dev);
-      for (u64 q; (q = next.fetch_add(1)) < pieces;) {
-        if (cudaEventSynchronize(evs[q]) != cudaSuccess) {
-          bad = true;
-          return;
-        }
-        const u64 o = q * kExportPiece, c = std::min(kExportPiece, m - o);
-        const u64 *k = e->pin_keys + o;
-        uint64_t *d = rows + (base + o) * ar;
-        if (ar == 2) {
-          for (u64 i = 0; i < c; i++) {
-            d[2 * i] = k[i] >> 32;
-            d[2 * i + 1] = (u32)k[i];
-          }
-        } else {
-          const u64 low = (1ull << k2) - 1;
-          for (u64 i = 0; i < c; i++) {
-            d[3 * i] = k[i] >> 32;
-            d[3 * i + 1] = (u32)k[i] >> k2;
-            d[3 * i + 2] = k[i] & low;
-          }
-        }
-      }
-    };
-    std::vector<std::thread> pool;
-    try {
-      for (int t = 1; t < nt; t++) pool.emplace_back(work);
-    } catch (const std::system_error &) {
-      // (fewer threads then)
-    }
-    work();
-    for (std::thread &t : pool) t.join();
-    const cudaError_t r = cudaStreamSynchronize(e->s);
-    if (bad || r != cudaSuccess) st = fail(e, GDL_E_CUDA, "export: %s", cudaGetErrorString(r));
+    return true;
   }
-  for (cudaEvent_t ev : evs) e->ev_pool.push_back(ev);
-  return st;
-}
+  bool copy(u64 *dst, const u64 *src, u64 n) {
+    return ok(cudaMemcpyAsync(dst, src, n * sizeof(u64), cudaMemcpyDeviceToHost, e->s));
+  }
+  bool mark(u64 i) { return ok(cudaEventRecord(evs[i], e->s)); }
+  bool wait(u64 i) { return ok(cudaSetDevice(e->device)) && ok(cudaEventSynchronize(evs[i])); }
+  bool finish() { return ok(cudaStreamSynchronize(e->s)); }
+};
 
 gdl_status gdl_relation_export(gdl_engine *e, int32_t rel, int32_t ver, uint64_t *rows,
                                uint64_t cap, uint64_t *out_n) {
@@ -4319,7 +4285,12 @@ gdl_status gdl_relation_export(gdl_engine *e, int32_t rel, int32_t ver, uint64_t
       if (n > cap)
         return fail(e, GDL_E_CAPACITY, "export needs %llu rows", (unsigned long long)n);
       if (!rows) return GDL_E_INVALID;
-      return export_keys(e, p, n, e->rels[rel].arity, rows);
+      ExportApi api(e);
+      const ExportEnd end = export_pieces(api, p, n, e->rels[rel].arity, e->k2, rows);
+      if (end == kExported) return GDL_OK;
+      if (end == kExportFailed)
+        return fail(e, GDL_E_CUDA, "export: %s", cudaGetErrorString((cudaError_t)api.err.load()));
+      cudaGetLastError();  // (no pinned memory: in one copy, below)
     }
   }
   std::vector<u64> k;
