@@ -15,8 +15,10 @@
 // From 2^14 ids an iteration's own work is larger than the launches, and the
 // TMA passes (tma.cuh) do it faster than the passes here.
 //
-// Every wait is bounded (Ctl::spin_limit polls): a block that gives up
-// raises Ctl::timeout and leaves, and the others leave when they see it.
+// Every wait is bounded: a block that gives up raises Ctl::timeout and leaves,
+// and the others leave when they see it.  At a barrier a block waits for the
+// others' whole steps, not for one tile, so the bound there is kBarrierPolls
+// or Ctl::spin_limit, whichever is more.
 #pragma once
 
 #include "common.cuh"
@@ -29,6 +31,8 @@ namespace gdl {
 
 constexpr int kLoopBlock = 256;
 constexpr int kLoopMaxBits = 13;
+
+constexpr u32 kBarrierPolls = 1u << 25;  // some twenty seconds
 
 constexpr int kLoopMaxSteps = 64;  // at most 32 of one level
 constexpr int kLoopMaxUpd = 32;
@@ -117,7 +121,7 @@ __device__ __forceinline__ u32 loop_barrier_flags(Ctl *ctl, u32 &gen, int *s_go,
                      : "memory");
       }
     } else if (lane == 0) {
-      const u32 limit = ctl->spin_limit;
+      const u32 limit = max(ctl->spin_limit, kBarrierPolls);
       for (u32 polls = 0;; polls++) {
         asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(word) : "l"(&ctl->bar_word) : "memory");
         if ((word >> 2) != gen) break;

@@ -161,7 +161,10 @@ typedef struct gdl_tuning {
                                   <= 4 GB; default), 3 = whenever possible */
   int32_t spin_limit_log2;     /* a bounded device-side wait (look-back of a scan)
                                   gives up after 2^this polls and the call
-                                  returns GDL_E_TIMEOUT (default 22; 1..30) */
+                                  returns GDL_E_TIMEOUT (default 22; 1..30).
+                                  A resident loop's barrier, where a block
+                                  waits for the others' steps, gives up after
+                                  2^25 polls, or 2^this where that is more */
   int32_t radix_bits;          /* digit width of the radix sort: 6, 8 (default) or
                                   10 bits (64 / 256 / 1024 buckets a pass); a
                                   width that would need more than 8 passes

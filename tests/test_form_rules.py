@@ -241,3 +241,16 @@ def test_first_tuples_out_of_their_instance(bad, refused, monkeypatch):
     assert isinstance(got, int) == refused
     monkeypatch.setenv("GDLOG_NO_GRAPH", "1")
     assert got == run()
+
+
+@pytest.mark.parametrize("polls_log2", [6, 7])
+def test_wait_limit_of_a_look_back_is_not_the_barriers(polls_log2):
+    """A block waits at a resident loop's barrier for the others' steps (here
+    over 100 us, some 200 polls), which a limit that suits a look-back must
+    not cut short."""
+    args = W.cspa_facts(2000, 4000, 1500, seed=1)
+    with Engine("gpu") as g:
+        want = P.cspa(g, *args).relations["value_alias"].digest()
+        g.clear()
+        g.set_tuning(spin_limit_log2=polls_log2)
+        assert P.cspa(g, *args).relations["value_alias"].digest() == want
