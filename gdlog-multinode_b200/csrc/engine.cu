@@ -1698,19 +1698,22 @@ gdl_status ensure_hash(gdl_engine *e, int r) {
   if (dep && !h.hord) TRY(dalloc(e, (void **)&h.hord, (h.hmask + 2) * sizeof(u32)));
   return GDL_OK;
 }
-// Lists and sets of a LIE in the hash form: room for a few million tuples
-// before the first growth.
+// Lists and sets of a LIE in the hash form, with room for its first growth
+// (kHashGrowth).
 gdl_status prepare_hash(gdl_engine *e, LieHost &L) {
+  u64 most = 0;
+  for (auto *v : {&L.update, &L.statics})
+    for (int r : *v) most = std::max<u64>(most, e->h[r].full.n);
+  const u64 rows = std::max<u64>(kMinCap, std::min<u64>(kHashGrowth * most, kHashFirstRows));
   for (int r : L.update) {
     RelDev &h = e->h[r];
-    TRY(ensure_arr(e, h.full, std::max<u64>(kHashMinRows, std::min<u64>(2 * h.full.n, kMaxRows)),
-                   true));
-    TRY(ensure_arr(e, h.delta, kHashMinRows, true));
+    TRY(ensure_arr(e, h.full, std::max<u64>(rows, std::min<u64>(2 * h.full.n, kMaxRows)), true));
+    TRY(ensure_arr(e, h.delta, rows, true));
     TRY(ensure_arr(e, h.delta_next, h.delta.cap, false));
     TRY(ensure_hash(e, r));
     h.dense = h.full_lazy = 1;  // (the commit only counts FULL's new rows)
   }
-  for (int r : L.tmps) TRY(ensure_arr(e, e->h[r].newt, kHashMinRows, false));
+  for (int r : L.tmps) TRY(ensure_arr(e, e->h[r].newt, rows, false));
   return GDL_OK;
 }
 u64 hash_prefix(const gdl_engine *e, int r) { return ~dep_low_mask(e, e->rels[r]); }

@@ -46,10 +46,15 @@
 namespace gdl {
 
 constexpr u64 kHashEmpty = ~0ull;
-// A set holds up to three quarters of its slots.  The first is 2^23 slots, 64
-// MB: half of L2, and room for 6.3 M tuples.
+// A set holds up to three quarters of its slots.  The first has room for
+// kHashGrowth times the largest relation that the LIE starts from, up to 2^23
+// slots, 64 MB: half of L2, and 6.3 M tuples.  (With 2^23 whatever the input,
+// a three-edge graph took 384 MB for its sets and lists, twenty relations of
+// one tuple 4.6 GB.  The 64 x 64 grid's shortest paths are 533 for an edge,
+// the most of the benchmarks' programs.)
 __host__ __device__ constexpr u64 hash_rows(u64 slots) { return slots / 4 * 3; }
-constexpr u64 kHashMinRows = hash_rows(1ull << 23);
+constexpr u64 kHashFirstRows = hash_rows(1ull << 23);
+constexpr u64 kHashGrowth = 1024;
 
 struct HashJoinArgs {
   JoinArgs j;

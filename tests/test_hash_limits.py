@@ -2,6 +2,10 @@
 that pass the first set by millions of tuples, and probe chains that no larger
 set shortens.  Contents, loop passes and traces are whole numbers and equal the
 sorted lists'."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -111,3 +115,57 @@ def test_pieces_past_the_record_buffer():
         assert lie.fixpoint() == 2
         got = out.rows()
     assert np.array_equal(got, np.concatenate([rows, run_rows[:, ::-1]]))
+
+
+MEMORY = """
+import sys
+sys.path[:0] = sys.argv[1:3]
+import torch
+import test_hash_limits as T
+torch.zeros(1, device="cuda")
+before = torch.cuda.mem_get_info()[0]
+with T.Engine("gpu") as g:
+    T.twenty_relations(g)
+    torch.cuda.synchronize()
+    print((before - torch.cuda.mem_get_info()[0]) >> 20)
+"""
+
+
+def twenty_relations(eng):
+    edge = eng.relation("edge")
+    paths = [eng.relation(f"p{i}", arity=3, dependent_column_size=1, index_flag=False)
+             for i in range(20)]
+    for p in paths:
+        eng.load(p, np.array([[1, 2, 3]], dtype=np.uint64))
+    eng.load(edge, np.array([[1, 0]], dtype=np.uint64))
+    lie = eng.lie()
+    lie.add_relations(edge, True)
+    for p in paths:
+        lie.add_relations(p, False)
+    for p in paths[:10]:
+        lie.add_join(edge, FULL, p, DELTA, p, (INNER(1), OUTER(1), PLUS(OUTER(2), 1)))
+    assert lie.fixpoint() == 2
+    assert [p.size() for p in paths] == [2] * 10 + [1] * 10
+
+
+def test_small_programs_take_little_memory():
+    """Twenty relations of one tuple: the lists and sets follow the input (in
+    a process of its own, whose memory pool starts empty)."""
+    here = os.path.dirname(os.path.abspath(__file__))
+    pkg = os.path.join(os.path.dirname(here), "gdlog-multinode_b200")
+    out = subprocess.run([sys.executable, "-c", MEMORY, here, pkg], stdout=subprocess.PIPE,
+                         text=True, timeout=300, check=True).stdout
+    assert int(out) < 256
+
+
+@pytest.mark.parametrize("prog", ["tc", "path_length"])
+def test_a_first_set_sized_for_its_input_grows(prog):
+    """4,400 edges through one node derive 4.84 million pairs at once, more
+    than the 1,024 for an edge that the first set has room for."""
+    k = np.arange(2200)
+    edges = np.concatenate([np.stack([k, np.full(2200, 5000)], axis=1),
+                            np.stack([np.full(2200, 5000), k + 6000], axis=1)])
+    args = (edges.astype(np.uint64) + np.uint64(BASE),)
+    got = outcome(getattr(P, prog), args)
+    assert got[0]["path"][0] == 4400 + 2200 * 2200
+    assert got == outcome(getattr(P, prog), args, "sort")
