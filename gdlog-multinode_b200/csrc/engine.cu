@@ -329,6 +329,7 @@ struct gdl_engine {
   // a loop's first iteration meanwhile; ev_first marks that iteration's end.
   cudaStream_t cap_s = nullptr;
   cudaEvent_t ev_first = nullptr;
+  cudaEvent_t ev_loop = nullptr;  // behind this engine's last resident loop (ResidentQueue)
   u64 kernels_launched = 0;
   bool broken = false;  // a bounded wait gave up or a bounds check fired
   // The control block's build generation (index epochs), tracked on the
@@ -2952,6 +2953,37 @@ gdl_status presize_lists(gdl_engine *e, LieHost &L, const Plan &plan, u64 cap) {
   return GDL_OK;
 }
 
+// A resident loop's blocks wait for one another, so all of them must be on the
+// GPU: the engines of one process run such loops one at a time per device.
+// The order is kept on the device: each launch waits for an event behind the
+// one before it, so an engine's setup, listing and host wait overlap another's
+// loop (with a lock held until the loop's stream was idle, eight engines on
+// 2^10-id same generation made 2,620 queries a second, 4,090 before there were
+// resident loops).
+struct ResidentQueue {
+  std::mutex mu;
+  cudaEvent_t last = nullptr;  // behind the last loop launched (an engine's ev_loop)
+};
+ResidentQueue &resident_queue(const gdl_engine *e) {
+  static ResidentQueue q[64];
+  return q[e->device & 63];
+}
+gdl_status launch_resident(gdl_engine *e, LieHost &L) {
+  ResidentQueue &q = resident_queue(e);
+  std::lock_guard<std::mutex> lock(q.mu);
+  if (q.last && q.last != e->ev_loop) CK(e, cudaStreamWaitEvent(e->s, q.last, 0));
+  CK(e, cudaGraphLaunch(L.gexec, e->s));
+  CK(e, cudaEventRecord(e->ev_loop, e->s));
+  q.last = e->ev_loop;
+  return GDL_OK;
+}
+// (the engine's stream is idle: nothing needs to wait for its loops any more)
+void leave_resident_queue(gdl_engine *e) {
+  ResidentQueue &q = resident_queue(e);
+  std::lock_guard<std::mutex> lock(q.mu);
+  if (q.last == e->ev_loop) q.last = nullptr;
+}
+
 gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
   if (e->broken) return fail(e, GDL_E_TIMEOUT, "engine is in a failed state; destroy it");
   if ((int)L.ops.size() > kMaxOps) return fail(e, GDL_E_UNSUPPORTED, "too many ops in one LIE");
@@ -3366,11 +3398,6 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
                           cudaMemcpyDeviceToHost, e->s));
     return GDL_OK;
   };
-  // A resident loop's blocks wait for one another, so all of them must be on
-  // the GPU: engines of one process run such loops one at a time per device
-  // (each fills the GPU anyhow).
-  static std::mutex resident_mu[64];
-  std::unique_lock<std::mutex> resident_lock(resident_mu[e->device & 63], std::defer_lock);
   while (true) {
     c.pause = 0;
     c.stop_at = c.iteration + (use_graph ? std::min<u64>(trace_rows, 1u << 20) : batch);
@@ -3426,8 +3453,10 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
       k_begin<<<1, 32, 0, e->s>>>(e->d_rels, L.d_lie, e->d_ctl);
       L.kernels++;
       e->prof_launches[kPControl]++;
-      if (L.resident) resident_lock.lock();
-      CK(e, cudaGraphLaunch(L.gexec, e->s));
+      if (L.resident)
+        TRY(launch_resident(e, L));
+      else
+        CK(e, cudaGraphLaunch(L.gexec, e->s));
       L.graph_launches++;
     } else if (!use_graph) {
       c.cond_set = 0;
@@ -3446,7 +3475,6 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
     }
     TRY(enqueue_tail(it0, c.stop_at));
     CK(e, cudaStreamSynchronize(e->s));
-    if (resident_lock.owns_lock()) resident_lock.unlock();
     prof_collect(e);
     c = *e->h_ctl;
     e->generation = c.generation;
@@ -3864,6 +3892,7 @@ gdl_status gdl_engine_create(int32_t device, void *stream, gdl_engine **out) {
       bad(cudaMalloc(&e->d_pull_count, sizeof(u64))) || bad(cudaEventCreate(&e->ev0)) ||
       bad(cudaEventCreate(&e->ev1)) ||
       bad(cudaEventCreateWithFlags(&e->ev_first, cudaEventDisableTiming)) ||
+      bad(cudaEventCreateWithFlags(&e->ev_loop, cudaEventDisableTiming)) ||
       bad(cudaStreamCreateWithFlags(&e->cap_s, cudaStreamNonBlocking)) ||
       bad(cudaMemsetAsync(e->d_rels, 0, kMaxRels * sizeof(RelDev), e->s)) ||
       bad(cudaMemsetAsync(e->d_ctl, 0, sizeof(Ctl), e->s)) ||
@@ -4030,6 +4059,10 @@ gdl_status gdl_engine_destroy(gdl_engine *e) {
   if (e->ev0) cudaEventDestroy(e->ev0);
   if (e->ev1) cudaEventDestroy(e->ev1);
   if (e->ev_first) cudaEventDestroy(e->ev_first);
+  if (e->ev_loop) {
+    leave_resident_queue(e);
+    cudaEventDestroy(e->ev_loop);
+  }
   if (e->cap_s) cudaStreamDestroy(e->cap_s);
   prof_collect(e);
   for (cudaEvent_t ev : e->ev_pool) cudaEventDestroy(ev);

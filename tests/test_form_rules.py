@@ -1,5 +1,7 @@
 """Programs at the edges of the rules that pick a fixpoint's form (hash sets,
 row gathers, resident loops, linear recursion), against the CPU oracle."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -254,3 +256,41 @@ def test_wait_limit_of_a_look_back_is_not_the_barriers(polls_log2):
         g.clear()
         g.set_tuning(spin_limit_log2=polls_log2)
         assert P.cspa(g, *args).relations["value_alias"].digest() == want
+
+
+def test_engines_on_threads_take_turns_with_resident_loops():
+    """Engines of several threads, one of them dropped and made again between
+    its queries: resident loops run one at a time, each query's answer is its
+    own."""
+    queries = [(P.tc, (W.grid_edges(16, 16),)), (P.sg, (W.rmat_edges(10, 4096, seed=1),)),
+               (P.cspa, W.cspa_facts(150, 300, 100, seed=1)),
+               (P.tc, (W.layered_dag(5, 301, 2) + np.uint64(1 << 20),))]
+
+    def answers(eng, k):
+        prog, args = queries[k % len(queries)]
+        eng.clear()
+        return [(r.size(), r.digest()) for r in prog(eng, *args).relations.values()]
+
+    with Engine("gpu") as g:
+        want = [answers(g, k) for k in range(len(queries))]
+    wrong = []
+
+    def work(t):
+        try:
+            eng = Engine("gpu")
+            for k in range(40):
+                if t == 0 and k % 5 == 4:
+                    eng.close()
+                    eng = Engine("gpu")
+                if answers(eng, t + k) != want[(t + k) % len(queries)]:
+                    wrong.append((t, k))
+            eng.close()
+        except Exception as exc:
+            wrong.append((t, repr(exc)))
+
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(6)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert wrong == []
