@@ -294,3 +294,24 @@ def test_engines_on_threads_take_turns_with_resident_loops():
     for th in threads:
         th.join()
     assert wrong == []
+
+
+@pytest.mark.parametrize("scale,edges", [(8, 900), (10, 3000), (11, 7000)])
+def test_paths_derived_again_with_other_lengths(scale, edges):
+    """Most candidates of a random graph meet their pair in FULL, shorter:
+    the lengths are a breadth-first search's."""
+    e = W.rmat_edges(scale, edges, seed=scale)
+    adj = np.zeros((1 << scale, 1 << scale), dtype=np.float32)
+    adj[e[:, 0].astype(int), e[:, 1].astype(int)] = 1
+    want, new, length = np.zeros(adj.shape, dtype=np.uint64), adj > 0, 1
+    while new.any():
+        want[new] = length
+        new = (adj @ new.astype(np.float32) > 0) & (want == 0)
+        length += 1
+    pairs = np.argwhere(want)
+    want = np.concatenate([pairs.astype(np.uint64), want[want > 0][:, None]], axis=1)
+    for mode in (None, "sort"):
+        with Engine("gpu", dedup=mode) as g:
+            r = P.path_length(g, e)
+            assert r.iterations["plen"] == length - 1
+            assert np.array_equal(r.relations["path"].rows(), want)
