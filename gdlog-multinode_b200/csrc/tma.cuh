@@ -171,6 +171,8 @@ __global__ void __launch_bounds__(kTrBlock, 2)
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const u64 per = side;
   const u64 tiles = per * per;
+  // (nothing transposed: whole lines of each row one after another)
+  const u32 strip = gt || has_dt ? kTileStrip : 1;
   const u32 limit = a.ctl->spin_limit;
   for (int i = tid; i < kTmaTile / 16; i += kTrBlock)
     reinterpret_cast<uint4 *>(zero)[i] = make_uint4(0, 0, 0, 0);
@@ -187,7 +189,7 @@ __global__ void __launch_bounds__(kTrBlock, 2)
   auto issue = [&](u64 j) {
     const u64 t = blockIdx.x + j * gridDim.x;
     u32 tr, tc;
-    tile_rc((u32)t, (u32)per, tr, tc);
+    tile_rc((u32)t, (u32)per, strip, tr, tc);
     const int st = (int)(j % ns);
     mbar_expect_tx(&s_bar[st], 2 * kTmaTile);
     if (gt)
@@ -205,7 +207,7 @@ __global__ void __launch_bounds__(kTrBlock, 2)
     const u64 t = blockIdx.x + k * gridDim.x;
     const int st = (int)(k % ns), slot = (int)(k & 1);
     u32 tr, tc;
-    tile_rc((u32)t, (u32)per, tr, tc);
+    tile_rc((u32)t, (u32)per, strip, tr, tc);
     // (stage (k + ns - 1) % ns held tile k - 1, read before the last barrier)
     if (tid == 0 && k + ns - 1 < mine) issue(k + ns - 1);
     const bool ok = mbar_wait(&s_bar[st], (u32)(k / ns) & 1u, limit);
@@ -355,7 +357,7 @@ __global__ void __launch_bounds__(kTrBlock, 2)
   auto issue = [&](u64 j) {
     const u64 t = blockIdx.x + j * gridDim.x;
     u32 tr, tc;
-    tile_rc((u32)t, (u32)per, tr, tc);
+    tile_rc((u32)t, (u32)per, kTileStrip, tr, tc);
     const int st = (int)(j % ns);
     mbar_expect_tx(&s_bar[st], ni * kTmaTile);
     tma_load(in_s(st), &m.src, tc * 8, tr * 256, &s_bar[st]);
@@ -370,7 +372,7 @@ __global__ void __launch_bounds__(kTrBlock, 2)
     const u64 t = blockIdx.x + k * gridDim.x;
     const int st = (int)(k % ns), slot = (int)(k & 1);
     u32 tr, tc;
-    tile_rc((u32)t, (u32)per, tr, tc);
+    tile_rc((u32)t, (u32)per, kTileStrip, tr, tc);
     if (tid == 0 && k + ns - 1 < mine) issue(k + ns - 1);
     const bool ok = mbar_wait(&s_bar[st], (u32)(k / ns) & 1u, limit);
     u32 v[8], q[8];

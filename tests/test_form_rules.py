@@ -315,3 +315,19 @@ def test_paths_derived_again_with_other_lengths(scale, edges):
             r = P.path_length(g, e)
             assert r.iterations["plen"] == length - 1
             assert np.array_equal(r.relations["path"].rows(), want)
+
+
+@pytest.mark.parametrize("ids", [8449, 16384, 20000])
+def test_closure_with_a_hub(ids):
+    """More sources of one node than linear recursion's form takes: rows
+    gathered along in-edges, an update pass with nothing transposed, over
+    sides of 34, 64 and 79 tiles."""
+    rng = np.random.default_rng(ids)
+    e = np.concatenate([rng.integers(0, ids, (ids // 2, 2)),
+                        np.stack([np.arange(99), np.full(99, ids - 1)], axis=1)]).astype(np.uint64)
+    got = []
+    for mode in (None, "dense_push"):
+        with Engine("gpu", dedup=mode) as g:
+            r = P.tc(g, e)
+            got.append([r.iterations] + state(r.lies["tc"], r.output))
+    assert got[0] == got[1]
