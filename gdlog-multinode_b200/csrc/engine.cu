@@ -350,6 +350,7 @@ struct gdl_engine {
   std::vector<cudaEvent_t> ev_pool;
   u64 *pin_keys = nullptr;  // exports' pinned buffer (at most kExportPinned keys)
   u64 pin_cap = 0;
+  u64 exported = 0;         // keys exported so far
   struct Pending {
     int kind;
     cudaEvent_t a, b;
@@ -4316,7 +4317,9 @@ gdl_status gdl_relation_export(gdl_engine *e, int32_t rel, int32_t ver, uint64_t
     u64 n = 0;
     bool sorted;
     TRY(version_view(e, rel, ver, &p, &n, &sorted));
-    if (sorted && n > kExportPiece) {
+    const u64 before = e->exported;
+    if (rows && n <= cap) e->exported += n;
+    if (sorted && export_in_pieces(n, before, e->pin_cap)) {
       *out_n = n;
       if (n > cap)
         return fail(e, GDL_E_CAPACITY, "export needs %llu rows", (unsigned long long)n);

@@ -5,6 +5,12 @@
 // untouched before (one thread spent 25 of 35 ms on faulting them in for 4.3 M
 // rows of three columns).
 //
+// Pinned memory costs some 0.65 ms a megabyte when it is first taken, more than
+// the pieces save in one export below kExportFirst keys: those take the keys in
+// one copy until as many have been exported.  (Taken by every first export,
+// 1.3 M rows took 6.2 ms the first time, 2.4 after that; 3.8 in one copy.  4.3
+// M rows of three columns: 27, 3.4 and 25 ms; 14.6 M rows: 38, 8.7 and 90.)
+//
 // What the copies need from the device is behind Api, so that the order of the
 // steps and every failure of one can be run without a device:
 //   Key *buffer(keys, &cap)  pinned room for cap keys (at most `keys`), or null
@@ -26,6 +32,14 @@ namespace gdl {
 
 constexpr uint64_t kExportPiece = 1ull << 18;   // keys
 constexpr uint64_t kExportPinned = 1ull << 23;  // keys the pinned buffer holds at most
+constexpr uint64_t kExportFirst = 1ull << 22;   // keys of an export that takes it at once
+
+// Whether an export of n keys goes in pieces, `before` keys having been
+// exported and the buffer having room for cap.
+inline bool export_in_pieces(uint64_t n, uint64_t before, uint64_t cap) {
+  return n > kExportPiece &&
+         (cap >= std::min(n, kExportPinned) || n >= kExportFirst || before >= n);
+}
 
 enum ExportEnd { kExported = 0, kExportNoRoom, kExportFailed };
 

@@ -110,6 +110,19 @@ int main() {
       }
       bad += check(arity, n, Fake::kFinish, (n - 1) / 1000, gdl::kExportFailed);
     }
+  const u64 some = gdl::kExportPiece + 1, first = gdl::kExportFirst, pinned = gdl::kExportPinned;
+  const struct {
+    u64 n, before, cap;
+    bool pieces;
+  } rule[] = {{some - 1, 9 * some, pinned, false}, {some, 0, 0, false},    {some, some - 1, 0, false},
+              {some, some, 0, true},               {some, 0, some, true},  {some, 0, some - 1, false},
+              {first - 1, 0, some, false},         {first, 0, 0, true},    {4 * pinned, 0, 0, true},
+              {4 * pinned, 0, pinned, true}};
+  for (auto &x : rule)
+    if (gdl::export_in_pieces(x.n, x.before, x.cap) != x.pieces) {
+      printf("rule: n %llu\n", (unsigned long long)x.n);
+      bad++;
+    }
   if (!bad) printf("ok\n");
   return bad != 0;
 }

@@ -331,3 +331,19 @@ def test_closure_with_a_hub(ids):
             r = P.tc(g, e)
             got.append([r.iterations] + state(r.lies["tc"], r.output))
     assert got[0] == got[1]
+
+
+@pytest.mark.parametrize("n", [(1 << 18) + 1, (1 << 19) + 77])
+@pytest.mark.parametrize("arity", [2, 3])
+def test_second_export_in_pieces(n, arity):
+    """A first export below 2^22 rows comes over in one copy, a second one of
+    the size in pieces: the same rows."""
+    rng = np.random.default_rng(n)
+    rows = np.stack([rng.integers(0, 4000, n + 5000), rng.integers(0, 4096, n + 5000)] +
+                    [rng.integers(0, 1000, n + 5000)] * (arity == 3), axis=1).astype(np.uint64)
+    want = np.unique(rows, axis=0)[:n]
+    with Engine("gpu") as g:
+        r = g.relation("r", arity=arity)
+        g.load(r, want[rng.permutation(len(want))])
+        for _ in range(3):
+            assert np.array_equal(r.rows(), want)
