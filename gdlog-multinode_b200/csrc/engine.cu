@@ -1642,6 +1642,7 @@ ProdArgs product_args(gdl_engine *e, LieHost &L, const Plan &plan, size_t oi, co
   pa.F = e->h[op.inner].bmF;
   pa.rows_rec = &e->recs[9];
   pa.list = e->prod_list;
+  pa.sms = (u32)e->sms;
   pa.G = plan.pull_t[oi] ? out.bmOT : out.bmG;
   pa.dirty = plan.pull_t[oi] ? nullptr : out.dirty;
   pa.dk = L.dk;
@@ -3889,7 +3890,7 @@ gdl_status gdl_engine_create(int32_t device, void *stream, gdl_engine **out) {
       bad(cudaMallocHost(&e->h_rels_pin, kMaxRels * sizeof(RelDev) + 4 * sizeof(u64))) ||
       bad(cudaMalloc(&e->recs, 16 * sizeof(LaunchRec))) ||
       bad(cudaMalloc(&e->d_tmp, 4 * sizeof(DArr))) || bad(cudaMalloc(&e->d_u64, 4 * sizeof(u64))) ||
-      bad(cudaMalloc(&e->d_u32, (4 + (1u << 16) + 1) * sizeof(u32))) ||
+      bad(cudaMalloc(&e->d_u32, (4 + kProdListWords) * sizeof(u32))) ||
       bad(cudaMalloc(&e->d_pull_count, sizeof(u64))) || bad(cudaEventCreate(&e->ev0)) ||
       bad(cudaEventCreate(&e->ev1)) ||
       bad(cudaEventCreateWithFlags(&e->ev_first, cudaEventDisableTiming)) ||
@@ -3900,7 +3901,7 @@ gdl_status gdl_engine_create(int32_t device, void *stream, gdl_engine **out) {
       bad(cudaMemcpyAsync(&e->d_ctl->spin_limit, &e->spin_limit, sizeof(u32),
                           cudaMemcpyHostToDevice, e->s)) ||
       bad(cudaMemsetAsync(e->recs, 0, 16 * sizeof(LaunchRec), e->s)) ||
-      bad(cudaMemsetAsync(e->d_u32, 0, 5 * sizeof(u32), e->s)) ||
+      bad(cudaMemsetAsync(e->d_u32, 0, (4 + kProdListHead) * sizeof(u32), e->s)) ||
       bad(cudaMemsetAsync(e->d_pull_count, 0, sizeof(u64), e->s)) ||
       bad(cudaStreamSynchronize(e->s))) {
     gdl_engine_destroy(e);
@@ -4000,7 +4001,7 @@ gdl_status gdl_engine_clear(gdl_engine *e) {
       CK(e, cudaMemsetAsync(e->sort_offsets, 0, kMaxPasses * kMaxRadix * sizeof(u32), e->s));
     CK(e, cudaMemsetAsync(e->d_u32, 0, 4 * sizeof(u32), e->s));
     CK(e, cudaMemsetAsync(e->d_pull_count, 0, sizeof(u64), e->s));
-    CK(e, cudaMemsetAsync(e->prod_list, 0, sizeof(u32), e->s));
+    CK(e, cudaMemsetAsync(e->prod_list, 0, kProdListHead * sizeof(u32), e->s));
     TRY(reset_ctl(e));
     CK(e, cudaStreamSynchronize(e->s));
     e->broken = false;

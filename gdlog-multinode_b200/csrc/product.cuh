@@ -34,9 +34,10 @@
 // in shared memory and its warps OR equal shares of the listed inner rows,
 // whole rows at a time, at L2's rate (6 TB/s: 0.4 ns a key at 20,000 ids,
 // where a row costs the tables 350 ns however many keys it has).
-// Both run: k_prod_rows counts each row's keys and lists the long ones for
-// k_join_product (points-to relations are reflexive, so half the rows hold a
-// few keys and the others thousands; 20,000 variables: 260 -> 195 ms).
+// Both run: k_prod_rows counts each row's keys and lists the long ones, and by
+// those counts both kernels decide which rows k_join_product takes (points-to
+// relations are reflexive, so half the rows hold a few keys and the others
+// thousands; 20,000 variables: 260 -> 195 ms).
 //
 // A tmp NEWT outer (points-to's two-step rule) is derived anew in every
 // iteration, mostly the tuples of the iteration before: joined with all of
@@ -71,11 +72,61 @@ constexpr int kProdWarpRows = 32;
 constexpr u32 kProdRows = kProdWarps * kProdWarpRows;  // per block
 constexpr u32 kProdUnits = 6;        // units of work a block, at least
 constexpr int kProdPart = 4;         // words of a step staged together
-// A row is short, its keys listed, below 1 / kProdShort of the ids: a third
-// of what the tables take for it.
-constexpr u32 kProdShort = 64;
-__device__ __forceinline__ bool prod_short(u32 keys, u32 side) {
-  return keys * kProdShort < side * 256;
+// Which rows the tables take, decided on the device from what k_prod_rows
+// counts: the rows with a 64th of the ids or more (long), those with an eighth
+// or more (full; a sixteenth once the inner's bitmap is beyond L2), or none.
+// The costs compared are in keys listed (k_join_product_rows reads a row of
+// the inner a key).  Points-to, ms with every long row in the tables / now
+// (variables, facts a variable; in brackets before there were products):
+//    2,100, 0.8:  10.4 /  6.2  (7.6)        8,100, 2.75:  20.5 / 20.2  (100)
+//    3,000, 0.55: 11.2 /  7.2  (8.7)       12,000, 0.8:   27.8 / 21.1  (46)
+//    4,000, 2.75:  8.1 /  7.6  (34)        16,300, 0.8:   46.2 / 36.2  (62)
+//    6,000, 0.8:  13.2 /  9.5  (15.3)      20,000, 2.75:   172 / 166   (1109)
+constexpr u32 kProdLong = 64;
+__device__ __forceinline__ u32 prod_full_part(int dk) { return dk <= 14 ? 8u : 16u; }
+__device__ __forceinline__ bool prod_reaches(u32 keys, u32 part, u32 side) {
+  return keys * part >= side * 256;
+}
+// ProdArgs::list: the counts of the full rows and of the long ones, their keys
+// (in 32s), then the rows themselves.
+enum ProdKind : u32 { kProdFullRows = 0, kProdLongRows = 1, kProdNone = 2 };
+constexpr u32 kProdListHead = 4, kProdListRows = 1u << 16;
+__host__ __device__ constexpr u32 prod_list_at(u32 kind) {
+  return kProdListHead + kind * kProdListRows;
+}
+constexpr u32 kProdListWords = kProdListHead + 2 * kProdListRows;
+// The units of work of n rows in the tables: row blocks by column slices by
+// key ranges.  The key range is split until there are kProdUnits units a
+// block: at 20,000 ids 400 row-by-column blocks share 148 SMs unevenly (3
+// rounds for 2.7), and few long rows are few blocks.
+struct ProdSplit {
+  u32 n_rb, n_sl, ksteps, n_kc;
+};
+__device__ __forceinline__ ProdSplit prod_split(u32 n, u32 side, u32 sms) {
+  ProdSplit x;
+  x.n_rb = (n + kProdRows - 1) / kProdRows;
+  x.n_sl = (side + 3) / 4;
+  x.ksteps = max(2u, side * x.n_rb * x.n_sl / (kProdUnits * sms));
+  x.n_kc = (side + x.ksteps - 1) / x.ksteps;
+  return x;
+}
+// What n rows cost in the tables, in 32 listed keys.  A block of 1024 rows
+// takes 4.3 us a word of keys and slice, a fifth of it to build the tables, and
+// a listed key side x 5.3 ps (20,000 ids: 0.42 ns; 840 keys a row are the
+// same).  Fewer units than SMs cost as many times more.  (Whole numbers, so
+// that both kernels decide alike; 32 bits hold them: units are fewer than SMs
+// below 2^14 ids only.)
+__device__ __forceinline__ u32 prod_table_cost(u32 n, u32 side, u32 sms) {
+  const ProdSplit x = prod_split(n, side, sms);
+  const u32 units = x.n_rb * x.n_sl * x.n_kc;
+  const u32 keys = side * (68 * x.n_rb + 17 * n / 64);
+  return units - 1 < sms - 1 ? keys * sms / units : keys;
+}
+__device__ __forceinline__ u32 prod_kind(const u32 *list, u32 side, u32 sms) {
+  const uint4 c = *reinterpret_cast<const uint4 *>(list);  // (reset by the last block of the second one)
+  const u32 all = prod_table_cost(c.y, side, sms);
+  const u32 full = prod_table_cost(c.x, side, sms) + (c.w - c.z);
+  return c.w <= min(all, full) ? kProdNone : full < all ? kProdFullRows : kProdLongRows;
 }
 // Dynamic shared memory: the tables, two stages of 256 inner row slices, and
 // kProdPart of a step's 8 outer words, as two words each.
@@ -88,7 +139,8 @@ struct ProdArgs {
   u32 *G;          // output rows: the output's NEWT or its transposed twin
   u8 *dirty;       // dirty map of G, or null
   LaunchRec *rows_rec;  // launch record of k_join_product_rows
-  u32 *list;       // [0]: long rows of OT, then (from [1]) those rows
+  u32 *list;       // long rows of OT (prod_kind, prod_list_at)
+  u32 sms;         // blocks of k_join_product
   int dk;          // rows of 2^(dk-5) words
   u32 side;        // 256-id groups that hold ids
   // Repeated outer: the fresh part of OT and its size; part 1 takes it in
@@ -146,11 +198,11 @@ __device__ __forceinline__ bool product_empty(const JoinArgs &j, u64 *n_outer) {
   return *n_outer == 0;
 }
 
-// The long rows of OT, listed for k_join_product (which sets the count back
-// to zero), nearly in order: 32 rows a block, one atomic.
+// The full and the long rows of OT, listed for k_join_product
+// (k_join_product_rows sets the counts back to zero), nearly in order: 32 rows
+// a block, two atomics a list.
 __global__ void __launch_bounds__(256) k_prod_rows(ProdArgs a) {
-  __shared__ u32 s_any[8];
-  __shared__ u32 s_base;
+  __shared__ u32 s_keys[32];
   if (ctl_stop(a.j.ctl)) return;
   const u64 n_outer = eff_count(a.j.outer, a.j.outer_vis);
   if (n_outer == 0 || eff_count(a.j.inner, a.j.inner_vis) == 0) return;
@@ -159,7 +211,8 @@ __global__ void __launch_bounds__(256) k_prod_rows(ProdArgs a) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const u32 n4 = a.side * 2;
   for (u32 g = blockIdx.x; g < a.side * 8; g += gridDim.x) {
-    u32 mask = 0;  // this warp's four rows
+    __syncthreads();
+    // this warp's four rows
 #pragma unroll
     for (int q = 0; q < 4; q++) {
       const uint4 *p =
@@ -169,17 +222,23 @@ __global__ void __launch_bounds__(256) k_prod_rows(ProdArgs a) {
         const uint4 v = p[i];
         keys += __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
       }
-      if (!prod_short(__reduce_add_sync(0xffffffffu, keys), a.side)) mask |= 1u << q;
+      keys = __reduce_add_sync(0xffffffffu, keys);
+      if (lane == 0) s_keys[wid * 4 + q] = keys;
     }
     __syncthreads();
-    if (lane == 0) s_any[wid] = mask;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      const bool on = (s_any[lane >> 2] >> (lane & 3)) & 1u;
+    if (wid < 2) {  // a warp a list, a row a lane
+      const u32 keys = s_keys[lane];
+      const bool on = prod_reaches(keys, wid ? kProdLong : prod_full_part(a.dk), a.side);
       const u32 b = __ballot_sync(0xffffffffu, on);
-      if (lane == 0) s_base = b ? atomicAdd(&a.list[0], (u32)__popc(b)) : 0u;
-      __syncwarp();
-      if (on) a.list[1 + s_base + __popc(b & ((1u << lane) - 1u))] = g * 32 + lane;
+      const u32 sum = __reduce_add_sync(0xffffffffu, on ? keys / 32 : 0u);
+      u32 base = 0;
+      if (lane == 0 && b) {
+        base = atomicAdd(&a.list[wid], (u32)__popc(b));
+        atomicAdd(&a.list[2 + wid], sum);
+      }
+      base = __shfl_sync(0xffffffffu, base, 0);
+      if (on)
+        a.list[prod_list_at(wid) + base + __popc(b & ((1u << lane) - 1u))] = g * 32 + lane;
     }
   }
 }
@@ -206,14 +265,12 @@ __global__ void __launch_bounds__(kProdBlock, 1) k_join_product(ProdArgs a) {
   const int rs = a.dk - 5;
   const u32 row_words = 1u << rs;
   const u32 ids = a.side * 256;  // at most 2^dk
-  const u32 n_rows = *((volatile u32 *)&a.list[0]);
-  const u32 n_rb = (n_rows + MR - 1) / MR, n_sl = (ids + 1023) / 1024;
-  // The key range is split until there are kProdUnits units a block: at 20,000
-  // ids 400 row-by-column blocks share 148 SMs unevenly (3 rounds for 2.7),
-  // and few long rows are few blocks.
-  const u32 ksteps = max(2u, a.side * n_rb * n_sl / (kProdUnits * gridDim.x));
-  const u32 n_kc = (a.side + ksteps - 1) / ksteps;
-  const u32 units = n_rb * n_sl * n_kc;
+  const u32 kind = prod_kind(a.list, a.side, a.sms);
+  const u32 n_rows = kind == kProdNone ? 0u : *((volatile u32 *)&a.list[kind]);
+  const u32 *rows = a.list + prod_list_at(kind == kProdNone ? 0 : kind);
+  const ProdSplit split = prod_split(n_rows, a.side, a.sms);
+  const u32 n_sl = split.n_sl, n_kc = split.n_kc, ksteps = split.ksteps;
+  const u32 units = split.n_rb * n_sl * n_kc;
   const u32 lane4 = lane * 4;
   u64 flushed = 0;
   while (true) {
@@ -227,7 +284,7 @@ __global__ void __launch_bounds__(kProdBlock, 1) k_join_product(ProdArgs a) {
 #pragma unroll
     for (int r = 0; r < RW; r++) acc[r] = 0;
     // this thread's outer row (also lane l's: output row l of the warp)
-    const u32 my_row = rb * MR + tid < n_rows ? a.list[1 + rb * MR + tid] : kNoRow;
+    const u32 my_row = rb * MR + tid < n_rows ? rows[rb * MR + tid] : kNoRow;
     u32 av[8];
     auto load_a = [&](u32 s) {
       if (my_row != kNoRow) {
@@ -386,10 +443,8 @@ __global__ void __launch_bounds__(kProdBlock, 1) k_join_product(ProdArgs a) {
   // algorithmic bytes of both kernels together: OT and the inner once, 4 per
   // word reduced into the output
   if (lane == 0) prof_add(a.j.ctl, kPJoinMat, 4 * flushed);
-  if (launch_rec_finish(a.j.rec) && tid == 0) {
-    a.list[0] = 0;
+  if (launch_rec_finish(a.j.rec) && tid == 0)
     prof_add(a.j.ctl, kPJoinMat, (u64)ids * a.side * 32);
-  }
 }
 
 // A product that leaves the repeated tuples out still counts as having found
@@ -534,6 +589,11 @@ __global__ void __launch_bounds__(kProdRowsBlock, V <= 8 ? 2 : 1) k_join_product
   const int rs = a.dk - 5;
   const u32 n4 = a.side * 2;  // 16-byte words of a row that hold ids
   const u32 tiles = a.side * 256 / kRows;
+  // (without the rows that the launch before this one took)
+  const u32 kind = prod_kind(a.list, a.side, a.sms);
+  const u32 part = kind == kProdNone       ? 0u
+                   : kind == kProdFullRows ? prod_full_part(a.dk)
+                                           : kProdLong;
   u64 words_out = 0;
   while (true) {
     const long long t = grab_tile(a.rows_rec, &s_tile);
@@ -551,7 +611,7 @@ __global__ void __launch_bounds__(kProdRowsBlock, V <= 8 ? 2 : 1) k_join_product
         w[4 * j] = x.x, w[4 * j + 1] = x.y, w[4 * j + 2] = x.z, w[4 * j + 3] = x.w;
         left += __popc(x.x) + __popc(x.y) + __popc(x.z) + __popc(x.w);
       }
-      if (!prod_short(__reduce_add_sync(0xffffffffu, left), a.side)) left = 0;
+      if (prod_reaches(__reduce_add_sync(0xffffffffu, left), part, a.side)) left = 0;
     }
     while (true) {
       // all keys that are left, or when they do not fit the list a share of
@@ -636,8 +696,10 @@ __global__ void __launch_bounds__(kProdRowsBlock, V <= 8 ? 2 : 1) k_join_product
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) words_out += __shfl_xor_sync(0xffffffffu, words_out, o);
   if (lane == 0) prof_add(a.j.ctl, kPJoinMat, 4 * words_out);
-  if (launch_rec_finish(a.rows_rec) && tid == 0)
+  if (launch_rec_finish(a.rows_rec) && tid == 0) {
+    for (u32 i = 0; i < kProdListHead; i++) a.list[i] = 0;
     prof_add(a.j.ctl, kPJoinMat, (u64)a.side * 256 * a.side * 32);
+  }
 }
 
 }  // namespace gdl

@@ -347,3 +347,21 @@ def test_second_export_in_pieces(n, arity):
         g.load(r, want[rng.permutation(len(want))])
         for _ in range(3):
             assert np.array_equal(r.rows(), want)
+
+
+@pytest.mark.parametrize("n,facts", [(2100, 0.3), (4097, 0.2), (8300, 0.1), (16385, 0.05)])
+def test_products_of_sparse_relations(n, facts):
+    """Rows around an eighth and a sixteenth of the ids, where listed keys and
+    tables meet, at each width of a row."""
+    args = W.cspa_facts(n, int(2 * n * facts), int(0.75 * n * facts), seed=2)
+    args[0][0] = (n - 1, 0)
+
+    def run(eng):
+        r = P.cspa(eng, *args)
+        return [r.iterations] + [state(r.lies["analysis"], *r.relations.values())]
+
+    got = []
+    for mode in (None, "dense_push"):
+        with Engine("gpu", dedup=mode) as g:
+            got.append(run(g))
+    assert got[0] == got[1]
