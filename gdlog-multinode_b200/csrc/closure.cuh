@@ -205,6 +205,13 @@ __device__ __forceinline__ u32 closure_row_of(const ClosureRows &m, u32 id) {
   return i < m.n_inst && x < m.seg[i].n ? m.row_first[i] + x : kNoWord;
 }
 
+// Whether both columns lie in one instance.
+__device__ __forceinline__ bool closure_inside(const ClosureRows &m, u64 k) {
+  return !m.row_first || (((key_c0(k) ^ key_c1(k)) >> m.shift) == 0 &&
+                          closure_row_of(m, key_c0(k)) != kNoWord &&
+                          closure_row_of(m, key_c1(k)) != kNoWord);
+}
+
 __global__ void __launch_bounds__(256) k_closure_rows(ClosureRows m, u32 *row_word, u32 *row_inst) {
   for (u32 i = blockIdx.x; i < m.n_inst; i += gridDim.x) {
     const SegInfo s = m.seg[i];
@@ -225,23 +232,32 @@ __global__ void __launch_bounds__(256) k_closure_swap(const DArr *list, u64 *out
   }
 }
 
+// Sources per row, and the most of one row (both zero before).  An edge out of
+// the instances or between two of them is written to *bad: the general path
+// runs, whose bit-sets report it.
+__global__ void __launch_bounds__(256) k_closure_count(const u64 *edges, u64 n, ClosureRows m,
+                                                       u32 *count, u32 *most, u32 *bad) {
+  u32 mx = 0;
+  for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (u64)gridDim.x * blockDim.x) {
+    if (closure_inside(m, edges[i]))
+      mx = max(mx, atomicAdd(&count[closure_row_of(m, key_c1(edges[i]))], 1u) + 1);
+    else
+      *bad = 1;
+  }
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if ((threadIdx.x & 31) == 0 && mx) atomicMax(most, mx);
+}
+
 // From keys (row id, source id) sorted: adj, and each row's range (rows
-// without sources keep start = end = 0).  An edge out of the instances or
-// between two of them is written to *bad: the general path runs, whose
-// bit-sets report it.
+// without sources keep start = end = 0).
 __global__ void __launch_bounds__(256) k_closure_adj(const u64 *keys, u64 n, ClosureRows m,
-                                                     u32 *start, u32 *end, u32 *adj,
-                                                     u32 *bad) {
+                                                     u32 *start, u32 *end, u32 *adj) {
   for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (u64)gridDim.x * blockDim.x) {
     const u64 k = keys[i];
-    const u32 src = closure_row_of(m, key_c1(k)), row = closure_row_of(m, key_c0(k));
-    if (src == kNoWord || row == kNoWord || (key_c0(k) >> m.shift) != (key_c1(k) >> m.shift)) {
-      *bad = 1;
-      adj[i] = 0;
-      continue;
-    }
-    adj[i] = src;
+    const u32 row = closure_row_of(m, key_c0(k));
+    adj[i] = closure_row_of(m, key_c1(k));
     if (i == 0 || key_c0(keys[i - 1]) != key_c0(k)) {
       start[row] = (u32)i;
       end[row] = (u32)run_end(keys, n, i);
@@ -258,12 +274,6 @@ __global__ void __launch_bounds__(256) k_closure_degree(const u32 *start, const 
   if ((threadIdx.x & 31) == 0 && m) atomicMax(max_degree, m);
 }
 
-// Whether both columns lie in one instance.
-__device__ __forceinline__ bool closure_inside(const ClosureRows &m, u64 k) {
-  return !m.row_first || (((key_c0(k) ^ key_c1(k)) >> m.shift) == 0 &&
-                          closure_row_of(m, key_c0(k)) != kNoWord &&
-                          closure_row_of(m, key_c1(k)) != kNoWord);
-}
 // The first DELTA's tuples out of the instances or between two: as bad edges.
 __global__ void __launch_bounds__(256) k_closure_check(const u64 *keys, u64 n, ClosureRows m,
                                                        u32 *bad) {

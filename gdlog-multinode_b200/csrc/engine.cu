@@ -2063,13 +2063,40 @@ gdl_status prepare_closure(gdl_engine *e, LieHost &L) {
   p += 4;
   CK(e, cudaMemsetAsync(maxdeg, 0, 2 * sizeof(u32), e->s));  // and the flag of bad tuples
   ClosureRows m{nullptr, nullptr, 1, 31};
+  u32 *start = p, *end = p + rows, *word = p + 2 * rows, *inst = p + 3 * rows;
+  u32 *adj = p + 4 * rows;
+  const int gn = grid_for(e, n, 256, 8);
   if (e->instances) {
-    u32 *start = p, *end = p + rows, *word = p + 2 * rows, *inst = p + 3 * rows;
-    u32 *adj = p + 4 * rows, *d_first = adj + n;
+    u32 *d_first = adj + n;
     CK(e, cudaMemcpyAsync(d_first, first.data(), first.size() * sizeof(u32),
                           cudaMemcpyHostToDevice, e->s));
     m = ClosureRows{e->d_segs, d_first, (u32)e->segs.size(), e->seg_shift};
     CK(e, cudaMemsetAsync(start, 0, 2 * rows * sizeof(u32), e->s));
+    if (n) {  // (`end` holds the counts)
+      k_closure_count<<<gn, 256, 0, e->s>>>(e->h[in].full.ptr, n, m, end, maxdeg, maxdeg + 1);
+      e->aux_launches++;
+    }
+    if (e->h[r].delta.n) {
+      k_closure_check<<<grid_for(e, e->h[r].delta.n, 256, 8), 256, 0, e->s>>>(
+          e->h[r].delta.ptr, e->h[r].delta.n, m, maxdeg + 1);
+      e->aux_launches++;
+    }
+  } else {
+    TRY(build_inverse(e, in, L.dk));
+    const RelHost &ih = e->rels[in];
+    a.start = ih.inv_off;
+    a.end = ih.inv_off + 1;
+    a.adj = ih.inv_keys;
+    k_closure_degree<<<grid_for(e, rows, 256, 4), 256, 0, e->s>>>(a.start, a.end, a.rows, maxdeg);
+    e->aux_launches++;
+  }
+  CK(e, cudaGetLastError());
+  CK(e, cudaMemcpyAsync(e->h_scalars, maxdeg, 2 * sizeof(u32), cudaMemcpyDeviceToHost, e->s));
+  CK(e, cudaStreamSynchronize(e->s));
+  const u32 *deg = reinterpret_cast<const u32 *>(e->h_scalars);
+  if (deg[0] > kClosureMaxDegree || deg[1]) return GDL_OK;
+  if (e->instances) {
+    CK(e, cudaMemsetAsync(end, 0, rows * sizeof(u32), e->s));
     k_closure_rows<<<(int)std::min<u64>(first.size(), (u64)e->sms * 8), 256, 0, e->s>>>(m, word,
                                                                                         inst);
     e->aux_launches++;
@@ -2077,20 +2104,14 @@ gdl_status prepare_closure(gdl_engine *e, LieHost &L) {
       // the edges by column 1
       u64 *keys = nullptr;
       TRY(dalloc(e, (void **)&keys, n * sizeof(u64)));
-      k_closure_swap<<<grid_for(e, n, 256, 8), 256, 0, e->s>>>(&e->d_rels[in].full, keys);
+      k_closure_swap<<<gn, 256, 0, e->s>>>(&e->d_rels[in].full, keys);
       e->aux_launches++;
       const DArr d{keys, n, n};
       CK(e, cudaMemcpyAsync(e->d_tmp, &d, sizeof d, cudaMemcpyHostToDevice, e->s));
       TRY(sort_in_place(e, e->d_tmp, d));
-      k_closure_adj<<<grid_for(e, n, 256, 8), 256, 0, e->s>>>(keys, n, m, start, end, adj,
-                                                                    maxdeg + 1);
+      k_closure_adj<<<gn, 256, 0, e->s>>>(keys, n, m, start, end, adj);
       e->aux_launches++;
       dfree(e, keys);  // stream-ordered
-    }
-    if (e->h[r].delta.n) {
-      k_closure_check<<<grid_for(e, e->h[r].delta.n, 256, 8), 256, 0, e->s>>>(
-          e->h[r].delta.ptr, e->h[r].delta.n, m, maxdeg + 1);
-      e->aux_launches++;
     }
     a.start = start;
     a.end = end;
@@ -2098,19 +2119,7 @@ gdl_status prepare_closure(gdl_engine *e, LieHost &L) {
     a.row_word = word;
     a.row_inst = inst;
     a.inst_last = L.d_inst_last;
-  } else {
-    TRY(build_inverse(e, in, L.dk));
-    const RelHost &ih = e->rels[in];
-    a.start = ih.inv_off;
-    a.end = ih.inv_off + 1;
-    a.adj = ih.inv_keys;
   }
-  k_closure_degree<<<grid_for(e, rows, 256, 4), 256, 0, e->s>>>(a.start, a.end, a.rows, maxdeg);
-  e->aux_launches++;
-  CK(e, cudaMemcpyAsync(e->h_scalars, maxdeg, 2 * sizeof(u32), cudaMemcpyDeviceToHost, e->s));
-  CK(e, cudaStreamSynchronize(e->s));
-  const u32 *deg = reinterpret_cast<const u32 *>(e->h_scalars);
-  if (deg[0] > kClosureMaxDegree || deg[1]) return GDL_OK;
   RelDev &h = e->h[r];
   const u64 words = L.map.words;
   if (!h.bmDN) TRY(dalloc(e, (void **)&h.bmDN, words * 4));
