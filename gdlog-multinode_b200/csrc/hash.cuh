@@ -34,8 +34,8 @@
 //
 // A key takes its slot before the list's counter counts it, so an iteration
 // may pass the three quarters before the overflow is seen: up to 224 keys a
-// warp wait uncounted, and a warp looks at the overflow flag once a step.  A
-// set may even fill up.  Probe chains are therefore bounded (kHashMaxProbe):
+// warp wait uncounted, and a warp looks at the overflow flag every four steps
+// of 32 candidates.  A set may even fill up.  Probe chains are therefore bounded (kHashMaxProbe):
 // past the bound the iteration ends uncommitted and runs again, from a larger
 // set where the rows counted ask for one, else (the chain is the tuples of one
 // prefix, which no larger set shortens) on sorted lists.
@@ -268,9 +268,10 @@ __device__ __forceinline__ void hash_join(const HashJoinArgs &a, HashSmem &hs) {
     sm.excl[wid][lane] = inc - l;
     __syncwarp();
     for (u64 base = 0; base < total; base += 32) {
-      // (a chunk may hold thousands of candidates; the load is under way with
-      // the step's others)
-      over = *((volatile u32 *)&j.ctl->overflow);
+      // (a chunk may hold thousands of candidates: a look every four steps,
+      // its load under way with the step's others)
+      const bool look = (base & 96) == 96;
+      if (look) over = *((volatile u32 *)&j.ctl->overflow);
       const u64 p = base + lane;
       u64 t = 0;
       bool ok = false;
@@ -284,7 +285,7 @@ __device__ __forceinline__ void hash_join(const HashJoinArgs &a, HashSmem &hs) {
       }
       emitted |= ok;
       hash_emit(a, s_out[wid], waiting, t, ok);
-      if (__any_sync(0xffffffffu, over != 0)) break;
+      if (look && __any_sync(0xffffffffu, over != 0)) break;
     }
     __syncwarp();
     cand += total;
@@ -311,10 +312,12 @@ __device__ __forceinline__ void hash_heavy(const HashJoinArgs &a, u64 np, WarpOu
   bool emitted = false;
   u32 waiting = 0;
   for (u64 k = blockIdx.x; k < np; k += gridDim.x) {
+    if (__any_sync(0xffffffffu, *((volatile u32 *)&j.ctl->overflow) != 0)) break;
     const u64 row = j.crow_key[k];
     const u32 s = j.crow_start[k], l = j.crow_len[k];
     for (u32 j0 = threadIdx.x & ~31u; j0 < l; j0 += blockDim.x) {  // (warp-uniform)
-      const u32 over = *((volatile u32 *)&j.ctl->overflow);
+      const bool look = ((j0 / blockDim.x) & 3) == 3;
+      const u32 over = look ? *((volatile u32 *)&j.ctl->overflow) : 0u;
       const u32 q = j0 + (threadIdx.x & 31);
       u64 t = 0;
       bool ok = false;
@@ -324,7 +327,7 @@ __device__ __forceinline__ void hash_heavy(const HashJoinArgs &a, u64 np, WarpOu
       }
       emitted |= ok;
       hash_emit(a, s_out[threadIdx.x >> 5], waiting, t, ok);
-      if (__any_sync(0xffffffffu, over != 0)) break;
+      if (look && __any_sync(0xffffffffu, over != 0)) break;
     }
     cand += l;
   }
