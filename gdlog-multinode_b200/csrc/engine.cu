@@ -3014,6 +3014,19 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
                   "op output %s is neither an update nor a tmp relation of the LIE",
                   e->rels[op.out].name.c_str());
   }
+  // A FULL kept as a bitmap only has a count and no list of that length: no
+  // relation to derive into, nor one whose FULL an operator reads.
+  std::vector<char> lists(is_update);
+  for (const OpHost &op : L.ops) {
+    if (op.kind == 0 ? op.inner_ver != GDL_DELTA : op.kind == 1 && op.inner_ver == GDL_FULL)
+      lists[op.inner] = 1;
+    if (op.outer >= 0 && op.outer_ver == GDL_FULL) lists[op.outer] = 1;
+  }
+  for (size_t r = 0; r < lists.size(); r++)
+    if (lists[r] && e->rels[r].full_resident)
+      return fail(e, GDL_E_UNSUPPORTED,
+                  "FULL of %s is kept as a bitmap only (batched form, too large for a list)",
+                  e->rels[r].name.c_str());
   Plan plan = make_plan(e, L);
   // The timed span is the whole call, as the reference's drivers time the
   // whole fixpoint_loop (test/tc.cu:120-140): setup, loop and finish.
@@ -3069,11 +3082,6 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
   mark("arrays");
   // Dense form (dense.cuh) when the key domain is small enough; always in
   // the batched form, whose block-diagonal bitmap is the only layout.
-  for (int r : L.update)
-    if (e->rels[r].full_resident)
-      return fail(e, GDL_E_UNSUPPORTED,
-                  "FULL of %s is kept as a bitmap only (batched form, too large for a list)",
-                  e->rels[r].name.c_str());
   {
     // (by default at least one 256 x 256-bit tile, so that every domain has
     // the passes over tiles; pull.cuh, product.cuh)

@@ -365,3 +365,34 @@ def test_products_of_sparse_relations(n, facts):
         with Engine("gpu", dedup=mode) as g:
             got.append(run(g))
     assert got[0] == got[1]
+
+
+def test_a_full_beyond_the_list_limit_is_not_read_as_a_list():
+    """32,768 sources and 32,767 targets of one node: 2^30 pairs and more, a
+    FULL that is kept as a bitmap.  A later LIE that reads it, as an inner or
+    as an outer, or derives into it, is refused; the relation stays as it is."""
+    k = np.arange(32768)
+    edges = np.concatenate([np.stack([k + 1, np.zeros_like(k)], axis=1),
+                            np.stack([np.zeros_like(k), k + 32769], axis=1)[:-1]]).astype(np.uint64)
+    total = len(edges) + 32768 * 32767
+    assert total > (1 << 30) - 4096 and edges.max() < 1 << 16
+    with Engine("gpu") as g:
+        path = P.tc(g, edges).output
+        assert path.size() == total
+        out = g.relation("out", index_flag=False)
+        other = g.relation("other")
+        g.load(out, edges[:5])
+        g.load(other, edges[:5])
+        digest = path.digest()
+        for inner, outer, ver, update in ((path, out, DELTA, out), (other, path, FULL, out),
+                                          (other, path, DELTA, path)):
+            lie = g.lie()
+            lie.add_relations(other, True)
+            if update is not path:
+                lie.add_relations(path, True)
+            lie.add_relations(update, False)
+            lie.add_join(inner, FULL, outer, ver, update, (OUTER(1), INNER(1)))
+            with pytest.raises(GdlError) as err:
+                lie.fixpoint()
+            assert err.value.code == 4
+            assert (path.size(), path.digest()) == (total, digest)
