@@ -251,6 +251,9 @@ struct gdl_engine {
   // (GDLOG_NO_TMA=1 keeps the LDG/STG passes of pull.cuh).
   bool tma_ok = false;
   void *tma_encode = nullptr;
+  // (dropped before a fixpoint when there are kTmapsMax: recycled addresses meet
+  // new sizes in a service)
+  static constexpr size_t kTmapsMax = 1024;
   std::map<std::tuple<const void *, int, u32>, CUtensorMap> tmaps;
   std::vector<cudaGraphExec_t> graveyard;
   std::mutex reap_mu;
@@ -3027,6 +3030,7 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
       return fail(e, GDL_E_UNSUPPORTED,
                   "FULL of %s is kept as a bitmap only (batched form, too large for a list)",
                   e->rels[r].name.c_str());
+  if (e->tmaps.size() >= gdl_engine::kTmapsMax) e->tmaps.clear();
   Plan plan = make_plan(e, L);
   // The timed span is the whole call, as the reference's drivers time the
   // whole fixpoint_loop (test/tc.cu:120-140): setup, loop and finish.
