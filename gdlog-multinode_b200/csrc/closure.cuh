@@ -16,9 +16,10 @@
 // The loop is resident (loop.cuh): one grid barrier an iteration.  A warp
 // looks at up to 32 rows at once (a lane a row: its sources' extents), then
 // takes the rows with something to do: four at a time by eight lanes each
-// (their loads overlap), a single one with a long extent by all lanes.  A row with many sources is one
-// warp's serial work, so in-degrees are bounded by kClosureMaxDegree; beyond
-// it the edge-balanced join (pull.cuh, k_join_rows_bm) runs instead.
+// (their loads overlap), a single one with a long extent by all lanes.  A row
+// with many sources is one warp's serial work, so in-degrees are bounded by
+// kClosureMaxDegree; beyond it the edge-balanced join (pull.cuh,
+// k_join_rows_bm) runs instead.
 //
 // Both layouts: the square domain (row x at x << rs) and the batched form's
 // block diagonal (rows numbered through all instances).

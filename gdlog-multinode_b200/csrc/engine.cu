@@ -1557,11 +1557,7 @@ JoinArgs join_args(gdl_engine *e, LieHost &L, const Plan &plan, size_t oi) {
   } else {
     a.outer = &R[op.outer].newt;
     a.outer_vis = nullptr;
-    if (dense && oh.bmG && plan.pull[oi]) {
-      // pull form: NEWT's bitmap transposed, its size counted (no list)
-      a.outer_bm = oh.bmG;
-      a.outer_bm_words = words;
-    } else if (dense && oh.bmG) {
+    if (dense && oh.bmG) {
       a.outer_bm = oh.bmG;
       a.outer_bm_words = words;
     }
@@ -2165,9 +2161,10 @@ gdl_status start_closure(gdl_engine *e, LieHost &L) {
   return GDL_OK;
 }
 
-// The resident loop as the graph body's one launch.  Two blocks an SM at
-// most (all resident); fewer where a domain has less work than that (a
-// barrier's cost grows with its blocks).
+// The resident loop as the graph body's one launch, all its blocks resident:
+// two an SM at most, four in the hash form, three in the closure form; fewer
+// where a domain has less work than that (a barrier's cost grows with its
+// blocks).
 cudaError_t launch_loop(gdl_engine *e, LieHost &L, Counts *kc) {
   if (L.hashed) {
     HashLoopArgs a;

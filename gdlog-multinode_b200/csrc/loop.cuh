@@ -531,7 +531,9 @@ __global__ void __launch_bounds__(kLoopBlock, 2) k_lie_loop(LoopArgs a) {
         if (nn) atomicAdd((unsigned long long *)&u.rd->scan.pop_g, (unsigned long long)nn);
       }
     }
-    go = loop_barrier(ctl, gen, &s_go, [&](int lane) { return loop_commit<false>(a.rels, a.lie, ctl, lists, lane); });
+    go = loop_barrier(ctl, gen, &s_go, [&](int lane) {
+      return loop_commit<false>(a.rels, a.lie, ctl, lists, lane);
+    });
   }
   if (blockIdx.x == 0 && threadIdx.x == 0 && ctl->cond_set)
     cudaGraphSetConditional((cudaGraphConditionalHandle)ctl->cond_handle, 0u);

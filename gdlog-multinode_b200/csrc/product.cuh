@@ -123,7 +123,8 @@ __device__ __forceinline__ u32 prod_table_cost(u32 n, u32 side, u32 sms) {
   return units - 1 < sms - 1 ? keys * sms / units : keys;
 }
 __device__ __forceinline__ u32 prod_kind(const u32 *list, u32 side, u32 sms) {
-  const uint4 c = *reinterpret_cast<const uint4 *>(list);  // (reset by the last block of the second one)
+  // (reset by the second kernel's last block, when all have read them)
+  const uint4 c = *reinterpret_cast<const uint4 *>(list);
   const u32 all = prod_table_cost(c.y, side, sms);
   const u32 full = prod_table_cost(c.x, side, sms) + (c.w - c.z);
   return c.w <= min(all, full) ? kProdNone : full < all ? kProdFullRows : kProdLongRows;
@@ -160,10 +161,6 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src, u32 bytes
                : "memory");
 }
 
-// src/join.cu:38-45 for a product: an empty inner empties the OUTER (every
-// block calls this; a NEWT outer's bitmap is cleared too).  Returns whether
-// there is nothing to join.  The inner is looked at first: no block reads
-// the outer's count while block 0 may be zeroing it.
 // The two parts against the whole: by their tuples, with room for what they
 // cost beyond that (at 20,000 variables: 8.2 ms for 6.6 where a tenth of NEWT
 // was fresh or DELTA, 1.2 for 6.6 at a fiftieth).
@@ -178,6 +175,10 @@ __device__ __forceinline__ const u32 *prod_outer(const ProdArgs &a) {
   return few && a.j.outer->n && a.j.inner->n ? a.OT : nullptr;
 }
 
+// src/join.cu:38-45 for a product: an empty inner empties the OUTER (every
+// block calls this; a NEWT outer's bitmap is cleared too).  Returns whether
+// there is nothing to join.  The inner is looked at first: no block reads
+// the outer's count while block 0 may be zeroing it.
 __device__ __forceinline__ bool product_empty(const JoinArgs &j, u64 *n_outer) {
   if (eff_count(j.inner, j.inner_vis) == 0) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -318,7 +319,8 @@ __global__ void __launch_bounds__(kProdBlock, 1) k_join_product(ProdArgs a) {
       const u32 *B = sB + st * kProdStep * 32;
 #pragma unroll
       for (int part = 0; part < 8; part += kPart) {
-        // the outer's words of this part, as table offsets: bytes 0, 1 (times 128) in one word, bytes 2, 3 in the next
+        // the outer's words of this part, as table offsets: bytes 0, 1 (times
+        // 128) in one word, bytes 2, 3 in the next
 #pragma unroll
         for (int w = 0; w < kPart; w++) {
           const u32 x = av[part + w];
