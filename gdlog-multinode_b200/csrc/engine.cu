@@ -1036,10 +1036,13 @@ Plan make_plan(gdl_engine *e, const LieHost &L) {
   p.product.assign(L.ops.size(), 0);
   p.repeats.assign(L.ops.size(), 0);
   {
-    std::vector<char> is_static(n, 0), is_update(n, 0), newt_read(n, 0);
+    // (an ACopy replaces its output's NEWT, and a Copy from an empty source
+    // empties it, the first time: what a join put there before is not in FULL)
+    std::vector<char> is_static(n, 0), is_update(n, 0), newt_read(n, 0), replaced(n, 0);
     for (int r : L.statics) is_static[r] = 1;
     for (int r : L.update) is_update[r] = 1;
     for (const OpHost &op : L.ops) {
+      if (op.kind != 0) replaced[op.out] = 1;
       if (op.kind == 0 && op.outer_ver == GDL_NEWT) newt_read[op.outer] = 1;
       if (op.kind == 2 || (op.kind == 1 && op.inner_ver == GDL_NEWT)) newt_read[op.inner] = 1;
     }
@@ -1047,7 +1050,7 @@ Plan make_plan(gdl_engine *e, const LieHost &L) {
       const OpHost &op = L.ops[oi];
       p.static_once[oi] = op.kind == 0 && !op.hook && op.inner_ver == GDL_FULL &&
                           op.outer_ver == GDL_FULL && is_static[op.inner] && is_static[op.outer] &&
-                          is_update[op.out] && !newt_read[op.out];
+                          is_update[op.out] && !newt_read[op.out] && !replaced[op.out];
     }
   }
   for (const OpHost &op : L.ops) {

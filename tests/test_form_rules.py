@@ -396,3 +396,35 @@ def test_a_full_beyond_the_list_limit_is_not_read_as_a_list():
                 lie.fixpoint()
             assert err.value.code == 4
             assert (path.size(), path.digest()) == (total, digest)
+
+
+def static_join_and_copy(eng, ids, base, kind):
+    """A join of two static relations whose output's NEWT an ACopy replaces,
+    or a Copy from an empty source empties in the first iteration only: its
+    tuples are not in FULL after the iteration that ran it."""
+    rng = np.random.default_rng(ids)
+    s, f, none = eng.relation("s"), eng.relation("f"), eng.relation("none")
+    u, v = eng.relation("u", index_flag=False), eng.relation("v", index_flag=False)
+    for r, n in ((s, ids // 2), (f, ids // 2), (u, ids // 8), (v, ids // 8)):
+        eng.load(r, rng.integers(0, ids, size=(n, 2)).astype(np.uint64) + np.uint64(base))
+    eng.load(none, None)
+    lie = eng.lie()
+    for r in (s, f, none):
+        lie.add_relations(r, True)
+    for r in (u, v):
+        lie.add_relations(r, False)
+    lie.add_join(s, FULL, f, FULL, u, (OUTER(1), INNER(1)))
+    lie.add_join(s, FULL, v, DELTA, v, (OUTER(1), INNER(1)))
+    if kind == "copy":
+        lie.add_copy(none, FULL, u, P.CP_SWAP)
+    else:
+        lie.add_acopy(v, u, P.CP_SWAP if kind == "swap" else (0, 1))
+    lie.max_iteration = 6
+    return [lie.fixpoint()] + state(lie, u, v)
+
+
+@pytest.mark.parametrize("kind", ["copy", "swap", "acopy"])
+@pytest.mark.parametrize("ids,base", [(200, 0), (1500, 0), (5000, 0), (300, 1 << 20)])
+def test_static_join_before_a_copy(ids, base, kind):
+    both(static_join_and_copy, ids, base, kind)
+    both(static_join_and_copy, ids, base, kind, mode="dense_push")
