@@ -1722,10 +1722,14 @@ gdl_status prepare_hash(gdl_engine *e, LieHost &L) {
   return GDL_OK;
 }
 u64 hash_prefix(const gdl_engine *e, int r) { return ~dep_low_mask(e, e->rels[r]); }
-gdl_status fill_hash(gdl_engine *e, int r) {
+gdl_status clear_hash(gdl_engine *e, int r) {
   const RelDev &h = e->h[r];
   CK(e, cudaMemsetAsync(h.hset, 0xFF, (h.hmask + 2) * sizeof(u64), e->s));
   if (h.hord) CK(e, cudaMemsetAsync(h.hord, 0xFF, (h.hmask + 2) * sizeof(u32), e->s));
+  return GDL_OK;
+}
+gdl_status fill_hash(gdl_engine *e, int r) {
+  const RelDev &h = e->h[r];
   if (h.full.n) {
     k_hash_fill<<<grid_for(e, h.full.n, 256, 8), 256, 0, e->s>>>(&e->d_rels[r], hash_prefix(e, r),
                                                                   e->d_ctl);
@@ -3205,6 +3209,9 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
   }
   TRY(ensure_scratch(e));
   mark("scratch");
+  // (the sets are emptied while the host goes on, 64 MB each)
+  if (L.hashed)
+    for (int r : L.update) TRY(clear_hash(e, r));
   TRY(push(e));
   mark("push");
   if (L.dense) {
@@ -3566,7 +3573,10 @@ gdl_status fixpoint(gdl_engine *e, LieHost &L, uint64_t *out_iters) {
         TRY(push(e));
         TRY(reset_ctl(e));
         c.generation = e->generation;
-        for (int r : L.update) TRY(fill_hash(e, r));
+        for (int r : L.update) {
+          TRY(clear_hash(e, r));
+          TRY(fill_hash(e, r));
+        }
         // (the scratch the joins write pieces to may have moved)
         if (L.resident) TRY(push_hash_loop(e, L, plan));
       }
